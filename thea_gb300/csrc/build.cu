@@ -599,79 +599,6 @@ __global__ void point_records_kernel(float const * __restrict__ P, int64_t n, in
   pt_rec[s] = make_float4(p.x, p.y, p.z, __int_as_float(e));
 }
 
-// Oriented slab of every child slot (slab_normal / slab_lower_bound in traverse_ops.cuh): n = the area-weighted mean of
-// the slot's triangle normals (triangles with a non-finite normal or area left out; +z if the mean vanishes), encoded
-// and decoded as the searches decode it, and the range of n . v over the slot's vertices, accumulated in double
-// (products of floats are exact in double) and rounded outwards to float. One block per slot, slots taken in a
-// grid-stride loop; slots with no elements get an empty slab.
-constexpr int SLAB_THREADS = 128;
-
-__global__ void __launch_bounds__(SLAB_THREADS)
-slab_kernel(int2 const * __restrict__ ranges, int64_t slots, float4 const * __restrict__ rec, float4 * __restrict__ out) {
-  __shared__ float s_n[3][SLAB_THREADS / 32];
-  __shared__ double s_d[2][SLAB_THREADS / 32];
-  __shared__ float4 s_enc;
-  int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int64_t slot = blockIdx.x; slot < slots; slot += gridDim.x) {
-    int2 r = ranges[slot];
-    if (r.y <= 0) {
-      if (t == 0) out[slot] = make_float4(0.f, 0.f, INFINITY, -INFINITY);
-      continue;
-    }
-    int64_t k0 = r.x, k1 = (int64_t)r.x + r.y;
-    float nx = 0.f, ny = 0.f, nz = 0.f;
-    for (int64_t k = k0 + t; k < k1; k += SLAB_THREADS) {
-      float4 nn = __ldg(rec + k * CP_REC_F4 + 3);
-      float area = __ldg(rec + k * CP_REC_F4 + 6).w;
-      if (isfinite(nn.x) && isfinite(nn.y) && isfinite(nn.z) && isfinite(area)) {
-        nx += nn.x * area;
-        ny += nn.y * area;
-        nz += nn.z * area;
-      }
-    }
-    for (int o = 16; o; o >>= 1) {
-      nx += __shfl_xor_sync(0xffffffffu, nx, o);
-      ny += __shfl_xor_sync(0xffffffffu, ny, o);
-      nz += __shfl_xor_sync(0xffffffffu, nz, o);
-    }
-    if (lane == 0) s_n[0][warp] = nx, s_n[1][warp] = ny, s_n[2][warp] = nz;
-    __syncthreads();
-    if (t == 0) {
-      float x = 0.f, y = 0.f, z = 0.f;
-      for (int w = 0; w < SLAB_THREADS / 32; ++w) x += s_n[0][w], y += s_n[1][w], z += s_n[2][w];
-      float l = sqrtf(x * x + y * y + z * z);
-      if (!(l > 0.f) || !isfinite(l)) x = 0.f, y = 0.f, z = 1.f, l = 1.f;
-      s_enc = slab_encode(V3{x / l, y / l, z / l});
-    }
-    __syncthreads();
-    float4 enc = s_enc;
-    V3 n = slab_normal(enc);
-    double lo = INFINITY, hi = -INFINITY;
-    for (int64_t k = k0 + t; k < k1; k += SLAB_THREADS) {
-#pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        float4 q = __ldg(rec + k * CP_REC_F4 + v);
-        double d = (double)n.x * (double)q.x + (double)n.y * (double)q.y + (double)n.z * (double)q.z;
-        lo = fmin(lo, d);
-        hi = fmax(hi, d);
-      }
-    }
-    for (int o = 16; o; o >>= 1) {
-      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (lane == 0) s_d[0][warp] = lo, s_d[1][warp] = hi;
-    __syncthreads();
-    if (t == 0) {
-      for (int w = 1; w < SLAB_THREADS / 32; ++w) lo = fmin(lo, s_d[0][w]), hi = fmax(hi, s_d[1][w]);
-      enc.z = __double2float_rd(lo);
-      enc.w = __double2float_ru(hi);
-      out[slot] = enc;
-    }
-    __syncthreads();
-  }
-}
-
 constexpr int COLLAPSE_LEVELS_PER_SYNC = 6;
 
 template <int W>
@@ -894,121 +821,238 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
   }
 }
 
-// Element range [first, end) of every node's subtree, from its children's: leaves carry their run, internal children
-// follow their parent in the node array (the collapse emits level by level). One pass settles every node whose
-// children are settled; a node array that breaks those rules (an image written by another build) sets `bad`.
+//============================================================================================================================
+// Oriented slabs of the child slots (slab_normal / slab_lower_bound in traverse_ops.cuh): n = the area-weighted mean of
+// the slot's triangle normals (triangles with a non-finite normal or area left out; +z if the mean vanishes), encoded and
+// decoded as the searches decode it, and the range of n . v over the slot's vertices, widened by the rounding of its
+// FP32 evaluation (in FP64 the pass took 64 us for 81,920 triangles, most of it on the FP64 pipe). Slots with no elements
+// get an empty slab.
+//
+// Every element contributes to the slot of each of its ancestors, so both passes (normals, then ranges) run one thread
+// per element, which climbs from its leaf's slot to the root. A warp's elements are neighbours in leaf order, hence
+// share nearly all of their ancestors: the lanes climb level by level together, the lanes under one slot (a contiguous
+// run) reduce with shuffles, and one lane per run issues the atomics. Work is n x depth spread evenly over the GPU.
+// (One block per slot over the slot's whole run left the four slots of the root, a quarter of the mesh each, to four
+// blocks: 646 us for 81,920 triangles, and 12 passes and three host synchronisations to find the runs; this form takes 54
+// in all, six launches. A rebuild of that mesh with 16,384 queries: 2.67 -> 1.96 ms.)
+//============================================================================================================================
+
+constexpr int SLAB_MAX_LEVEL = 254;
+
+// parent[i]: the slot (node * W + child) under which wide node i hangs; -2 - s for the root of segment s; -1 if none.
+// A node array that does not follow the build's layout (a child before its parent, or under two slots) sets *bad.
 template <int W>
-__global__ void subtree_range_kernel(WideNode<W> const * __restrict__ nodes, int64_t num_nodes, int64_t n,
-                                     int2 * __restrict__ range, int * __restrict__ changed, int * __restrict__ bad) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += (int64_t)gridDim.x * blockDim.x) {
-    if (range[i].y >= 0) continue;
-    int lo = INT_MAX, hi = -1;
-    bool ready = true;
+__global__ void slab_parent_kernel(WideNode<W> const * __restrict__ nodes, int64_t num_nodes, int * __restrict__ parent,
+                                   int * __restrict__ bad) {
+  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= num_nodes * W) return;
+  int code = nodes[k / W].child[k % W];
+  if (code < 0) return;  // a leaf or empty
+  if ((int64_t)code >= num_nodes || (int64_t)code <= k / W || atomicCAS(&parent[code], -1, (int)k) != -1)
+    atomicOr(bad, 1);
+}
+
+__global__ void slab_roots_kernel(int32_t const * __restrict__ seg_root, int M, int64_t num_nodes,
+                                  int * __restrict__ parent, int * __restrict__ bad) {
+  int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= M) return;
+  int r = seg_root[s];
+  if (r < 0 || (int64_t)r >= num_nodes || atomicCAS(&parent[r], -1, -2 - s) != -1) atomicOr(bad, 1);
+}
+
+// leaf_slot[k] / leaf_level[k]: the slot whose leaf holds the element at sorted position k, and its distance from the
+// root (the root's own slots are level 0). The climb to the root gives the segment, to which leaf codes are relative.
+template <int W>
+__global__ void slab_leaf_kernel(WideNode<W> const * __restrict__ nodes, int64_t num_nodes,
+                                 int const * __restrict__ parent, int64_t const * __restrict__ seg_start, int M,
+                                 int64_t n, int * __restrict__ leaf_slot, uint8_t * __restrict__ leaf_level,
+                                 int * __restrict__ bad) {
+  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= num_nodes * W) return;
+  int code = nodes[k / W].child[k % W];
+  if (code >= 0 || code == CHILD_EMPTY) return;
+  int level = 0;
+  int up = parent[k / W];
+  while (up >= 0 && level < SLAB_MAX_LEVEL) {
+    up = parent[up / W];
+    ++level;
+  }
+  if (up > -2 || -2 - up >= M) {
+    atomicOr(bad, 1);
+    return;
+  }
+  int64_t a = seg_start[-2 - up], b = seg_start[-1 - up];
+  int first, count;
+  decode_leaf(code, first, count);
+  if (a < 0 || b > n || first < 0 || a + first + count > b) {
+    atomicOr(bad, 1);
+    return;
+  }
+  for (int64_t e = a + first; e < a + first + count; ++e) {
+    if (atomicCAS(&leaf_slot[e], -1, (int)k) != -1) atomicOr(bad, 1);
+    leaf_level[e] = (uint8_t)level;
+  }
+}
+
+// Adds (or takes the minimum and maximum of) a float at x without a return value; fmin/fmax of floats of either sign
+// through their integer encodings, with *x starting at +inf (minimum) or -inf (maximum).
+__device__ __forceinline__ void atomic_min_float(float * x, float v) {
+  if (v >= 0.f) atomicMin(reinterpret_cast<int *>(x), __float_as_int(v));
+  else atomicMax(reinterpret_cast<unsigned *>(x), __float_as_uint(v));
+}
+__device__ __forceinline__ void atomic_max_float(float * x, float v) {
+  if (v >= 0.f) atomicMax(reinterpret_cast<int *>(x), __float_as_int(v));
+  else atomicMin(reinterpret_cast<unsigned *>(x), __float_as_uint(v));
+}
+
+// RANGE = false: sums of (normal * area) into slabs[slot].xyz. RANGE = true: the range of n . v into slabs[slot].zw.
+template <int W, bool RANGE>
+__global__ void __launch_bounds__(BUILD_THREADS)
+slab_climb_kernel(int64_t n, int const * __restrict__ leaf_slot, uint8_t const * __restrict__ leaf_level,
+                  int const * __restrict__ parent, float4 const * __restrict__ rec, float4 * slabs,
+                  int * __restrict__ bad) {
+  unsigned const FULL = 0xffffffffu;
+  int lane = threadIdx.x & 31;
+  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int slot = k < n ? leaf_slot[k] : -1;
+  if (k < n && slot < 0) atomicOr(bad, 1);  // an element under no leaf
+  int level = slot >= 0 ? leaf_level[k] : -1;
+  V3 v0 = V3{0.f, 0.f, 0.f}, v1 = v0, v2 = v0;  // RANGE: the vertices; else v0 = normal * area
+  if (slot >= 0) {
+    float4 const * r = rec + k * CP_REC_F4;
+    if constexpr (RANGE) {
+      v0 = xyz(__ldg(r));
+      v1 = xyz(__ldg(r + 1));
+      v2 = xyz(__ldg(r + 2));
+    } else {
+      V3 nn = xyz(__ldg(r + 3));
+      float area = __ldg(r + 6).w;
+      if (isfinite(nn.x) && isfinite(nn.y) && isfinite(nn.z) && isfinite(area)) v0 = nn * area;
+    }
+  }
+  int top = __reduce_max_sync(FULL, level);
+  for (int l = top; l >= 0; --l) {
+    bool on = slot >= 0 && level >= l;  // this lane's slot at level l
+    int run = on ? slot : -1 - lane;    // equal only among the lanes under one slot
+    float a = 0.f, b = 0.f, c = 0.f;
+    if constexpr (RANGE) {
+      a = INFINITY;
+      b = -INFINITY;
+      if (on) {
+        float2 enc = *reinterpret_cast<float2 const *>(slabs + slot);
+        V3 nv = slab_normal(make_float4(enc.x, enc.y, 0.f, 0.f));
+        // n . v in FP32 is within 3 * 2^-24 of m = sum |n_i v_i| of its value; 2^-21 m also covers the subtraction
+        V3 v[3] = {v0, v1, v2};
+        float m = 0.f;
+        bool finite = true;
+        a = INFINITY;
+        b = -INFINITY;
 #pragma unroll
-    for (int c = 0; c < W; ++c) {
-      int code = nodes[i].child[c];
-      if (code == CHILD_EMPTY) continue;
-      if (code < 0) {
-        int first, count;
-        decode_leaf(code, first, count);
-        if (first < 0 || count <= 0 || (int64_t)first + count > n) {
-          atomicOr(bad, 1);
-          ready = false;
-          break;
+        for (int j = 0; j < 3; ++j) {
+          float x = nv.x * v[j].x, y = nv.y * v[j].y, z = nv.z * v[j].z;
+          float d = x + y + z;
+          float mag = fabsf(x) + fabsf(y) + fabsf(z);
+          finite = finite && mag < INFINITY;
+          m = fmaxf(m, mag);
+          a = fminf(a, d);
+          b = fmaxf(b, d);
         }
-        lo = min(lo, first);
-        hi = max(hi, first + count);
-      } else {
-        if ((int64_t)code >= num_nodes || (int64_t)code <= i) {
-          atomicOr(bad, 1);
-          ready = false;
-          break;
+        m = m * (1.0f / 2097152.0f) + 1e-44f;  // (the constant: products below the normal range)
+        a -= m;
+        b += m;
+        if (!finite) a = -INFINITY, b = INFINITY;  // the slab bounds nothing
+      }
+    } else if (on) {
+      a = v0.x;
+      b = v0.y;
+      c = v0.z;
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int ro = __shfl_down_sync(FULL, run, o);
+      float ao = __shfl_down_sync(FULL, a, o), bo = __shfl_down_sync(FULL, b, o);
+      float co = RANGE ? 0.f : __shfl_down_sync(FULL, c, o);
+      if (lane + o < 32 && ro == run) {
+        if constexpr (RANGE) {
+          a = fminf(a, ao);
+          b = fmaxf(b, bo);
+        } else {
+          a += ao;
+          b += bo;
+          c += co;
         }
-        int2 r = range[code];
-        if (r.y < 0) {
-          ready = false;
-          continue;
-        }
-        lo = min(lo, r.x);
-        hi = max(hi, r.y);
       }
     }
-    if (!ready) continue;
-    range[i] = hi >= 0 ? make_int2(lo, hi) : make_int2(0, 0);
-    *changed = 1;
-  }
-}
-
-// Run of sorted element positions (first, count) under each child slot
-template <int W>
-__global__ void slot_range_kernel(WideNode<W> const * __restrict__ nodes, int64_t num_nodes,
-                                  int2 const * __restrict__ range, int2 * __restrict__ slot) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < num_nodes * W;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    int code = nodes[k / W].child[k % W];
-    int2 r = make_int2(0, 0);
-    if (code != CHILD_EMPTY && code < 0) {
-      int first, count;
-      decode_leaf(code, first, count);
-      r = make_int2(first, count);
-    } else if (code >= 0) {
-      int2 sub = range[code];
-      r = make_int2(sub.x, sub.y - sub.x);
+    int before = __shfl_up_sync(FULL, run, 1);
+    if (on && (lane == 0 || before != run)) {
+      float * out = reinterpret_cast<float *>(slabs + slot);
+      if constexpr (RANGE) {
+        atomic_min_float(out + 2, a);
+        atomic_max_float(out + 3, b);
+      } else {
+        atomicAdd(out, a);
+        atomicAdd(out + 1, b);
+        atomicAdd(out + 2, c);
+      }
     }
-    slot[k] = r;
+    if (on && l > 0) slot = parent[slot / W];
   }
 }
 
+// Summed normals -> encoded unit normal with an empty range
+__global__ void slab_normal_kernel(int64_t slots, float4 * __restrict__ slabs) {
+  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= slots) return;
+  float4 s = slabs[k];
+  float x = s.x, y = s.y, z = s.z;
+  float l = sqrtf(x * x + y * y + z * z);
+  if (!(l > 0.f) || !isfinite(l)) x = 0.f, y = 0.f, z = 1.f, l = 1.f;
+  float4 e = slab_encode(V3{x / l, y / l, z / l});
+  slabs[k] = make_float4(e.x, e.y, INFINITY, -INFINITY);
+}
+
 template <int W>
-bool slot_ranges(thea_bvh const * b, Scratch & slots, cudaStream_t stream) {
+static void build_slabs(thea_bvh * b, cudaStream_t stream) {
   WideNode<W> const * nodes = (WideNode<W> const *)b->nodes;
-  int64_t nn = b->num_nodes;
-  Scratch range((size_t)nn * sizeof(int2), stream), flags(2 * sizeof(int), stream);
-  THEA_CUDA_CHECK(cudaMemsetAsync(range.ptr, 0xff, range.bytes, stream));
-  THEA_CUDA_CHECK(cudaMemsetAsync(flags.ptr, 0, flags.bytes, stream));
-  unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nn, BUILD_THREADS), 152 * 8));
-  // every pass settles at least the deepest unsettled level; a pass that settles nothing ends the loop, and any node
-  // still unsettled then (or after the pass limit) means the array is not a tree of this build's layout
-  // Passes run four at a time between reads of the flags (a pass after the one that settled the last node changes
-  // nothing, so the extra passes are no-ops); the flags are those of the group's last pass, `bad` accumulates.
-  bool settled = false;
-  int limit = 2 * b->depth + 4;
-  int2 root = make_int2(-1, -1);
-  for (int pass = 0; pass < limit && !settled;) {
-    for (int k = 0; k < 4 && pass < limit; ++k, ++pass) {
-      THEA_CUDA_CHECK(cudaMemsetAsync(flags.ptr, 0, sizeof(int), stream));
-      THEA_LAUNCH(subtree_range_kernel<W>, grid, BUILD_THREADS, 0, stream, nodes, nn, b->n, range.as<int2>(),
-                  flags.as<int>(), flags.as<int>() + 1);
-    }
-    int h[2];
-    THEA_CUDA_CHECK(cudaMemcpyAsync(h, flags.ptr, sizeof(h), cudaMemcpyDeviceToHost, stream));
-    THEA_CUDA_CHECK(cudaMemcpyAsync(&root, range.ptr, sizeof(root), cudaMemcpyDeviceToHost, stream));
-    THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
-    if (h[1]) return false;
-    settled = !h[0];
+  int64_t nn = b->num_nodes, slots = nn * W, n = b->n;
+  int M = b->num_segments;
+  Scratch parent((size_t)nn * sizeof(int), stream), leaf_slot((size_t)n * sizeof(int), stream);
+  Scratch leaf_level((size_t)n, stream), bad(sizeof(int), stream);
+  THEA_CUDA_CHECK(cudaMemsetAsync(parent.ptr, 0xff, parent.bytes, stream));
+  THEA_CUDA_CHECK(cudaMemsetAsync(leaf_slot.ptr, 0xff, leaf_slot.bytes, stream));
+  THEA_CUDA_CHECK(cudaMemsetAsync(bad.ptr, 0, sizeof(int), stream));
+  THEA_CUDA_CHECK(thea_malloc_async((void **)&b->slabs, (size_t)slots * sizeof(float4), stream));
+  THEA_CUDA_CHECK(cudaMemsetAsync(b->slabs, 0, (size_t)slots * sizeof(float4), stream));
+  unsigned sgrid = (unsigned)ceil_div(slots, BUILD_THREADS), egrid = (unsigned)ceil_div(n, BUILD_THREADS);
+  THEA_LAUNCH(slab_roots_kernel, (unsigned)ceil_div(M, BUILD_THREADS), BUILD_THREADS, 0, stream, b->seg_root, M, nn,
+              parent.as<int>(), bad.as<int>());
+  THEA_LAUNCH(slab_parent_kernel<W>, sgrid, BUILD_THREADS, 0, stream, nodes, nn, parent.as<int>(), bad.as<int>());
+  THEA_LAUNCH(slab_leaf_kernel<W>, sgrid, BUILD_THREADS, 0, stream, nodes, nn, parent.as<int>(), b->seg_start, M, n,
+              leaf_slot.as<int>(), leaf_level.as<uint8_t>(), bad.as<int>());
+  THEA_LAUNCH((slab_climb_kernel<W, false>), egrid, BUILD_THREADS, 0, stream, n, leaf_slot.as<int>(),
+              leaf_level.as<uint8_t>(), parent.as<int>(), b->cp_rec, b->slabs, bad.as<int>());
+  THEA_LAUNCH(slab_normal_kernel, sgrid, BUILD_THREADS, 0, stream, slots, b->slabs);
+  THEA_LAUNCH((slab_climb_kernel<W, true>), egrid, BUILD_THREADS, 0, stream, n, leaf_slot.as<int>(),
+              leaf_level.as<uint8_t>(), parent.as<int>(), b->cp_rec, b->slabs, bad.as<int>());
+  int h = 0;
+  THEA_CUDA_CHECK(cudaMemcpyAsync(&h, bad.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if (h) {
+    cudaFree(b->slabs);
+    b->slabs = nullptr;  // searches use boxes alone
   }
-  if (!settled) return false;
-  // the root (node 0) must cover every element once settled
-  if (root.x != 0 || (int64_t)root.y != b->n) return false;
-  slots = Scratch((size_t)nn * W * sizeof(int2), stream);
-  unsigned sgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nn * W, BUILD_THREADS), 152 * 8));
-  THEA_LAUNCH(slot_range_kernel<W>, sgrid, BUILD_THREADS, 0, stream, nodes, nn, range.as<int2>(), slots.as<int2>());
-  return true;
 }
 
 // Oriented slabs go with single-mesh BVHs that have the closest layout: they shorten the longest searches of the
-// one-query-per-thread kernels (small batches, serving), whose warps wait for their slowest lane. The persistent
-// batched kernels, which refill a lane as soon as its query ends, ran faster with boxes alone, so forests have none.
+// one-query-per-thread kernels (small batches, serving), whose warps wait for their slowest lane, and of the
+// warp-per-query kernel. The persistent batched kernels, which refill a lane as soon as its query ends, ran faster with
+// boxes alone, so forests have none (with them in the second phase alone, 256 meshes of 320 to 327,680 triangles with
+// 5.2 M queries: 12.4 -> 12.0 ms, for a build of 25 -> 29 ms).
 void init_slabs(thea_bvh * b, cudaStream_t stream) {
   if (!b->is_mesh || b->num_segments != 1 || !b->cp_rec || b->slabs) return;
-  Scratch slots;
-  bool ok = b->width == 4 ? slot_ranges<4>(b, slots, stream) : slot_ranges<8>(b, slots, stream);
-  if (!ok) return;  // searches use boxes alone
-  int64_t n_slots = b->num_nodes * b->width;
-  THEA_CUDA_CHECK(thea_malloc_async((void **)&b->slabs, (size_t)n_slots * sizeof(float4), stream));
-  unsigned grid = (unsigned)std::min<int64_t>(n_slots, (int64_t)sm_count() * 16);
-  THEA_LAUNCH(slab_kernel, grid, SLAB_THREADS, 0, stream, slots.as<int2>(), n_slots, b->cp_rec, b->slabs);
-  THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if (b->num_nodes * b->width >= (int64_t(1) << 31)) return;  // slots are addressed with 31 bits
+  if (b->width == 4) build_slabs<4>(b, stream);
+  else build_slabs<8>(b, stream);
 }
 
 void init_segment_roots(thea_bvh * b, cudaStream_t stream) {
