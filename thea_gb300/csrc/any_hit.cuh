@@ -50,11 +50,15 @@ any_hit_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict
   int64_t qb = 0, qe = 0;  // warp-local block of ray ids, warp-uniform
   bool exhausted = false;  // warp-uniform
   int64_t q = -1;          // this lane's ray (-1: idle)
-  V3 o = V3{0.f, 0.f, 0.f}, d = V3{0.f, 0.f, 1.f};
-  float ix = 0.f, iy = 0.f, iz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f;
+  RayState ray;
+  ray_setup(ray, V3{0.f, 0.f, 0.f}, V3{0.f, 0.f, 1.f});
   float const bound = max_time >= 0.f ? max_time : INFINITY;
-  bool hit = false;
-  int2 stk[STACK];
+  // the first-hit step; any element it accepts ends the search (TriangleN<3>::rayIntersection: a hit at t >= 0, and
+  // t <= max_time when bounded)
+  float best = 0.f;
+  int best_idx = INT_MAX;
+  int64_t best_slot = -1;
+  LocalStack<STACK> stk;
   int sp = 0;
   int next = CHILD_EMPTY;
   while (true) {
@@ -74,14 +78,11 @@ any_hit_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict
         int64_t avail = qe - qb;
         if (q < 0 && rank < avail) {
           q = qb + rank;
+          V3 o, d;
           src.get(q, o, d);
-          ix = 1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x));
-          iy = 1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y));
-          iz = 1.0f / (fabsf(d.z) > 1e-30f ? d.z : copysignf(1e-30f, d.z));
-          ox = -o.x * ix;
-          oy = -o.y * iy;
-          oz = -o.z * iz;
-          hit = false;
+          ray_setup(ray, o, d);
+          best = bound;
+          best_idx = INT_MAX;
           sp = 0;
           next = 0;
         }
@@ -91,40 +92,14 @@ any_hit_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict
     if (__ballot_sync(FULL, q >= 0) == 0) break;
     if (q < 0) continue;
     int code = next;
+    bool hit = best_idx != INT_MAX;
     if (hit || (code == CHILD_EMPTY && sp == 0)) {
       sink.put(q, hit);
       q = -1;
       continue;
     }
-    if (code == CHILD_EMPTY) code = stk[--sp].x;  // entries were pushed within the fixed bound
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-#pragma unroll
-      for (int c = 0; c < W; ++c) {
-        float tx0 = __fmaf_rn(nd.lox[c], ix, ox), tx1 = __fmaf_rn(nd.hix[c], ix, ox);
-        float ty0 = __fmaf_rn(nd.loy[c], iy, oy), ty1 = __fmaf_rn(nd.hiy[c], iy, oy);
-        float tz0 = __fmaf_rn(nd.loz[c], iz, oz), tz1 = __fmaf_rn(nd.hiz[c], iz, oz);
-        float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.f));
-        float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
-        lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);  // a miss: NaN passes no bound
-      }
-      push_children_next<W, STACK>(nd, lb, bound * PRUNE_SLACK, stk, sp, next, err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      for (int64_t k = first; k < first + count; ++k) {
-        float4 const * r = rec + k * RAY_REC_F4;
-        float t = ray_triangle_time(o, d, xyz(__ldg(r)), xyz(__ldg(r + 1)), xyz(__ldg(r + 2)));
-        // TriangleN<3>::rayIntersection: a hit at t >= 0, and t <= max_time when bounded
-        if (t >= 0.f && t <= bound) {
-          hit = true;
-          break;
-        }
-      }
-    }
+    if (code == CHILD_EMPTY) code = stk.get(--sp).x;  // entries were pushed within the fixed bound
+    ray_step<W>(nodes, rec, 0, code, ray, best, best_idx, best_slot, stk, sp, next, err);
   }
 }
 

@@ -167,42 +167,37 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
 // Persistent-lane form of batch_closest_kernel: each lane takes a new query as soon as its query is done, instead of
 // idling until the slowest query of its warp's round (the queries deep inside a mesh take ten times the steps of the
 // others). Every loop iteration advances each busy lane by one stack entry; idle lanes are refilled from a warp-local
-// block of 64 query indices. In the mixed-precision mode a lane whose traversal is done waits, its band entries kept,
-// until 8 lanes of its warp are waiting (or nothing else is left), and the warp then evaluates all their entries in FP64
-// together (f64_resolve_warp). Results are the round-based kernel's: each query's search is the same sequence of steps.
+// block of 64 query indices. FP32 search only (the mixed-precision search is bound by the FP64 pipe, and rounds of 32
+// queries fill its FP64 step better: 25.7 against 27.5 ms on 256 meshes). Results are the round-based kernel's: each
+// query's search is the same sequence of steps. What bounds it: the L1 data pipe (65 % busy) and the latency of the node
+// and record loads (a third of the lanes active: a warp mixes lanes at nodes, at leaves and between queries). One
+// 128-byte line per lane and step through 32-byte loads, issued before node and leaf lanes part ways (closest_step), and
+// the first 24 stack entries in shared memory (SharedStack): 262,144 queries on 81,920 triangles 1.41 -> 1.13 ms, 256
+// meshes with 5.2 M queries 12.4 -> 9.85 ms. Blocks of 16 or 32 indices: within 3 % of 64. A lower step budget once the
+// indices run out: slower (1.27 -> 1.74 ms at 128). Queries in Morton order: 1.18 -> 1.21 ms before the sort's own time.
 constexpr int REFILL_BLOCK = 64;
-constexpr int REFILL_RESOLVE_AT = 8;
 
-template <int W, int STACK, int PREC>
+template <int W, int STACK>
 __global__ void __launch_bounds__(BATCH_THREADS)
 batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long long * counter, int budget,
                             HardQueue hq) {
-  F64WarpBuf * buf = nullptr;
-  if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-    __shared__ F64WarpBuf s_buf[BATCH_THREADS / 32];
-    buf = &s_buf[threadIdx.x >> 5];
-  }
   unsigned const FULL = 0xffffffffu;
   int lane = threadIdx.x & 31;
   WideNode<W> const * nodes = (WideNode<W> const *)f.nodes;
   int64_t qb = 0, qe = 0;  // warp-local block of query indices, warp-uniform
   bool exhausted = false;  // warp-uniform
   int64_t q = -1;          // this lane's query (-1: idle)
-  bool pending = false;    // mixed precision: traversal done, waiting for the warp's FP64 step
   int64_t ebase = 0;
   V3 p = V3{0.f, 0.f, 0.f};
-  int2 stk[STACK];  // (child code, bound bits)
+  __shared__ int2 s_stk[CLOSEST_SHARED_STACK][BATCH_THREADS];
+  SharedStack<STACK, CLOSEST_SHARED_STACK, BATCH_THREADS> stk(s_stk);
   int sp = 0;
   int next = CHILD_EMPTY;  // nearest child of the last node, visited next without a stack round trip
-  float best = 0.f;  // FP32 mode: best squared distance; mixed mode: band limit
+  float best = 0.f;  // best squared distance
   int best_idx = INT_MAX;
   int64_t best_slot = -1;
   V3 best_cp = V3{0.f, 0.f, 0.f};
-  F64Search s;
-  float best32 = INFINITY, abs_tol = 0.f;
   int pops = 0;  // stack entries taken by this lane's query (two-phase form: budget > 0)
-  double bound2 = a.bound2;  // this lane's mesh's FP64 bound
-  if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) f64_search_init(s);
   while (true) {
     unsigned idle = __ballot_sync(FULL, q < 0);
     if (idle && !exhausted) {
@@ -226,48 +221,19 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
           sp = 0;
           next = __ldg(f.seg_root + m);
           pops = 0;
-          bound2 = bound2_of(a, m);
-          if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-            f64_search_init(s);
-            float scale = fmaxf(a.scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
-            best = f64_band_start(bound2, scale, abs_tol);
-            best32 = INFINITY;
-          } else {
-            best = thresh_of(a, m);
-            best_idx = INT_MAX;
-            best_slot = -1;
-          }
+          best = thresh_of(a, m);
+          best_idx = INT_MAX;
+          best_slot = -1;
         }
         qb += take < avail ? take : avail;
       }
     }
-    if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-      unsigned pend = __ballot_sync(FULL, pending);
-      unsigned trav = __ballot_sync(FULL, q >= 0 && !pending);
-      if (pend && (__popc(pend) >= REFILL_RESOLVE_AT || trav == 0)) {
-        f64_resolve_warp(s, pending, f.cp_rec, ebase, p, bound2, *buf);
-        if (pending) {
-          ClosestOut r = f64_result(s);
-          write_closest(q, r.idx != INT_MAX, (float)sqrt(r.d2_64), r.cp, r.idx, r.d2_64, a.out_index, a.out_dist,
-                        a.out_cp, a.out_err);
-          q = -1;
-          pending = false;
-        }
-        continue;
-      }
-    }
     if (__ballot_sync(FULL, q >= 0) == 0) break;
-    if (q < 0 || pending) continue;
+    if (q < 0) continue;
     if (next == CHILD_EMPTY && sp == 0) {
-      if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-        s.lim = best;
-        s.best32 = best32;
-        pending = true;
-      } else {
-        write_closest(q, best_idx != INT_MAX, sqrtf(best), best_cp, best_idx, 0.0, a.out_index, a.out_dist, a.out_cp,
-                      nullptr);
-        q = -1;
-      }
+      write_closest(q, best_idx != INT_MAX, sqrtf(best), best_cp, best_idx, 0.0, a.out_index, a.out_dist, a.out_cp,
+                    nullptr);
+      q = -1;
       continue;
     }
     if (budget > 0 && ++pops > budget) {
@@ -275,39 +241,21 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
       // by a warp of its own in the second kernel
       unsigned long long pos = atomicAdd(hq.count, 1ull);
       hq.q[pos] = q;
-      if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-        hq.bound[pos] = best32;
-        hq.idx[pos] = INT_MAX;
-        hq.slot[pos] = -1;
-      } else {
-        hq.bound[pos] = best;
-        hq.idx[pos] = best_idx;
-        hq.slot[pos] = best_slot;
-      }
+      hq.bound[pos] = best;
+      hq.idx[pos] = best_idx;
+      hq.slot[pos] = best_slot;
       q = -1;
       continue;
     }
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-      point_child_bounds<W>(nd, p, lb);
-      push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, f.err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      if constexpr (PREC == THEA_PRECISION_FP64_RECHECK)
-        cp_leaf_f64(f.cp_rec, ebase, first, count, p, bound2, abs_tol, best, best32, s);
-      else
-        cp_leaf_fp32(f.cp_rec, ebase, first, count, p, best, best_idx, best_slot, best_cp);
-    }
+    closest_step<W>(nodes, f.cp_rec, ebase, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, f.err, nullptr,
+                    0.f);
   }
 }
 
@@ -405,7 +353,8 @@ closest_stream_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lo
   int slot = 0;
   int64_t qbase = 0;
   V3 p = V3{0.f, 0.f, 0.f};
-  int2 stk[STACK];
+  __shared__ int2 s_stk[CLOSEST_SHARED_STACK][BATCH_THREADS];
+  SharedStack<STACK, CLOSEST_SHARED_STACK, BATCH_THREADS> stk(s_stk);
   int sp = 0;
   int next = CHILD_EMPTY;
   float best = 0.f;
@@ -503,21 +452,12 @@ closest_stream_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lo
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-      point_child_bounds<W>(nd, p, lb);
-      push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, f.err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      cp_leaf_fp32(f.cp_rec, 0, first, count, p, best, best_idx, best_slot, best_cp);
-    }
+    closest_step<W>(nodes, f.cp_rec, 0, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, f.err, nullptr,
+                           0.f);
   }
 }
 
@@ -602,29 +542,22 @@ template <int W, int STACK, int PREC>
 void launch_closest_prec(BatchForest const & f, ClosestArgs const & a, int64_t nq, int budget,
                          unsigned long long * counters, int chunk, HardQueue const & hq, cudaStream_t s) {
   auto k1 = batch_closest_kernel<W, STACK, PREC>;
+  int phase1_budget = budget > 0 ? budget : 0;
+  char const * name = budget > 0                             ? "batch_closest_phase1_kernel"
+                      : PREC == THEA_PRECISION_FP64_RECHECK ? "batch_closest_kernel_fp64"
+                                                            : "batch_closest_kernel_fp32";
   // FP32 without error estimates: persistent lanes (1.5x on the 256-mesh case), also as the first phase of the
-  // two-phase form. The mixed-precision search stays on rounds: it is bound by the FP64 pipe, and rounds fill the FP64
-  // step better (27.5 against 25.7 ms measured).
+  // two-phase form
   bool refill = PREC != THEA_PRECISION_FP64_RECHECK && !a.out_err;
-  if (budget <= 0) {
-    if (refill) {
-      auto kr = batch_closest_refill_kernel<W, STACK, PREC>;
-      THEA_LAUNCH_NAMED("batch_closest_kernel_fp32", kr, persistent_grid((void const *)kr), BATCH_THREADS, 0, s, f, a,
-                        nq, counters, 0, hq);
-      return;
-    }
-    THEA_LAUNCH_NAMED(PREC == THEA_PRECISION_FP64_RECHECK ? "batch_closest_kernel_fp64" : "batch_closest_kernel_fp32",
-                      k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk, 0, hq);
-    return;
-  }
   if (refill) {
-    auto kr = batch_closest_refill_kernel<W, STACK, PREC>;
-    THEA_LAUNCH_NAMED("batch_closest_phase1_kernel", kr, persistent_grid((void const *)kr), BATCH_THREADS, 0, s, f, a,
-                      nq, counters, budget, hq);
+    auto kr = batch_closest_refill_kernel<W, STACK>;
+    THEA_LAUNCH_NAMED(name, kr, persistent_grid((void const *)kr), BATCH_THREADS, 0, s, f, a, nq, counters,
+                      phase1_budget, hq);
   } else {
-    THEA_LAUNCH_NAMED("batch_closest_phase1_kernel", k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a,
-                      nq, counters, chunk, budget, hq);
+    THEA_LAUNCH_NAMED(name, k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk,
+                      phase1_budget, hq);
   }
+  if (budget <= 0) return;
   auto k2 = batch_closest_phase2_kernel<W, PREC>;
   THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, persistent_grid((void const *)k2), BATCH_THREADS, 0, s, f, a, hq,
                     counters + 1);

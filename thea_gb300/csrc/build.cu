@@ -780,7 +780,8 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
         rec_bytes += n * CP_REC_F4 * (int64_t)sizeof(float4);
       }
       if (layouts & THEA_LAYOUT_RAY) {
-        THEA_CUDA_CHECK(thea_malloc_async((void **)&b->ray_rec, (size_t)n * RAY_REC_F4 * sizeof(float4), stream));
+        THEA_CUDA_CHECK(thea_malloc_async((void **)&b->ray_rec, (size_t)n * RAY_REC_F4 * sizeof(float4) + RAY_REC_PAD,
+                                          stream));
         rec_bytes += n * RAY_REC_F4 * (int64_t)sizeof(float4);
       }
       THEA_LAUNCH(mesh_records_kernel, grid, BUILD_THREADS, 0, stream, V, F, n, seg, M, vals.as<uint32_t>(),

@@ -233,6 +233,8 @@ __device__ __forceinline__ float ray_triangle_time(V3 origin, V3 dir, V3 v0, V3 
 constexpr int CP_REC_F4 = 8;
 // Ray record: 3 x float4 = 48 bytes: (v0, original index bits), (e01, 0), (e02, 0)
 constexpr int RAY_REC_F4 = 3;
+// bytes allocated past the last ray record: the searches read records with 32-byte loads, two of them half a load apart
+constexpr int RAY_REC_PAD = 32;
 // Point record: 1 x float4 = 16 bytes: (p, original index bits)
 
 //============================================================================================================================
@@ -255,7 +257,7 @@ __host__ __device__ __forceinline__ void decode_leaf(int code, int & first, int 
   count = (v & (MAX_LEAF_SIZE - 1)) + 1;
 }
 
-template <int W> struct alignas(16) WideNode {
+template <int W> struct alignas(32) WideNode {
   float lox[W], hix[W], loy[W], hiy[W], loz[W], hiz[W];
   int child[W];
   int pad[W == 4 ? 4 : 8];  // 128 bytes for W = 4, 256 bytes for W = 8

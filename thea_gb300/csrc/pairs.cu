@@ -419,15 +419,16 @@ __global__ void __launch_bounds__(PAIR_THREADS) mesh_pair_kernel(
   float best = thresh;
   int best_t = INT_MAX;
   int64_t best_slot = -1;
-  int2 stk[STACK];
+  LocalStack<STACK> stk;
   int sp = 0, next = 0;
   while (next != CHILD_EMPTY || sp > 0) {
     float lim = fminf(best, key_d2(*(volatile unsigned long long *)best_key)) * PRUNE_SLACK;
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > lim) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > lim) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) mesh_pair_kernel(
 #pragma unroll
       for (int c = 0; c < W; ++c)
         lb[c] = box_box_d2(nd.lox[c], nd.loy[c], nd.loz[c], nd.hix[c], nd.hiy[c], nd.hiz[c], qlo, qhi);
-      push_children_next<W, STACK>(nd, lb, lim, stk, sp, next, err);
+      push_children_next<W>(nd, lb, lim, stk, sp, next, err);
     } else {
       int first, count;
       decode_leaf(code, first, count);

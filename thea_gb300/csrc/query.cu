@@ -166,7 +166,11 @@ ray_recheck_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __rest
 // same as ray_kernel's: each ray's traversal is the same sequence of steps. (Measured on the 2 M-triangle heightfield:
 // skipping pruned entries in an inner loop, or postponing leaves so that node steps run converged, were both slower,
 // since a lane's extra steps then stall its whole warp; keeping the nearest child in a register and packing stack
-// entries into 8 bytes gained 4.5 %.)
+// entries into 8 bytes gained 4.5 %.) What bounds it: the L1 data pipe (81 % of its peak with 16-byte loads inside the
+// node and leaf branches, each lane's line a wavefront per load) and the latency of those loads. Node or leaf read
+// through one set of 32-byte loads (ray_step) and the first 16 stack entries in shared memory: 4.2 M rays on 2.1 M
+// triangles 1.011 -> 0.871 ms; from pinned host arrays (ray_stream_kernel, seven blocks per SM: eight would spill) 1.130
+// -> 1.006 ms.
 constexpr int RAY_WARP_BLOCK = 64;
 constexpr int64_t RAY_PERSISTENT_MIN = 1 << 16;
 
@@ -182,13 +186,13 @@ ray_persistent_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __r
   int64_t qb = 0, qe = 0;  // warp-local block of ray ids [qb, qe), warp-uniform
   bool exhausted = false;  // warp-uniform
   int64_t q = -1;          // this lane's ray (-1: idle)
-  V3 o = V3{0.f, 0.f, 0.f};
-  float ix = 0.f, iy = 0.f, iz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f;
-  V3 d = V3{0.f, 0.f, 1.f};
+  RayState ray;
+  ray_setup(ray, V3{0.f, 0.f, 0.f}, V3{0.f, 0.f, 1.f});
   float best = 0.f;
   int best_idx = INT_MAX;
   int64_t best_slot = -1;
-  int2 stk[STACK];  // (child code, bit pattern of its entry-time lower bound): one 8-byte access per push and pop
+  __shared__ int2 s_stk[RAY_SHARED_STACK][QUERY_THREADS];
+  SharedStack<STACK, RAY_SHARED_STACK, QUERY_THREADS> stk(s_stk);
   int sp = 0;
   int next = CHILD_EMPTY;  // the nearest child of the last node: visited next without a stack round trip
   while (true) {
@@ -210,14 +214,7 @@ ray_persistent_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __r
           q = qb + rank;
           int64_t r = order ? (int64_t)order[q] : q;
           q = r;
-          o = load_v3(origins + 3 * r);
-          d = load_v3(dirs + 3 * r);
-          ix = 1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x));
-          iy = 1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y));
-          iz = 1.0f / (fabsf(d.z) > 1e-30f ? d.z : copysignf(1e-30f, d.z));
-          ox = -o.x * ix;
-          oy = -o.y * iy;
-          oz = -o.z * iz;
+          ray_setup(ray, load_v3(origins + 3 * r), load_v3(dirs + 3 * r));
           best = max_time >= 0.f ? max_time : INFINITY;
           best_idx = INT_MAX;
           best_slot = -1;
@@ -250,40 +247,11 @@ ray_persistent_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __r
         continue;
       }
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-#pragma unroll
-      for (int c = 0; c < W; ++c) {
-        float tx0 = __fmaf_rn(nd.lox[c], ix, ox), tx1 = __fmaf_rn(nd.hix[c], ix, ox);
-        float ty0 = __fmaf_rn(nd.loy[c], iy, oy), ty1 = __fmaf_rn(nd.hiy[c], iy, oy);
-        float tz0 = __fmaf_rn(nd.loz[c], iz, oz), tz1 = __fmaf_rn(nd.hiz[c], iz, oz);
-        float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.f));
-        float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
-        lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);  // a miss: NaN passes no bound
-      }
-      // nearest child next (it would be on top of the stack), the others pushed farthest first
-      push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      for (int64_t k = first; k < first + count; ++k) {
-        float4 const * r = rec + k * RAY_REC_F4;
-        float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-        float t = ray_triangle_time(o, d, xyz(a), xyz(b), xyz(c));
-        int idx = __float_as_int(a.w);
-        if (t >= 0.f && t <= best && (t < best || idx < best_idx)) {
-          best = t;
-          best_idx = idx;
-          best_slot = k;
-        }
-      }
-    }
+    ray_step<W>(nodes, rec, 0, code, ray, best, best_idx, best_slot, stk, sp, next, err);
   }
 }
 
@@ -299,7 +267,7 @@ constexpr int STREAM_RING = 4;
 constexpr int STREAM_WARPS = QUERY_THREADS / 32;
 
 template <int W, int STACK>
-__global__ void __launch_bounds__(QUERY_THREADS)
+__global__ void __launch_bounds__(QUERY_THREADS, 7)
 ray_stream_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
                   float const * __restrict__ origins, float const * __restrict__ dirs, int64_t n, float max_time,
                   float * __restrict__ out_time, int32_t * __restrict__ out_index, unsigned * __restrict__ err,
@@ -320,12 +288,13 @@ ray_stream_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restr
   int64_t q = -1;           // this lane's ray (-1: idle)
   int slot = 0;             // ring slot of this lane's ray
   int64_t qbase = 0;        // first ray of that slot's block
-  V3 o = V3{0.f, 0.f, 0.f};
-  float ix = 0.f, iy = 0.f, iz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f;
-  V3 d = V3{0.f, 0.f, 1.f};
+  RayState ray;
+  ray_setup(ray, V3{0.f, 0.f, 0.f}, V3{0.f, 0.f, 1.f});
   float best = 0.f;
   int best_idx = INT_MAX;
-  int2 stk[STACK];
+  int64_t best_slot = -1;  // (not an output here)
+  __shared__ int2 s_stk[RAY_SHARED_STACK][QUERY_THREADS];
+  SharedStack<STACK, RAY_SHARED_STACK, QUERY_THREADS> stk(s_stk);
   int sp = 0;
   int next = CHILD_EMPTY;
   while (true) {
@@ -378,14 +347,7 @@ ray_stream_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restr
           slot = (int)((taken - 1) % STREAM_RING);
           qbase = s_base[warp][slot];
           float const * r = in + (q - qbase) * 6;
-          o = V3{r[0], r[1], r[2]};
-          d = V3{r[3], r[4], r[5]};
-          ix = 1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x));
-          iy = 1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y));
-          iz = 1.0f / (fabsf(d.z) > 1e-30f ? d.z : copysignf(1e-30f, d.z));
-          ox = -o.x * ix;
-          oy = -o.y * iy;
-          oz = -o.z * iz;
+          ray_setup(ray, V3{r[0], r[1], r[2]}, V3{r[3], r[4], r[5]});
           best = max_time >= 0.f ? max_time : INFINITY;
           best_idx = INT_MAX;
           sp = 0;
@@ -412,38 +374,11 @@ ray_stream_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restr
         continue;
       }
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-#pragma unroll
-      for (int c = 0; c < W; ++c) {
-        float tx0 = __fmaf_rn(nd.lox[c], ix, ox), tx1 = __fmaf_rn(nd.hix[c], ix, ox);
-        float ty0 = __fmaf_rn(nd.loy[c], iy, oy), ty1 = __fmaf_rn(nd.hiy[c], iy, oy);
-        float tz0 = __fmaf_rn(nd.loz[c], iz, oz), tz1 = __fmaf_rn(nd.hiz[c], iz, oz);
-        float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.f));
-        float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
-        lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);
-      }
-      push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      for (int64_t k = first; k < first + count; ++k) {
-        float4 const * r = rec + k * RAY_REC_F4;
-        float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-        float t = ray_triangle_time(o, d, xyz(a), xyz(b), xyz(c));
-        int idx = __float_as_int(a.w);
-        if (t >= 0.f && t <= best && (t < best || idx < best_idx)) {
-          best = t;
-          best_idx = idx;
-        }
-      }
-    }
+    ray_step<W>(nodes, rec, 0, code, ray, best, best_idx, best_slot, stk, sp, next, err);
   }
 }
 

@@ -135,7 +135,7 @@ thea_bvh * deserialize_bvh(void const * in, int64_t bytes, cudaStream_t s) {
     char const * p = (char const *)in + sizeof(h);
     auto h2d = [&](void ** dst, int64_t nbytes) {
       if (nbytes > 0) {
-        THEA_CUDA_CHECK(thea_malloc_async(dst, (size_t)nbytes, s));
+        THEA_CUDA_CHECK(thea_malloc_async(dst, (size_t)nbytes + RAY_REC_PAD, s));
         THEA_CUDA_CHECK(cudaMemcpyAsync(*dst, p, (size_t)nbytes, cudaMemcpyHostToDevice, s));
       }
       p += nbytes;

@@ -122,10 +122,25 @@ __device__ __forceinline__ double ray_triangle_watertight_f64(V3 fo, V3 fd, V3 f
 // Closest element
 //============================================================================================================================
 
+// Squared distance and closest point of a record held in registers (FP32, reference arithmetic)
+__device__ __forceinline__ float cp_record_eval(float4 const (&r)[8], V3 p, V3 & cp) {
+  V3 v0 = xyz(r[0]), v1 = xyz(r[1]), v2 = xyz(r[2]), nrm = xyz(r[3]);
+  // HyperplaneN::closestPoint: p - signedDistance(p) * normal, signedDistance = p . normal - dist
+  float sd = dot(p, nrm) - r[0].w;
+  V3 proj = p - sd * nrm;
+  if (point_inside_triangle(v0, v1, v2, __float_as_int(r[3].w), proj))
+    cp = proj;
+  else
+    cp = closest_on_perimeter(v0, v1, v2, xyz(r[4]), r[1].w, xyz(r[5]), r[2].w, xyz(r[6]), r[4].w, p);
+  return squared_norm(cp - p);
+}
+
 // Squared distance and closest point of the record at sorted position k (FP32, reference arithmetic)
 __device__ __forceinline__ float cp_record_test(float4 const * __restrict__ rec, int64_t k, V3 p, V3 & cp) {
   float4 const * r = rec + k * CP_REC_F4;
-  float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), nn = __ldg(r + 3);
+  float4 a, b, c, nn;
+  ldg8(r, a, b);
+  ldg8(r + 2, c, nn);
   V3 v0 = xyz(a), v1 = xyz(b), v2 = xyz(c), nrm = xyz(nn);
   // HyperplaneN::closestPoint: p - signedDistance(p) * normal, signedDistance = p . normal - dist
   float sd = dot(p, nrm) - a.w;
@@ -133,7 +148,9 @@ __device__ __forceinline__ float cp_record_test(float4 const * __restrict__ rec,
   if (point_inside_triangle(v0, v1, v2, __float_as_int(nn.w), proj)) {
     cp = proj;
   } else {
-    float4 e0 = __ldg(r + 4), e1 = __ldg(r + 5), e2 = __ldg(r + 6);
+    float4 e0, e1, e2, unused;
+    ldg8(r + 4, e0, e1);
+    ldg8(r + 6, e2, unused);
     cp = closest_on_perimeter(v0, v1, v2, xyz(e0), b.w, xyz(e1), c.w, xyz(e2), e0.w, p);
   }
   return squared_norm(cp - p);
@@ -263,9 +280,9 @@ struct ClosestOut {
 // order: the nearest is returned in `next` (the
 // next step visits it without a stack round trip) and the others are pushed farthest first as packed (code, bound bits)
 // entries, one 8-byte access each. `next` is CHILD_EMPTY when no child is kept.
-template <int W, int STACK>
+template <int W, class Stk>
 __device__ __forceinline__ void push_children_next(NodeRegs<W> const & nd, float const (&lb)[W], float lim,
-                                                   int2 (&stk)[STACK], int & sp, int & next, unsigned * err) {
+                                                   Stk & stk, int & sp, int & next, unsigned * err) {
   uint32_t key[W];
   int cc[W];
 #pragma unroll
@@ -276,11 +293,17 @@ __device__ __forceinline__ void push_children_next(NodeRegs<W> const & nd, float
   }
   sort_children<W>(key, cc);
   next = key[0] != 0xffffffffu ? cc[0] : CHILD_EMPTY;
+  if (sp + W - 1 <= Stk::FAST) {  // room for every child in the stack's first part: no test per push
+#pragma unroll
+    for (int c = W - 1; c >= 1; --c)
+      if (key[c] != 0xffffffffu) stk.set_fast(sp++, make_int2(cc[c], (int)key[c]));
+    return;
+  }
 #pragma unroll
   for (int c = W - 1; c >= 1; --c) {
     if (key[c] != 0xffffffffu) {
-      if (sp < STACK) {
-        stk[sp] = make_int2(cc[c], (int)key[c]);
+      if (sp < Stk::SIZE) {
+        stk.set(sp, make_int2(cc[c], (int)key[c]));
         ++sp;
       } else {
         atomicOr(err, ERR_STACK_OVERFLOW);
@@ -366,9 +389,9 @@ __device__ __forceinline__ void slab_child_bounds(NodeRegs<W> const & nd, float4
 
 // push_children_next with a visiting key apart from the pruning bound: the children whose bound passes `lim` are kept,
 // the one with the smallest key goes to `next`, the others are pushed with their bounds, largest key first.
-template <int W, int STACK>
+template <int W, class Stk>
 __device__ __forceinline__ void push_children_ordered(NodeRegs<W> const & nd, float const (&lb)[W],
-                                                      float const (&order)[W], float lim, int2 (&stk)[STACK], int & sp,
+                                                      float const (&order)[W], float lim, Stk & stk, int & sp,
                                                       int & next, unsigned * err) {
   uint32_t key[W];
   int slot[W];
@@ -387,7 +410,7 @@ __device__ __forceinline__ void push_children_ordered(NodeRegs<W> const & nd, fl
 #pragma unroll
   for (int c = W - 1; c >= 1; --c) {
     if (key[c] != 0xffffffffu) {
-      if (sp < STACK) {
+      if (sp < Stk::SIZE) {
         int code = CHILD_EMPTY;
         float bound = 0.f;
 #pragma unroll
@@ -395,7 +418,7 @@ __device__ __forceinline__ void push_children_ordered(NodeRegs<W> const & nd, fl
           code = u == slot[c] ? nd.child[u] : code;
           bound = u == slot[c] ? lb[u] : bound;
         }
-        stk[sp] = make_int2(code, __float_as_int(bound));
+        stk.set(sp, make_int2(code, __float_as_int(bound)));
         ++sp;
       } else {
         atomicOr(err, ERR_STACK_OVERFLOW);
@@ -424,6 +447,61 @@ __device__ __forceinline__ void cp_leaf_fp32(float4 const * __restrict__ rec, in
   }
 }
 
+// One step of the FP32 closest-element search at `code`: a node's children bounded (by box, and by slab where the BVH
+// has them) and pushed, or an element of a leaf tested (the rest of the leaf comes back in `next`). Some lanes of a warp
+// sit at a node and others at a leaf; a width-4 node and a record are one 128-byte line each and are read through one set
+// of loads before the lanes part ways, so a step waits for memory once (with the loads inside the two branches: for the
+// node lanes', then twice for each element of the leaf lanes).
+template <int W, class Stk>
+__device__ __forceinline__ void closest_step(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
+                                             int64_t elem_base, int code, V3 p, float & best, int & best_idx,
+                                             int64_t & best_slot, V3 & best_cp, Stk & stk, int & sp,
+                                             int & next, unsigned * err, float4 const * __restrict__ slabs, float q1) {
+  next = CHILD_EMPTY;
+  int first = 0, count = 0;
+  if (code < 0) decode_leaf(code, first, count);
+  auto children = [&](NodeRegs<W> const & nd) {
+    float lb[W];
+    point_child_bounds<W>(nd, p, lb);
+    if (slabs) {
+      float order[W];
+      slab_child_bounds<W>(nd, slabs, code, p, q1, lb, order);
+      push_children_ordered<W>(nd, lb, order, best * PRUNE_SLACK, stk, sp, next, err);
+    } else {
+      push_children_next<W>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
+    }
+  };
+  if constexpr (W == 4) {
+    int64_t k = elem_base + first;
+    float4 r[8];
+    load_line(code >= 0 ? reinterpret_cast<float4 const *>(nodes + code) : rec + k * CP_REC_F4, r);
+    if (code >= 0) {
+      NodeRegs<W> nd;
+      node_from_line(r, nd);
+      children(nd);
+    } else {
+      V3 cp;
+      float d2 = cp_record_eval(r, p, cp);
+      int idx = __float_as_int(r[5].w);
+      if (d2 <= best && (d2 < best || idx < best_idx)) {
+        best = d2;
+        best_idx = idx;
+        best_slot = k;
+        best_cp = cp;
+      }
+      if (count > 1) next = encode_leaf(first + 1, count - 1);
+    }
+  } else {
+    if (code >= 0) {
+      NodeRegs<W> nd;
+      load_node(nodes, code, nd);
+      children(nd);
+    } else {
+      cp_leaf_fp32(rec, elem_base, first, count, p, best, best_idx, best_slot, best_cp);
+    }
+  }
+}
+
 // FP32 reference-arithmetic search: smallest (d2, index), accepting d2 <= thresh. With budget > 0 the search stops
 // after that many stack pops (done = false), leaving the best found so far. With the BVH's oriented slabs (single
 // mesh BVHs) the children's bounds are raised to their slab bounds; the result is the same, the search shorter.
@@ -438,7 +516,7 @@ __device__ __forceinline__ ClosestOut closest_query(WideNode<W> const * __restri
   int best_idx = INT_MAX;
   int64_t best_slot = -1;
   V3 best_cp = V3{0.f, 0.f, 0.f};
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;  // nearest child of the last node, visited without a stack round trip
   int pops = 0;
@@ -450,27 +528,12 @@ __device__ __forceinline__ ClosestOut closest_query(WideNode<W> const * __restri
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-      point_child_bounds<W>(nd, p, lb);
-      if (slabs) {
-        float order[W];
-        slab_child_bounds<W>(nd, slabs, code, p, q1, lb, order);
-        push_children_ordered<W, STACK>(nd, lb, order, best * PRUNE_SLACK, stk, sp, next, err);
-      } else {
-        push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
-      }
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      cp_leaf_fp32(rec, elem_base, first, count, p, best, best_idx, best_slot, best_cp);
-    }
+    closest_step<W>(nodes, rec, elem_base, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, err, slabs,
+                           q1);
   }
   ClosestOut o;
   o.idx = best_idx;
@@ -607,7 +670,7 @@ __device__ __forceinline__ void closest_search_f64(WideNode<W> const * __restric
   float abs_tol;
   float lim = f64_band_start(bound2, scale, abs_tol);
   float best32 = INFINITY;
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;  // nearest child of the last node, visited without a stack round trip
   while (next != CHILD_EMPTY || sp > 0) {
@@ -618,8 +681,9 @@ __device__ __forceinline__ void closest_search_f64(WideNode<W> const * __restric
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > lim * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > lim * PRUNE_SLACK) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -630,9 +694,9 @@ __device__ __forceinline__ void closest_search_f64(WideNode<W> const * __restric
       if (slabs) {
         float order[W];
         slab_child_bounds<W>(nd, slabs, code, p, q1, lb, order);
-        push_children_ordered<W, STACK>(nd, lb, order, lim * PRUNE_SLACK, stk, sp, next, err);
+        push_children_ordered<W>(nd, lb, order, lim * PRUNE_SLACK, stk, sp, next, err);
       } else {
-        push_children_next<W, STACK>(nd, lb, lim * PRUNE_SLACK, stk, sp, next, err);
+        push_children_next<W>(nd, lb, lim * PRUNE_SLACK, stk, sp, next, err);
       }
     } else {
       int first, count;
@@ -730,6 +794,95 @@ static __device__ __noinline__ double watertight_f64_call(V3 o, V3 d, float4 a, 
   return ray_triangle_watertight_f64(o, d, xyz(a), xyz(b), xyz(c));
 }
 
+// A ray with the reciprocal directions of its slab tests
+struct RayState {
+  V3 o, d;
+  float ix, iy, iz, ox, oy, oz;
+};
+
+__device__ __forceinline__ void ray_setup(RayState & r, V3 o, V3 d) {
+  r.o = o;
+  r.d = d;
+  r.ix = 1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x));
+  r.iy = 1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y));
+  r.iz = 1.0f / (fabsf(d.z) > 1e-30f ? d.z : copysignf(1e-30f, d.z));
+  r.ox = -o.x * r.ix;
+  r.oy = -o.y * r.iy;
+  r.oz = -o.z * r.iz;
+}
+
+// Entry-time lower bounds of a node's children (NaN for a miss: it passes no bound)
+template <int W>
+__device__ __forceinline__ void ray_child_bounds(NodeRegs<W> const & nd, RayState const & r, float (&lb)[W]) {
+#pragma unroll
+  for (int c = 0; c < W; ++c) {
+    float tx0 = __fmaf_rn(nd.lox[c], r.ix, r.ox), tx1 = __fmaf_rn(nd.hix[c], r.ix, r.ox);
+    float ty0 = __fmaf_rn(nd.loy[c], r.iy, r.oy), ty1 = __fmaf_rn(nd.hiy[c], r.iy, r.oy);
+    float tz0 = __fmaf_rn(nd.loz[c], r.iz, r.oz), tz1 = __fmaf_rn(nd.hiz[c], r.iz, r.oz);
+    float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.f));
+    float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
+    lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);
+  }
+}
+
+// One step of the first-hit search at `code`: a node's children bounded and pushed, or up to two elements of a leaf
+// tested (the rest of a larger leaf comes back in `next`). As in closest_step, a width-4 node and two ray records are
+// read through one set of loads before the lanes part ways.
+template <int W, class Stk>
+__device__ __forceinline__ void ray_step(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
+                                         int64_t elem_base, int code, RayState const & ray, float & best,
+                                         int & best_idx, int64_t & best_slot, Stk & stk, int & sp, int & next,
+                                         unsigned * err) {
+  auto take = [&](float4 a, float4 b, float4 c, int64_t k) {
+    float t = ray_triangle_time(ray.o, ray.d, xyz(a), xyz(b), xyz(c));
+    int idx = __float_as_int(a.w);
+    if (t >= 0.f && t <= best && (t < best || idx < best_idx)) {
+      best = t;
+      best_idx = idx;
+      best_slot = k;
+    }
+  };
+  next = CHILD_EMPTY;
+  int first = 0, count = 0;
+  if (code < 0) decode_leaf(code, first, count);
+  int64_t k = elem_base + first;
+  if constexpr (W == 4) {
+    // records are 48 bytes: an odd one starts half way through a 32-byte load
+    bool odd = code < 0 && (k & 1);
+    int need = code >= 0 ? 8 : 3 * (count > 1 ? 2 : 1) + (odd ? 1 : 0);  // float4s from src on
+    float4 const * src = code >= 0 ? reinterpret_cast<float4 const *>(nodes + code) : rec + (k * RAY_REC_F4 - (odd ? 1 : 0));
+    float4 r[8];
+    ldg8(src, r[0], r[1]);
+    ldg8(src + 2, r[2], r[3]);
+    if (need > 4) ldg8(src + 4, r[4], r[5]);
+    if (need > 6) ldg8(src + 6, r[6], r[7]);
+    if (code >= 0) {
+      NodeRegs<W> nd;
+      node_from_line(r, nd);
+      float lb[W];
+      ray_child_bounds<W>(nd, ray, lb);
+      push_children_next<W>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
+    } else {
+      take(odd ? r[1] : r[0], odd ? r[2] : r[1], odd ? r[3] : r[2], k);
+      if (count > 1) take(odd ? r[4] : r[3], odd ? r[5] : r[4], odd ? r[6] : r[5], k + 1);
+      if (count > 2) next = encode_leaf(first + 2, count - 2);
+    }
+  } else {
+    if (code >= 0) {
+      NodeRegs<W> nd;
+      load_node(nodes, code, nd);
+      float lb[W];
+      ray_child_bounds<W>(nd, ray, lb);
+      push_children_next<W>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
+    } else {
+      for (int64_t e = k; e < k + count; ++e) {
+        float4 const * r = rec + e * RAY_REC_F4;
+        take(__ldg(r), __ldg(r + 1), __ldg(r + 2), e);
+      }
+    }
+  }
+}
+
 // The reference's verdict: FP32 Eberly test with its parallel threshold (TriangleN<3>::rayIntersection), nearest hit
 // with t >= 0 and, with a bound, t <= max_time; ties to the lowest index. (The FP64 watertight verdict is
 // ray_search_f64 + ray_resolve_warp below.) The template flag is kept for the callers' signatures and must be false.
@@ -737,54 +890,23 @@ template <int W, int STACK, bool RECHECK>
 __device__ __forceinline__ RayOut ray_query(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
                                             int root, int64_t elem_base, V3 o, V3 d, float max_time, unsigned * err) {
   static_assert(!RECHECK, "the FP64 re-test is ray_search_f64 + ray_resolve_warp");
-  float ix = 1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x));
-  float iy = 1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y));
-  float iz = 1.0f / (fabsf(d.z) > 1e-30f ? d.z : copysignf(1e-30f, d.z));
-  float ox = -o.x * ix, oy = -o.y * iy, oz = -o.z * iz;
+  RayState ray;
+  ray_setup(ray, o, d);
   float best = max_time >= 0.f ? max_time : INFINITY;
   int best_idx = INT_MAX;
   int64_t best_slot = -1;
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;  // nearest child of the last node, visited without a stack round trip
   while (next != CHILD_EMPTY || sp > 0) {
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > best * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-#pragma unroll
-      for (int c = 0; c < W; ++c) {
-        float tx0 = __fmaf_rn(nd.lox[c], ix, ox), tx1 = __fmaf_rn(nd.hix[c], ix, ox);
-        float ty0 = __fmaf_rn(nd.loy[c], iy, oy), ty1 = __fmaf_rn(nd.hiy[c], iy, oy);
-        float tz0 = __fmaf_rn(nd.loz[c], iz, oz), tz1 = __fmaf_rn(nd.hiz[c], iz, oz);
-        float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.f));
-        float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
-        lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);  // a miss: NaN passes no bound
-      }
-      push_children_next<W, STACK>(nd, lb, best * PRUNE_SLACK, stk, sp, next, err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      int64_t k0 = elem_base + first;
-      for (int64_t k = k0; k < k0 + count; ++k) {
-        float4 const * r = rec + k * RAY_REC_F4;
-        float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
-        float t = ray_triangle_time(o, d, xyz(a), xyz(b), xyz(c));
-        int idx = __float_as_int(a.w);
-        if (t >= 0.f && t <= best && (t < best || idx < best_idx)) {
-          best = t;
-          best_idx = idx;
-          best_slot = k;
-        }
-      }
-    }
+    ray_step<W>(nodes, rec, elem_base, code, ray, best, best_idx, best_slot, stk, sp, next, err);
   }
   RayOut out;
   out.t = best;
@@ -865,7 +987,7 @@ __device__ __forceinline__ void ray_search_f64(WideNode<W> const * __restrict__ 
   float ox = -o.x * ix, oy = -o.y * iy, oz = -o.z * iz;
   float nd = l1(d);
   float dd = dot(d, d);
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;  // nearest child of the last node, visited without a stack round trip
   while (next != CHILD_EMPTY || sp > 0) {
@@ -874,8 +996,9 @@ __device__ __forceinline__ void ray_search_f64(WideNode<W> const * __restrict__ 
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > bound * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > bound * PRUNE_SLACK) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -891,7 +1014,7 @@ __device__ __forceinline__ void ray_search_f64(WideNode<W> const * __restrict__ 
         float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fmaxf(tz0, tz1));
         lb[c] = tmin <= tmax ? tmin : __int_as_float(0x7fffffff);  // a miss: NaN passes no bound
       }
-      push_children_next<W, STACK>(nd4, lb, bound * PRUNE_SLACK, stk, sp, next, err);
+      push_children_next<W>(nd4, lb, bound * PRUNE_SLACK, stk, sp, next, err);
       continue;
     }
     int first, count;
@@ -1063,15 +1186,16 @@ template <int W, int K, int STACK>
 __device__ __forceinline__ void knn_query(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ pts,
                                           int root, int64_t elem_base, V3 p, int excl, float (&bd)[K], int (&bi)[K],
                                           unsigned * err) {
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;  // nearest child of the last node, visited without a stack round trip
   while (next != CHILD_EMPTY || sp > 0) {
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > bd[K - 1] * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > bd[K - 1] * PRUNE_SLACK) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -1079,7 +1203,7 @@ __device__ __forceinline__ void knn_query(WideNode<W> const * __restrict__ nodes
       load_node(nodes, code, nd);
       float lb[W];
       point_child_bounds<W>(nd, p, lb);
-      push_children_next<W, STACK>(nd, lb, bd[K - 1] * PRUNE_SLACK, stk, sp, next, err);
+      push_children_next<W>(nd, lb, bd[K - 1] * PRUNE_SLACK, stk, sp, next, err);
     } else {
       int first, count;
       decode_leaf(code, first, count);
@@ -1106,15 +1230,16 @@ __device__ __forceinline__ void knn_search_shared(WideNode<W> const * __restrict
                                                   V3 p, int excl, float (*sd)[B], int (*si)[B], float & kth,
                                                   int & kth_i, unsigned * err, Elem elem) {
   int t = threadIdx.x;
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;
   while (next != CHILD_EMPTY || sp > 0) {
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > kth * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > kth * PRUNE_SLACK) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -1122,7 +1247,7 @@ __device__ __forceinline__ void knn_search_shared(WideNode<W> const * __restrict
       load_node(nodes, code, nd);
       float lb[W];
       point_child_bounds<W>(nd, p, lb);
-      push_children_next<W, STACK>(nd, lb, kth * PRUNE_SLACK, stk, sp, next, err);
+      push_children_next<W>(nd, lb, kth * PRUNE_SLACK, stk, sp, next, err);
     } else {
       int first, count;
       decode_leaf(code, first, count);
@@ -1188,15 +1313,16 @@ template <int W, int K, int STACK>
 __device__ __forceinline__ void knn_mesh_query(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
                                                int root, int64_t elem_base, V3 p, int excl, float (&bd)[K],
                                                int (&bi)[K], unsigned * err) {
-  int2 stk[STACK];  // (child code, bound bits)
+  LocalStack<STACK> stk;  // (child code, bound bits)
   int sp = 0;
   int next = root;
   while (next != CHILD_EMPTY || sp > 0) {
     int code = next;
     if (code == CHILD_EMPTY) {
       --sp;
-      code = stk[sp].x;
-      if (__int_as_float(stk[sp].y) > bd[K - 1] * PRUNE_SLACK) continue;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > bd[K - 1] * PRUNE_SLACK) continue;
     }
     next = CHILD_EMPTY;
     if (code >= 0) {
@@ -1204,7 +1330,7 @@ __device__ __forceinline__ void knn_mesh_query(WideNode<W> const * __restrict__ 
       load_node(nodes, code, nd);
       float lb[W];
       point_child_bounds<W>(nd, p, lb);
-      push_children_next<W, STACK>(nd, lb, bd[K - 1] * PRUNE_SLACK, stk, sp, next, err);
+      push_children_next<W>(nd, lb, bd[K - 1] * PRUNE_SLACK, stk, sp, next, err);
     } else {
       int first, count;
       decode_leaf(code, first, count);
