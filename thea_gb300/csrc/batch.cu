@@ -7,6 +7,7 @@
 // asynchronous and allocation-stable, so it can be captured once into a CUDA graph and replayed.
 #include "batch.hpp"
 #include "device_util.cuh"
+#include "knn_points.cuh"
 #include "traverse_ops.cuh"
 #include "warp_traverse.cuh"
 
@@ -482,7 +483,7 @@ batch_ray_kernel(BatchForest f, float const * __restrict__ origins, float const 
 }
 
 template <int W, int K, int STACK>
-__global__ void __launch_bounds__(BATCH_THREADS)
+__global__ void __launch_bounds__(BATCH_THREADS, K <= 16 ? 8 : 4)
 batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t const * __restrict__ qoff, int64_t nq,
                  int k_out, float thresh, int32_t * __restrict__ out_index, float * __restrict__ out_d2,
                  unsigned long long * counter, int chunk) {
@@ -492,41 +493,28 @@ batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t cons
     int64_t end = base + chunk < nq ? base + chunk : nq;
     for (int64_t q = base + (threadIdx.x & 31); q < end; q += 32) {
       int m = mesh_of_query(qoff, f.M, q);
-      float bd[K];
-      int bi[K];
+      int pad = K - k_out;
+      float start = thresh + 0.0f;  // (no negative zero)
+      bool any = start >= 0.f;      // a negative threshold admits nothing
+      uint64_t none = knn_key(any ? start : 0.f, INT_MAX);
+      auto entry = [&](int j) { return j < pad ? (uint64_t)0 : none; };
+      V3 p = load_v3(queries + 3 * q);
+      int root = __ldg(f.seg_root + m);
+      int64_t ebase = __ldg(f.seg_start + m);
+      uint64_t keys[K];
       if constexpr (K >= 8) {
-        // the K-best list in shared memory, as the point k-NN kernel keeps it (more warps resident)
-        __shared__ float s_d[K][BATCH_THREADS];
-        __shared__ int s_i[K][BATCH_THREADS];
-        int th = threadIdx.x;
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-          s_d[j][th] = thresh;
-          s_i[j][th] = INT_MAX;
-        }
-        float kth = thresh;
-        int kth_i = INT_MAX;
-        knn_query_shared<W, K, STACK, BATCH_THREADS>(nodes, f.pt_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m),
-                                                     load_v3(queries + 3 * q), -1, s_d, s_i, kth, kth_i, f.err);
-        // the row from shared memory
-        for (int j = 0; j < k_out; ++j) {
-          int bij = s_i[j][th];
-          bool v = bij != INT_MAX;
-          out_index[q * k_out + j] = v ? bij : -1;
-          out_d2[q * k_out + j] = v ? s_d[j][th] : -1.f;
-        }
-        continue;
+        __shared__ uint64_t s_list[K][BATCH_THREADS];
+        SharedKnnList<K, BATCH_THREADS> list(s_list);
+        list.init(entry);
+        if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
+        list.finish(keys);
       } else {
-#pragma unroll
-        for (int j = 0; j < K; ++j) { bd[j] = thresh; bi[j] = INT_MAX; }
-        knn_query<W, K, STACK>(nodes, f.pt_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m),
-                               load_v3(queries + 3 * q), -1, bd, bi, f.err);
+        RegisterKnnList<K> list;
+        list.init(entry);
+        if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
+        list.finish(keys);
       }
-      for (int j = 0; j < k_out; ++j) {
-        bool v = bi[j] != INT_MAX;
-        out_index[q * k_out + j] = v ? bi[j] : -1;
-        out_d2[q * k_out + j] = v ? bd[j] : -1.f;
-      }
+      write_knn_keys<K>(out_index, out_d2, q, k_out, keys);
     }
   }
 }

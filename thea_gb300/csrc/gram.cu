@@ -9,7 +9,7 @@
 // |a_r - b_j|^2 - |a_r|^2, so the row's order of the keys is the order of the squared distances (up to FP16 rounding).
 // Each thread owns one row (one tensor-memory lane), keeps the KP smallest keys, re-computes those candidates' squared
 // distances with the reference's FP32 arithmetic and outputs the k-th smallest as an upper bound on the query's k-th
-// neighbour distance. The exact search (knn_query, seeded with that bound) then returns the same neighbours as the
+// neighbour distance. The exact search (knn_points_search, seeded with that bound) then returns the same neighbours as the
 // plain traversal; the Gram tile only tightens its pruning from the first node on.
 //
 // Every wait on the MMA's completion barrier is bounded; on expiry the kernel records THEA_ERR_BIT_GRAM_TIMEOUT in the

@@ -7,6 +7,7 @@
 #include "traverse_ops.cuh"
 #include "warp_traverse.cuh"
 #include "batch.hpp"
+#include "knn_points.cuh"
 
 #include <algorithm>
 
@@ -14,6 +15,27 @@ namespace thea {
 namespace {
 
 constexpr int QUERY_THREADS = 128;
+
+// Queries a warp of the one-query-per-thread kernels takes: all its lanes once that gives every SM 24 warps, fewer below.
+// The lanes of a warp wait for one another's branches and for the slowest of them, and a small batch packed 32 to a warp
+// leaves most of the GPU idle meanwhile. Call times at 8 / 16 / 24 / 32 / 64 warps per SM, and always packed: 1,000 rays on
+// 32,768 triangles 55 / 60 / 49 / 64 / 50, 64 us; 10,000 rays on 178,802 78 / 72 / 64 / 66 / 75, 78 us; the 8 nearest of
+// 262,144 points, 1,000 queries of 65,536: 70 / 71 / 66 / 70 / 73, 105 us; 10,000: 118 / 108 / 108 / 114 / 137, 124 us.
+constexpr int SPARSE_WARPS_PER_SM = 24;
+int queries_per_warp(int64_t n, int most = 8) {
+  int64_t warps = (int64_t)sm_count() * SPARSE_WARPS_PER_SM;
+  int per = 1;
+  while ((int64_t)per * warps < n) per *= 2;
+  return per <= most ? per : 32;
+}
+unsigned sparse_grid(int64_t n, int per) { return (unsigned)ceil_div(ceil_div(n, per) * 32, QUERY_THREADS); }
+// This thread's query, or n where it has none
+__device__ __forceinline__ int64_t sparse_query(int64_t n, int per) {
+  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int lane = threadIdx.x & 31;
+  int64_t q = (t >> 5) * per + lane;
+  return lane < per && q < n ? q : n;
+}
 
 //============================================================================================================================
 // Closest element (BvhN::closestPair -> processNeighbors -> TriangleN<3>::closestPoint; BvhN.hpp:1082-1114, 1868-1893,
@@ -82,8 +104,8 @@ __device__ __forceinline__ void ray_body(WideNode<W> const * __restrict__ nodes,
            float const * __restrict__ dirs, int64_t n, float max_time, float * __restrict__ out_time,
            int32_t * __restrict__ out_index, float * __restrict__ out_normal, float * __restrict__ out_time64,
            int32_t * __restrict__ out_index64, int32_t * __restrict__ out_flags, unsigned * __restrict__ err,
-           uint32_t const * __restrict__ order) {
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+           uint32_t const * __restrict__ order, int per_warp) {
+  int64_t q = sparse_query(n, per_warp);
   float t;
   int idx;
   int64_t slot;
@@ -143,9 +165,9 @@ ray_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ r
            float const * __restrict__ dirs, int64_t n, float max_time, float * __restrict__ out_time,
            int32_t * __restrict__ out_index, float * __restrict__ out_normal, float * __restrict__ out_time64,
            int32_t * __restrict__ out_index64, int32_t * __restrict__ out_flags, unsigned * __restrict__ err,
-           uint32_t const * __restrict__ order) {
+           uint32_t const * __restrict__ order, int per_warp) {
   ray_body<W, STACK, false>(nodes, rec, origins, dirs, n, max_time, out_time, out_index, out_normal, out_time64,
-                            out_index64, out_flags, err, order);
+                            out_index64, out_flags, err, order, per_warp);
 }
 
 // The FP64 re-check form: register use capped so that five blocks of 128 threads fit on an SM
@@ -155,9 +177,9 @@ ray_recheck_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __rest
                    float const * __restrict__ origins, float const * __restrict__ dirs, int64_t n, float max_time,
                    float * __restrict__ out_time, int32_t * __restrict__ out_index, float * __restrict__ out_normal,
                    float * __restrict__ out_time64, int32_t * __restrict__ out_index64, int32_t * __restrict__ out_flags,
-                   unsigned * __restrict__ err, uint32_t const * __restrict__ order) {
+                   unsigned * __restrict__ err, uint32_t const * __restrict__ order, int per_warp) {
   ray_body<W, STACK, true>(nodes, rec, origins, dirs, n, max_time, out_time, out_index, out_normal, out_time64,
-                           out_index64, out_flags, err, order);
+                           out_index64, out_flags, err, order, per_warp);
 }
 
 // Persistent form of ray_kernel for large batches (FP32 verdict only). Rays that leave the mesh after a few nodes and
@@ -402,7 +424,7 @@ void launch_ray_stream(thea_bvh const * b, float const * o, float const * d, int
 // BoundedSortedArrayN.hpp:137-214)
 //============================================================================================================================
 
-// The k-NN kernels keep lists of K >= 8 in shared memory (knn_search_shared): 48-56 registers for K = 16, and the
+// The k-NN kernels keep lists of K >= 8 in shared memory: 48-56 registers for K = 16, and the
 // register allocator is asked for eight resident blocks of 128 threads (four for K = 32, whose lists take 32 KB)
 template <int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 8; }
 template <int K> constexpr int knn_point_min_blocks() { return knn_lists_shared<K>() ? (K <= 16 ? 8 : 4) : 8; }
@@ -443,8 +465,8 @@ __global__ void __launch_bounds__(QUERY_THREADS, knn_point_min_blocks<K>())
 knn_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ pts, float const * __restrict__ queries,
            int64_t n, int k_out, float thresh, int32_t const * __restrict__ exclude, int32_t * __restrict__ out_index,
            float * __restrict__ out_d2, unsigned * __restrict__ err, uint32_t const * __restrict__ order,
-           float const * __restrict__ init_bound) {
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+           float const * __restrict__ init_bound, int per_warp) {
+  int64_t q = sparse_query(n, per_warp);
   if (q >= n) return;
   if (order) q = order[q];
   V3 p;
@@ -463,29 +485,41 @@ knn_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ p
   }
   // init_bound (self mode, per leaf position): an upper bound on the k-th neighbour's squared distance, inclusive, from
   // actual points; the search keeps every point within it, so the result is the same as without it
-  float start = init_bound ? fminf(thresh, init_bound[q]) : thresh;
-  if constexpr (knn_lists_shared<K>()) {
-    __shared__ float s_d[K][QUERY_THREADS];
-    __shared__ int s_i[K][QUERY_THREADS];
-    int t = threadIdx.x;
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      s_d[j][t] = start;
-      s_i[j][t] = INT_MAX;
-    }
-    float kth = start;
-    int kth_i = INT_MAX;
-    knn_query_shared<W, K, STACK, QUERY_THREADS>(nodes, pts, 0, 0, p, excl, s_d, s_i, kth, kth_i, err);
-    // the row straight from shared memory (no register copy, which the dynamic row length would put in local memory)
-    write_knn_row<K>(out_index, out_d2, row, k_out, [&](int j) { return s_d[j][t]; }, [&](int j) { return s_i[j][t]; });
-  } else {
-    float bd[K];
-    int bi[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) { bd[j] = start; bi[j] = INT_MAX; }
-    knn_query<W, K, STACK>(nodes, pts, 0, 0, p, excl, bd, bi, err);
-    write_knn_row<K>(out_index, out_d2, row, k_out, [&](int j) { return bd[j]; }, [&](int j) { return bi[j]; });
+  float start = (init_bound ? fminf(thresh, init_bound[q]) : thresh) + 0.0f;  // (no negative zero)
+  bool any = start >= 0.f;  // a negative threshold admits nothing
+  // self mode starts from the points around its own in leaf order: a bound from the first step on, for a few loads that a
+  // warp shares
+  int pad = K - k_out;
+  int64_t lo = 0, hi = 0;
+  if (!queries && any) {
+    hi = q + 1 + k_out / 2 < n ? q + 1 + k_out / 2 : n;
+    lo = hi - (k_out + 1) > 0 ? hi - (k_out + 1) : 0;
+    hi = lo + k_out + 1 < n ? lo + k_out + 1 : n;
   }
+  uint64_t none = knn_key(any ? start : 0.f, INT_MAX);
+  auto entry = [&](int j) {  // initial entry j
+    if (j < pad) return (uint64_t)0;
+    int64_t k = lo + (j - pad);
+    if (k >= q) ++k;  // past the query's own point
+    if (k >= hi) return none;
+    float4 a = __ldg(pts + k);
+    uint64_t key = knn_key(squared_norm(xyz(a) - p), __float_as_int(a.w));
+    return key < none ? key : none;
+  };
+  uint64_t keys[K];
+  if constexpr (knn_lists_shared<K>()) {
+    __shared__ uint64_t s_list[K][QUERY_THREADS];
+    SharedKnnList<K, QUERY_THREADS> list(s_list);
+    list.init(entry);
+    if (any) knn_points_search<W, STACK>(nodes, pts, 0, 0, p, excl, lo, hi, list, err);
+    list.finish(keys);
+  } else {
+    RegisterKnnList<K> list;
+    list.init(entry);
+    if (any) knn_points_search<W, STACK>(nodes, pts, 0, 0, p, excl, lo, hi, list, err);
+    list.finish(keys);
+  }
+  write_knn_keys<K>(out_index, out_d2, row, k_out, keys);
 }
 
 // k nearest triangles of a mesh BVH to each query point (kClosestPairs on a MeshBvh)
@@ -494,8 +528,8 @@ __global__ void __launch_bounds__(QUERY_THREADS, knn_point_min_blocks<K>())
 knn_mesh_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
                 float const * __restrict__ queries, int64_t n, int k_out, float thresh,
                 int32_t const * __restrict__ exclude, int32_t * __restrict__ out_index, float * __restrict__ out_d2,
-                unsigned * __restrict__ err, uint32_t const * __restrict__ order) {
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                unsigned * __restrict__ err, uint32_t const * __restrict__ order, int per_warp) {
+  int64_t q = sparse_query(n, per_warp);
   if (q >= n) return;
   if (order) q = order[q];
   V3 p = load_v3(queries + 3 * q);
@@ -600,11 +634,11 @@ __device__ __forceinline__ void range_search(WideNode<W> const * __restrict__ no
 template <int W, int STACK, int MODE>
 __global__ void __launch_bounds__(QUERY_THREADS)
 range_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ pts, float const * __restrict__ queries,
-             int64_t n, float r2, int32_t const * __restrict__ exclude, int64_t * __restrict__ count_or_offset,
+             int64_t n, int per_warp, float r2, int32_t const * __restrict__ exclude, int64_t * __restrict__ count_or_offset,
              uint64_t * __restrict__ keys, float * __restrict__ out_d2, unsigned * __restrict__ err,
              int32_t * __restrict__ out_idx = nullptr, int row_cap = 0, unsigned * __restrict__ overflow = nullptr) {
   constexpr bool FILL = MODE == 1 || MODE == 2;
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t q = sparse_query(n, per_warp);
   if (q >= n) return;
   V3 p = load_v3(queries + 3 * q);
   int ex = exclude ? exclude[q] : -1;
@@ -720,16 +754,17 @@ __global__ void range_emit_kernel(uint64_t const * __restrict__ keys, uint32_t c
 template <int W, int STACK>
 void launch_range(thea_bvh const * b, float const * q, int64_t n, float r2, int32_t const * ex, int64_t * offsets,
                   int32_t * out_idx, float * out_d2, unsigned * err, bool sorted, cudaStream_t s) {
-  unsigned grid = (unsigned)ceil_div(n, QUERY_THREADS);
+  int per = queries_per_warp(n);
+  unsigned grid = sparse_grid(n, per);
   if (out_idx && !sorted) {
     THEA_LAUNCH((range_kernel<W, STACK, 2>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec, q,
-                n, r2, ex, offsets, (uint64_t *)nullptr, out_d2, err, out_idx);
+                n, per, r2, ex, offsets, (uint64_t *)nullptr, out_d2, err, out_idx);
     return;
   }
   if (!out_idx) {
     Scratch counts((size_t)n * sizeof(int64_t), s);
     THEA_LAUNCH((range_kernel<W, STACK, 0>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec,
-                q, n, r2, ex, counts.as<int64_t>(), (uint64_t *)nullptr, (float *)nullptr, err);
+                q, n, per, r2, ex, counts.as<int64_t>(), (uint64_t *)nullptr, (float *)nullptr, err);
     exclusive_scan<int64_t>(counts.as<int64_t>(), offsets, n, s);
     THEA_LAUNCH(range_total_kernel, 1, 1, 0, s, counts.as<int64_t>(), n, offsets);
     return;
@@ -748,7 +783,7 @@ void launch_range(thea_bvh const * b, float const * q, int64_t n, float r2, int3
   THEA_REQUIRE(total < (int64_t(1) << 32), "radius_neighbors: more than 2^32 neighbours in one call");
   if (extent[1] <= (unsigned long long)ROW_SORT_MAX) {
     THEA_LAUNCH((range_kernel<W, STACK, 2>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec, q,
-                n, r2, ex, offsets, (uint64_t *)nullptr, out_d2, err, out_idx);
+                n, per, r2, ex, offsets, (uint64_t *)nullptr, out_d2, err, out_idx);
     THEA_LAUNCH(range_sort_rows_kernel, (unsigned)ceil_div(n, ROW_SORT_WARPS), ROW_SORT_WARPS * 32, 0, s, offsets, n,
                 out_idx, out_d2);
     return;
@@ -756,7 +791,7 @@ void launch_range(thea_bvh const * b, float const * q, int64_t n, float r2, int3
   Scratch keys((size_t)total * sizeof(uint64_t), s), d2((size_t)total * sizeof(float), s);
   Scratch perm((size_t)total * sizeof(uint32_t), s);
   THEA_LAUNCH((range_kernel<W, STACK, 1>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec, q,
-              n, r2, ex, offsets, keys.as<uint64_t>(), d2.as<float>(), err);
+              n, per, r2, ex, offsets, keys.as<uint64_t>(), d2.as<float>(), err);
   THEA_LAUNCH(range_iota_kernel, (unsigned)ceil_div(total, 256), 256, 0, s, total, perm.as<uint32_t>());
   int qbits = 1;
   while ((int64_t(1) << qbits) < n) ++qbits;
@@ -768,9 +803,10 @@ void launch_range(thea_bvh const * b, float const * q, int64_t n, float r2, int3
 template <int W, int STACK>
 void launch_range_rows(thea_bvh const * b, float const * q, int64_t n, float r2, int32_t const * ex, int64_t * offsets,
                        int32_t * rows, int row_cap, unsigned * overflow, unsigned * err, cudaStream_t s) {
-  unsigned grid = (unsigned)ceil_div(n, QUERY_THREADS);
+  int per = queries_per_warp(n);
+  unsigned grid = sparse_grid(n, per);
   Scratch counts((size_t)n * sizeof(int64_t), s);
-  THEA_LAUNCH((range_kernel<W, STACK, 3>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec, q, n,
+  THEA_LAUNCH((range_kernel<W, STACK, 3>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->pt_rec, q, n, per,
               r2, ex, counts.as<int64_t>(), (uint64_t *)nullptr, (float *)nullptr, err, rows, row_cap, overflow);
   exclusive_scan<int64_t>(counts.as<int64_t>(), offsets, n, s);
   THEA_LAUNCH(range_total_kernel, 1, 1, 0, s, counts.as<int64_t>(), n, offsets);
@@ -949,26 +985,30 @@ void launch_ray(thea_bvh const * b, float const * o, float const * d, int64_t n,
                       b->ray_rec, o, d, n, rp.max_time, t, idx, nrm, err, order, counter.as<unsigned long long>());
     return;
   }
+  int per = queries_per_warp(n);
+  grid = sparse_grid(n, per);
   if (rp.recheck)
     THEA_LAUNCH((ray_recheck_kernel<W, STACK>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->ray_rec,
-                o, d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order);
+                o, d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order, per);
   else
     THEA_LAUNCH((ray_kernel<W, STACK, false>), grid, QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes, b->ray_rec, o,
-                d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order);
+                d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order, per);
 }
 
 template <int W, int K, int STACK>
 void launch_knn_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,
                   int32_t * idx, float * d2, unsigned * err, uint32_t const * order, float const * ib, cudaStream_t s) {
-  THEA_LAUNCH((knn_kernel<W, K, STACK>), (unsigned)ceil_div(n, QUERY_THREADS), QUERY_THREADS, 0, s,
-              (WideNode<W> const *)b->nodes, b->pt_rec, q, n, k, thresh, ex, idx, d2, err, order, ib);
+  int per = queries_per_warp(n, q ? 8 : 4);
+  THEA_LAUNCH((knn_kernel<W, K, STACK>), sparse_grid(n, per), QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes,
+              b->pt_rec, q, n, k, thresh, ex, idx, d2, err, order, ib, per);
 }
 
 template <int W, int K, int STACK>
 void launch_knn_mesh_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,
                        int32_t * idx, float * d2, unsigned * err, uint32_t const * order, cudaStream_t s) {
-  THEA_LAUNCH((knn_mesh_kernel<W, K, STACK>), (unsigned)ceil_div(n, QUERY_THREADS), QUERY_THREADS, 0, s,
-              (WideNode<W> const *)b->nodes, b->cp_rec, q, n, k, thresh, ex, idx, d2, err, order);
+  int per = queries_per_warp(n);
+  THEA_LAUNCH((knn_mesh_kernel<W, K, STACK>), sparse_grid(n, per), QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes,
+              b->cp_rec, q, n, k, thresh, ex, idx, d2, err, order, per);
 }
 
 template <int W, int STACK>

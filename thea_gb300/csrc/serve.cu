@@ -10,6 +10,7 @@
 #include "serve.hpp"
 
 #include "device_util.cuh"
+#include "knn_points.cuh"
 #include "query.hpp"
 #include "traverse_ops.cuh"
 #include "warp_traverse.cuh"
@@ -242,19 +243,23 @@ serve_knn_kernel(ServeTask const * __restrict__ tasks, int64_t const * __restric
     int ti = task_of(off, T, q);
     ServeTask const * t = tasks + ti;
     int64_t i = q - __ldg(off + ti);
-    float bd[K];
-    int bi[K];
+    // the list in registers: with shared lists the launch's blocks crowd out the other slots' batches
+    int k = t->k;
+    float start = t->thresh + 0.0f;  // (no negative zero)
+    bool any = start >= 0.f;         // a negative threshold admits nothing
+    uint64_t none = knn_key(any ? start : 0.f, INT_MAX);
+    RegisterKnnList<K> list;
+    list.init([&](int j) { return j < K - k ? (uint64_t)0 : none; });
+    if (any)
+      knn_points_search<W, STACK>((WideNode<W> const *)t->nodes, t->rec, 0, 0, load_v3(t->in0 + 3 * i), -1, 0, 0, list,
+                                  t->err);
+    int pad = K - k;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      bd[j] = t->thresh;
-      bi[j] = INT_MAX;
-    }
-    knn_query<W, K, STACK>((WideNode<W> const *)t->nodes, t->rec, 0, 0, load_v3(t->in0 + 3 * i), -1, bd, bi, t->err);
-    int k = t->k;
-    for (int j = 0; j < k; ++j) {
-      bool v = bi[j] != INT_MAX;
-      t->out_index[i * k + j] = v ? bi[j] : -1;
-      if (t->out_value) t->out_value[i * k + j] = v ? bd[j] : -1.f;
+      if (j < pad) continue;
+      int e = knn_key_index(list.r[j]);
+      t->out_index[i * k + j - pad] = e != INT_MAX ? e : -1;
+      if (t->out_value) t->out_value[i * k + j - pad] = e != INT_MAX ? knn_key_d2(list.r[j]) : -1.f;
     }
   }
 }

@@ -1165,7 +1165,7 @@ __device__ __forceinline__ void ray_resolve_warp(RaySearch64 & s, bool active, f
 }
 
 //============================================================================================================================
-// k nearest points
+// k nearest elements (points: knn_points.cuh)
 //============================================================================================================================
 
 // Insert (d, i) into sorted register arrays, lexicographic (distance, index); the last entry falls off.
@@ -1182,45 +1182,7 @@ template <int K> __device__ __forceinline__ void knn_insert(float (&bd)[K], int 
   }
 }
 
-template <int W, int K, int STACK>
-__device__ __forceinline__ void knn_query(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ pts,
-                                          int root, int64_t elem_base, V3 p, int excl, float (&bd)[K], int (&bi)[K],
-                                          unsigned * err) {
-  LocalStack<STACK> stk;  // (child code, bound bits)
-  int sp = 0;
-  int next = root;  // nearest child of the last node, visited without a stack round trip
-  while (next != CHILD_EMPTY || sp > 0) {
-    int code = next;
-    if (code == CHILD_EMPTY) {
-      --sp;
-      int2 top = stk.get(sp);
-      code = top.x;
-      if (__int_as_float(top.y) > bd[K - 1] * PRUNE_SLACK) continue;
-    }
-    next = CHILD_EMPTY;
-    if (code >= 0) {
-      NodeRegs<W> nd;
-      load_node(nodes, code, nd);
-      float lb[W];
-      point_child_bounds<W>(nd, p, lb);
-      push_children_next<W>(nd, lb, bd[K - 1] * PRUNE_SLACK, stk, sp, next, err);
-    } else {
-      int first, count;
-      decode_leaf(code, first, count);
-      int64_t k0 = elem_base + first;
-      for (int64_t k = k0; k < k0 + count; ++k) {
-        float4 a = __ldg(pts + k);
-        int idx = __float_as_int(a.w);
-        if (idx == excl) continue;
-        // MetricL2Impl<point, point>::closestPoints: (element - query).squaredNorm()
-        float d2 = squared_norm(xyz(a) - p);
-        if (d2 < bd[K - 1] || (d2 == bd[K - 1] && idx < bi[K - 1])) knn_insert<K>(bd, bi, d2, idx);
-      }
-    }
-  }
-}
-
-// knn_query with the sorted list in shared memory instead of registers: sd / si are [K][B] arrays of the block (B
+// k-nearest search with the sorted list in shared memory instead of registers: sd / si are [K][B] arrays of the block (B
 // threads, entry j of thread t at [j][t], so a warp's accesses fall in distinct banks) and the k-th entry is mirrored in
 // kth / kth_i for the reject test. An insertion shifts the larger entries up one place (the same (distance, index)
 // order as knn_insert). Holding the lists out of registers lets twice as many warps stay resident. `elem(k, idx, d2)`
@@ -1274,21 +1236,6 @@ __device__ __forceinline__ void knn_search_shared(WideNode<W> const * __restrict
       }
     }
   }
-}
-
-// Points: MetricL2Impl<point, point>::closestPoints, (element - query).squaredNorm()
-template <int W, int K, int STACK, int B>
-__device__ __forceinline__ void knn_query_shared(WideNode<W> const * __restrict__ nodes,
-                                                 float4 const * __restrict__ pts, int root, int64_t elem_base, V3 p,
-                                                 int excl, float (*sd)[B], int (*si)[B], float & kth, int & kth_i,
-                                                 unsigned * err) {
-  knn_search_shared<W, K, STACK, B>(nodes, root, elem_base, p, excl, sd, si, kth, kth_i, err,
-                                    [&](int64_t k, int & idx, float & d2) {
-                                      float4 a = __ldg(pts + k);
-                                      idx = __float_as_int(a.w);
-                                      d2 = squared_norm(xyz(a) - p);
-                                      return true;
-                                    });
 }
 
 // Triangles: the closest-point record test (FP32 reference arithmetic); a NaN distance is never kept
