@@ -168,7 +168,7 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
 // Persistent-lane form of batch_closest_kernel: each lane takes a new query as soon as its query is done, instead of
 // idling until the slowest query of its warp's round (the queries deep inside a mesh take ten times the steps of the
 // others). Every loop iteration advances each busy lane by one stack entry; idle lanes are refilled from a warp-local
-// block of 64 query indices. FP32 search only (the mixed-precision search is bound by the FP64 pipe, and rounds of 32
+// block of up to 64 query indices. FP32 search only (the mixed-precision search is bound by the FP64 pipe, and rounds of 32
 // queries fill its FP64 step better: 25.7 against 27.5 ms on 256 meshes). Results are the round-based kernel's: each
 // query's search is the same sequence of steps. What bounds it: the L1 data pipe (65 % busy) and the latency of the node
 // and record loads (a third of the lanes active: a warp mixes lanes at nodes, at leaves and between queries). One
@@ -181,7 +181,7 @@ constexpr int REFILL_BLOCK = 64;
 template <int W, int STACK>
 __global__ void __launch_bounds__(BATCH_THREADS)
 batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long long * counter, int budget,
-                            HardQueue hq) {
+                            HardQueue hq, int block) {
   unsigned const FULL = 0xffffffffu;
   int lane = threadIdx.x & 31;
   WideNode<W> const * nodes = (WideNode<W> const *)f.nodes;
@@ -204,10 +204,10 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
     if (idle && !exhausted) {
       if (qb >= qe) {
         unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(counter, (unsigned long long)REFILL_BLOCK);
+        if (lane == 0) b = atomicAdd(counter, (unsigned long long)block);
         b = __shfl_sync(FULL, b, 0);
         qb = (int64_t)b;
-        qe = qb + REFILL_BLOCK < nq ? qb + REFILL_BLOCK : nq;
+        qe = qb + block < nq ? qb + block : nq;
         if (qb >= nq) exhausted = true;
       }
       if (!exhausted) {
@@ -320,6 +320,29 @@ batch_closest_phase2_kernel(BatchForest f, ClosestArgs a, HardQueue hq, unsigned
       }
     }
     __syncwarp();
+  }
+}
+
+// TEAM lanes per query from the root, FP32, one BVH: the small-batch form, in one launch. What bounds it is the longest
+// query's chain of dependent steps; a search on one thread takes four to ten times as many.
+template <int W, int TEAM>
+__global__ void __launch_bounds__(BATCH_THREADS)
+closest_team_kernel(BatchForest f, ClosestArgs a, int64_t nq) {
+  constexpr int TEAMS = BATCH_THREADS / TEAM;
+  constexpr int CAP = TEAM == 32 ? WARP_STACK : 256;
+  __shared__ int s_code[TEAMS][CAP];
+  __shared__ float s_lb[TEAMS][CAP];
+  int team = threadIdx.x / TEAM;
+  int64_t q = (int64_t)blockIdx.x * TEAMS + team;
+  bool active = q < nq;
+  V3 p = active ? load_v3(a.queries + 3 * q) : V3{0.f, 0.f, 0.f};
+  WarpBest b = closest_team_query<W, TEAM>((WideNode<W> const *)f.nodes, f.cp_rec, active, p, a.thresh, s_code[team],
+                                           s_lb[team], CAP, f.err, f.slabs);
+  if (active && threadIdx.x % TEAM == 0) {
+    bool found = b.idx != INT_MAX;
+    V3 cp = V3{0.f, 0.f, 0.f};
+    if (found) cp_record_test(f.cp_rec, b.slot, p, cp);
+    write_closest(q, found, sqrtf(b.d2), cp, b.idx, 0.0, a.out_index, a.out_dist, a.out_cp, nullptr);
   }
 }
 
@@ -539,8 +562,11 @@ void launch_closest_prec(BatchForest const & f, ClosestArgs const & a, int64_t n
   bool refill = PREC != THEA_PRECISION_FP64_RECHECK && !a.out_err;
   if (refill) {
     auto kr = batch_closest_refill_kernel<W, STACK>;
-    THEA_LAUNCH_NAMED(name, kr, persistent_grid((void const *)kr), BATCH_THREADS, 0, s, f, a, nq, counters,
-                      phase1_budget, hq);
+    // a block of indices no larger than a warp's share: a small batch keeps every warp busy
+    int pg = persistent_grid((void const *)kr);
+    int64_t per = ceil_div(nq, (int64_t)pg * (BATCH_THREADS / 32));
+    THEA_LAUNCH_NAMED(name, kr, pg, BATCH_THREADS, 0, s, f, a, nq, counters, phase1_budget, hq,
+                      (int)std::min<int64_t>(REFILL_BLOCK, std::max<int64_t>(1, per)));
   } else {
     THEA_LAUNCH_NAMED(name, k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk,
                       phase1_budget, hq);
@@ -726,6 +752,22 @@ void run_batch_closest(thea_bvh const * b, float const * q, int64_t const * qoff
   }
   ClosestArgs a{q, qoff, cp.thresh, cp.bound2, cp.scene_scale, idx, dist, cpt, err, cp.seg_cut};
   batch_closest_core(b, a, nq, cp, chunk, s);
+}
+
+template <int W, int TEAM>
+void launch_closest_team(BatchForest const & f, ClosestArgs const & a, int64_t nq, cudaStream_t s) {
+  unsigned grid = (unsigned)ceil_div(nq, BATCH_THREADS / TEAM);
+  THEA_LAUNCH((closest_team_kernel<W, TEAM>), grid, BATCH_THREADS, 0, s, f, a, nq);
+}
+
+void run_closest_teams(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,
+                       float * dist, float * cpt, cudaStream_t s) {
+  if (nq <= 0) return;
+  BatchForest f = forest_view(b);
+  ClosestArgs a{q, nullptr, cp.thresh, cp.bound2, cp.scene_scale, idx, dist, cpt, nullptr};
+  bool whole = nq < CLOSEST_WHOLE_WARP_MAX;
+  if (b->width == 4) whole ? launch_closest_team<4, 32>(f, a, nq, s) : launch_closest_team<4, 16>(f, a, nq, s);
+  else whole ? launch_closest_team<8, 32>(f, a, nq, s) : launch_closest_team<8, 16>(f, a, nq, s);
 }
 
 template <int W, int STACK>

@@ -33,6 +33,11 @@ inline int batch_closest_budget(int64_t nq) { return nq >= 98304 ? 256 : 32; }
 // takes per fetch (a multiple of 32).
 void run_batch_closest(thea_bvh const * b, float const * q, int64_t const * qoff, int64_t nq, ClosestParams const & cp,
                        int chunk, int32_t * idx, float * dist, float * cpt, float * err, cudaStream_t s);
+// FP32 closest point of a small batch on one BVH (num_segments == 1, small_stack_ok), a whole warp per query below
+// CLOSEST_WHOLE_WARP_MAX queries and half a warp from there.
+constexpr int64_t CLOSEST_WHOLE_WARP_MAX = 3072;
+void run_closest_teams(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,
+                       float * dist, float * cpt, cudaStream_t s);
 // FP32 closest point of one BVH with queries and results in pinned host memory accessed by the kernels in place
 // (device-usable pointers); cp.budget > 0 enables the warp-per-query second phase.
 void run_closest_stream(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,

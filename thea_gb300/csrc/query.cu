@@ -557,13 +557,16 @@ knn_mesh_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restric
   }
 }
 
-// FP32 calls on one BVH by size (config-0 sweep of 1,024 .. 262,144 queries, event-timed):
-//  * fewer than CLOSEST_WARP_MAX queries: two kernels with a 16-step budget, so nearly every query runs as one warp
-//    over up to 8 nodes a step (4,096 queries: 0.19 ms against 0.59 ms one per thread, whose time is the longest
-//    query's chain of dependent loads);
-//  * up to CLOSEST_TWO_PHASE_MIN: one query per thread (65,536 queries: 0.71 ms; 0.72 with a 16-step budget);
-//  * from there: two kernels with a 256-step budget (persistent lanes, then a warp per query past it; 262,144 queries:
-//    1.30 ms against 1.84 one per thread).
+// FP32 calls on one BVH by size. Call times in ms on 81,920 triangles, queries near the surface / uniform in its box grown
+// by half (a seventh of them deep inside, ten times the steps of the others):
+//  * fewer than CLOSEST_WARP_MAX queries: 32 or 16 lanes per query (run_closest_teams). 1,000 queries: 0.047 / 0.088 with
+//    32 lanes, 0.041 / 0.113 with 16; 4,000: 0.078 / 0.119 and 0.043 / 0.137; 16,000: 0.189 / 0.287 and 0.091 / 0.240;
+//    57,000: 0.616 / 0.882 and 0.260 / 0.617; with 8 lanes 0.175 / 0.764. (Two kernels, a 16-step budget on one thread and
+//    then a warp: 0.059 / 0.093, 0.077 / 0.118, 0.146 / 0.233, 0.374 / 0.608; that form stays for trees too deep for the
+//    teams' stacks.)
+//  * up to CLOSEST_TWO_PHASE_MIN: one query per thread (65,536 queries in the box: 0.71 ms; 0.72 with a 16-step budget);
+//  * from there: two kernels with a 256-step budget (persistent lanes, then a warp per query past it; 262,144 queries in
+//    the box: 1.06 ms against 1.84 one per thread).
 constexpr int64_t CLOSEST_WARP_MAX = 57344;
 constexpr int CLOSEST_WARP_BUDGET = 16;
 constexpr int64_t CLOSEST_TWO_PHASE_MIN = 98304;
@@ -1048,6 +1051,10 @@ void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams c
   if (n <= 0) return;
   if (cp.precision == THEA_PRECISION_FP32_REFERENCE && !errout && !b->query_order &&
       (n < CLOSEST_WARP_MAX || n >= CLOSEST_TWO_PHASE_MIN)) {
+    if (n < CLOSEST_WARP_MAX && small_stack_ok(b)) {
+      run_closest_teams(b, q, n, cp, idx, dist, cpt, s);
+      return;
+    }
     // Persistent lanes with a step budget, then one warp per query over budget (the BVH is a one-mesh forest). The
     // same searches, so the same results.
     Scratch qoff(2 * sizeof(int64_t), s);

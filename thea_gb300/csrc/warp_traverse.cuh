@@ -163,6 +163,121 @@ __device__ WarpBest closest_warp_query(WideNode<W> const * __restrict__ nodes, f
   return best;
 }
 
+// closest_warp_query from the root of one BVH with TEAM lanes to a query (16 or 32: 32 / TEAM queries a warp). With fewer
+// lanes a step expands fewer nodes (TEAM / W), so fewer of the expansions are ones that a sequential search would have
+// pruned, and the sort is shorter; the chain of steps is longer. All lanes of the warp call it together; a team without a
+// query passes active = false. s_code / s_lb: this team's stack of `cap` entries; a tree of depth D needs at most
+// (TEAM / W) ((W - 1) D + 1).
+template <int W, int TEAM>
+__device__ WarpBest closest_team_query(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec, bool active,
+                                       V3 p, float thresh, int * s_code, float * s_lb, int cap, unsigned * err,
+                                       float4 const * __restrict__ slabs) {
+  constexpr int NPOP = TEAM / W;
+  unsigned const FULL = 0xffffffffu;
+  float q1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
+  int lane = threadIdx.x & 31, tl = lane % TEAM;
+  unsigned team_mask = (TEAM == 32 ? FULL : ((1u << TEAM) - 1u)) << (lane - tl);
+  int e = tl / W, c = tl % W;
+  int sp = active ? 1 : 0;
+  if (tl == 0) {
+    s_code[0] = 0;
+    s_lb[0] = 0.f;
+  }
+  __syncwarp();
+  unsigned long long bkey = best_key(thresh, INT_MAX);
+  int64_t best_slot = -1;  // of this lane's own best
+  unsigned long long mine = ~0ull;
+  while (__any_sync(FULL, sp > 0)) {
+    int npop = sp < NPOP ? sp : NPOP;
+    int base = sp - npop;
+    int code = CHILD_EMPTY;
+    float lbe = 0.f;
+    if (e < npop) {
+      code = s_code[base + e];
+      lbe = s_lb[base + e];
+    }
+    __syncwarp();
+    sp = base;
+    float bd = __uint_as_float((unsigned)(bkey >> 32));
+    float lim = bd * PRUNE_SLACK;
+    uint32_t key = 0xffffffffu;
+    int push_code = CHILD_EMPTY;
+    if (code != CHILD_EMPTY && lbe <= lim) {
+      float lx, hx, ly, hy, lz, hz;
+      int child;
+      load_child<W>(nodes, code, c, lx, hx, ly, hy, lz, hz, child);
+      float d2b = point_box_d2(p.x, p.y, p.z, lx, ly, lz, hx, hy, hz);
+      if (slabs && child != CHILD_EMPTY) {
+        float d;
+        d2b = fmaxf(d2b, slab_lower_bound(__ldg(slabs + (int64_t)code * W + c), p, q1, d));
+      }
+      if (child != CHILD_EMPTY && d2b <= lim) {
+        if (child >= 0) {
+          key = __float_as_uint(d2b);
+          push_code = child;
+        } else {
+          int first, count;
+          decode_leaf(child, first, count);
+          for (int64_t k = first; k < first + count; ++k) {
+            V3 cp;
+            float d2 = cp_record_test(rec, k, p, cp);
+            if (d2 <= bd) {
+              unsigned long long kk = best_key(d2, cp_record_index(rec, k));
+              if (kk < mine) {
+                mine = kk;
+                best_slot = k;
+              }
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+    // agree on the best element
+    unsigned long long m = mine;
+#pragma unroll
+    for (int o = TEAM / 2; o > 0; o >>= 1) {
+      unsigned long long u = __shfl_xor_sync(FULL, m, o);
+      m = u < m ? u : m;
+    }
+    bkey = m < bkey ? m : bkey;
+    // sort the surviving internal children, nearest first
+#pragma unroll
+    for (int k = 2; k <= TEAM; k <<= 1) {
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        uint32_t pk = __shfl_xor_sync(FULL, key, j);
+        int pc = __shfl_xor_sync(FULL, push_code, j);
+        bool ascending = (tl & k) == 0;
+        bool lower = (tl & j) == 0;
+        bool take = (lower == ascending) ? (pk < key) : (pk > key);
+        if (take) {
+          key = pk;
+          push_code = pc;
+        }
+      }
+    }
+    int n = __popc(__ballot_sync(FULL, key != 0xffffffffu) & team_mask);
+    if (sp + n > cap) {
+      if (tl == 0) atomicOr(err, ERR_STACK_OVERFLOW);
+      n = cap - sp;
+    }
+    if (tl < n) {
+      int pos = sp + (n - 1 - tl);
+      s_code[pos] = push_code;
+      s_lb[pos] = __uint_as_float(key);
+    }
+    __syncwarp();
+    sp += n;
+  }
+  WarpBest best;
+  unsigned who = __ballot_sync(FULL, mine == bkey && mine != ~0ull) & team_mask;
+  best.slot = __shfl_sync(FULL, best_slot, who ? __ffs(who) - 1 : lane);
+  best.d2 = __uint_as_float((unsigned)(bkey >> 32));
+  best.idx = (int)(unsigned)(bkey & 0xffffffffu);
+  return best;
+}
+
 constexpr int WARP_CAND = 64;  // FP64 candidates per warp
 
 struct WarpBest64 {
