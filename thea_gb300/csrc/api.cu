@@ -73,9 +73,8 @@ void note_launch_end(char const * kernel_name, cudaStream_t stream, cudaEvent_t 
 // Scratch memory pool
 //============================================================================================================================
 
-cudaMemPool_t scratch_pool() {
-  static std::mutex m;
-  static std::map<int, cudaMemPool_t> pools;
+// One pool per device, created on first use; `keep`: bytes kept mapped beyond what is in use
+static cudaMemPool_t device_pool(std::map<int, cudaMemPool_t> & pools, std::mutex & m, uint64_t keep) {
   int dev = 0;
   THEA_CUDA_CHECK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(m);
@@ -88,10 +87,68 @@ cudaMemPool_t scratch_pool() {
   props.location.id = dev;
   cudaMemPool_t pool;
   THEA_CUDA_CHECK(cudaMemPoolCreate(&pool, &props));
-  uint64_t keep = ~uint64_t(0);
   THEA_CUDA_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
   pools[dev] = pool;
   return pool;
+}
+
+cudaMemPool_t scratch_pool() {
+  static std::mutex m;
+  static std::map<int, cudaMemPool_t> pools;
+  return device_pool(pools, m, ~uint64_t(0));
+}
+
+cudaMemPool_t handle_pool() {
+  static std::mutex m;
+  static std::map<int, cudaMemPool_t> pools;
+  return device_pool(pools, m, HANDLE_POOL_KEEP);
+}
+
+namespace {
+constexpr int HOST_WORDS = 1024;
+struct HostWords {
+  unsigned * base;
+  std::vector<int> free;
+};
+std::mutex g_words_mutex;
+std::vector<HostWords> & host_words() {  // never destroyed: handles may outlive static destruction
+  static auto * v = new std::vector<HostWords>;
+  return *v;
+}
+}  // namespace
+
+unsigned * take_host_word() {
+  std::lock_guard<std::mutex> lk(g_words_mutex);
+  auto & blocks = host_words();
+  HostWords * from = nullptr;
+  for (auto & b : blocks)
+    if (!b.free.empty()) from = &b;
+  if (!from) {
+    HostWords b;
+    THEA_CUDA_CHECK(thea_malloc_host(&b.base, HOST_WORDS * sizeof(unsigned)));
+    for (int i = HOST_WORDS - 1; i >= 0; --i) b.free.push_back(i);
+    blocks.push_back(std::move(b));
+    from = &blocks.back();
+  }
+  unsigned * w = from->base + from->free.back();
+  from->free.pop_back();
+  *w = 0;
+  return w;
+}
+
+void release_host_word(unsigned * w) {
+  std::lock_guard<std::mutex> lk(g_words_mutex);
+  auto & blocks = host_words();
+  for (size_t i = 0; i < blocks.size(); ++i) {
+    HostWords & b = blocks[i];
+    if (w < b.base || w >= b.base + HOST_WORDS) continue;
+    b.free.push_back((int)(w - b.base));
+    if ((int)b.free.size() == HOST_WORDS && blocks.size() > 1) {
+      cudaFreeHost(b.base);
+      blocks.erase(blocks.begin() + (long)i);
+    }
+    return;
+  }
 }
 
 //============================================================================================================================

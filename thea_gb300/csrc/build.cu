@@ -56,9 +56,19 @@ __device__ __forceinline__ int segment_of(int64_t const * __restrict__ start, in
 // [6..8] min of box lo, [9..11] max of box hi. A warp whose lanes share one segment reduces before its atomics, and a
 // block whose warps all share one segment reduces once more, so a single large segment takes 12 atomics per block
 // rather than per warp (the per-warp form spent 0.5 ms of contended atomics on 2 M triangles).
-__global__ void elem_box_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t n, int is_mesh,
-                                int64_t const * __restrict__ seg_start, int M, float4 * __restrict__ elo,
-                                float4 * __restrict__ ehi, int * __restrict__ bounds) {
+//
+// A face index outside [0, nv) sets *bad and reads vertex 0 in its place (nv > 0); the host refuses the build when it next
+// synchronizes.
+__device__ __forceinline__ int64_t face_vertex(int32_t const * __restrict__ F, int64_t k, int64_t nv, bool & out) {
+  int64_t f = F[k];
+  if (f >= 0 && f < nv) return f;
+  out = true;
+  return 0;
+}
+
+__global__ void elem_box_kernel(float const * __restrict__ V, int64_t nv, int32_t const * __restrict__ F, int64_t n,
+                                int is_mesh, int64_t const * __restrict__ seg_start, int M, float4 * __restrict__ elo,
+                                float4 * __restrict__ ehi, int * __restrict__ bounds, int * __restrict__ bad) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool ok = i < n;
   int v[12];
@@ -66,9 +76,11 @@ __global__ void elem_box_kernel(float const * __restrict__ V, int32_t const * __
   if (ok) {
     V3 lo, hi;
     if (is_mesh) {
-      V3 a = load_v3(V + 3 * (int64_t)F[3 * i]);
-      V3 b = load_v3(V + 3 * (int64_t)F[3 * i + 1]);
-      V3 c = load_v3(V + 3 * (int64_t)F[3 * i + 2]);
+      bool out = false;
+      V3 a = load_v3(V + 3 * face_vertex(F, 3 * i, nv, out));
+      V3 b = load_v3(V + 3 * face_vertex(F, 3 * i + 1, nv, out));
+      V3 c = load_v3(V + 3 * face_vertex(F, 3 * i + 2, nv, out));
+      if (out) *bad = 1;
       lo = V3{fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z))};
       hi = V3{fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z))};
     } else {
@@ -149,8 +161,18 @@ __global__ void face_range_kernel(int32_t const * __restrict__ F, int64_t count,
   if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
 }
 
-__global__ void init_bounds_kernel(int * __restrict__ bounds, int M) {
+// Start values: bounds, the error words and, for one segment, its start, its root and the collapse's first level
+__global__ void build_init_kernel(int * __restrict__ bounds, int M, int * __restrict__ bad, unsigned * __restrict__ err,
+                                  int64_t * __restrict__ seg_start, int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    *bad = 0;
+    *err = 0;
+    if (M == 1) {
+      seg_start[0] = 0;
+      seg_start[1] = n;
+    }
+  }
   if (i >= 12 * (int64_t)M) return;
   int t = (int)(i % 12);
   bounds[i] = ((t < 3) || (t >= 6 && t < 9)) ? INT_MAX : INT_MIN;
@@ -209,12 +231,15 @@ __device__ __forceinline__ int kdelta(uint64_t const * __restrict__ codes, int64
 __global__ void karras_kernel(uint64_t const * __restrict__ codes, int64_t n, int64_t const * __restrict__ seg_start,
                               int M, int mbits, int * __restrict__ left, int * __restrict__ right,
                               int * __restrict__ first, int * __restrict__ last, int * __restrict__ parent,
-                              int * __restrict__ leaf_parent) {
+                              int * __restrict__ leaf_parent, unsigned * __restrict__ visits) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int s = M > 1 ? (int)(codes[i] >> mbits) : 0;
   int64_t a = M > 1 ? seg_start[s] : 0, b = M > 1 ? seg_start[s + 1] : n;
+  if (b - a == 1) leaf_parent[i] = -1;  // no internal node
   if (i >= b - 1) return;  // a segment of m elements has m - 1 internal nodes, at positions a .. b - 2
+  visits[i - s] = 0;
+  if (i == a) parent[i - s] = -1;  // the segment's root
   int d = (kdelta(codes, a, b, i, i + 1) - kdelta(codes, a, b, i, i - 1)) >= 0 ? 1 : -1;
   int dmin = kdelta(codes, a, b, i, i - d);
   int64_t lmax = 2;
@@ -256,7 +281,13 @@ __device__ __forceinline__ void child_box(int code, float4 const * __restrict__ 
 }
 
 // Bottom-up refit: the second thread to reach a node merges its two children and continues upwards.
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+  float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
+  return x * y + y * z + z * x;
+}
+
 __global__ void refit_kernel(int64_t n, int const * __restrict__ left, int const * __restrict__ right,
+                             int const * __restrict__ first, int const * __restrict__ last,
                              int const * __restrict__ parent, int const * __restrict__ leaf_parent,
                              float4 const * __restrict__ elo, float4 const * __restrict__ ehi,
                              uint32_t const * __restrict__ sorted, float4 * ilo, float4 * ihi,
@@ -271,8 +302,13 @@ __global__ void refit_kernel(int64_t n, int const * __restrict__ left, int const
     float4 al, ah, bl, bh;
     child_box(left[p], elo, ehi, sorted, ilo, ihi, al, ah);
     child_box(right[p], elo, ehi, sorted, ilo, ihi, bl, bh);
-    __stcg(ilo + p, make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f));
-    __stcg(ihi + p, make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f));
+    // the box, with its half area in lo.w and the number of elements in hi.w
+    float4 lo = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f);
+    float4 hi = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f);
+    lo.w = half_area(lo, hi);
+    hi.w = __int_as_float(last[p] - first[p] + 1);
+    __stcg(ilo + p, lo);
+    __stcg(ihi + p, hi);
     p = parent[p];
   }
 }
@@ -293,70 +329,81 @@ struct CollapseArgs {
 };
 
 __device__ __forceinline__ int code_count(CollapseArgs const & a, int code) {
-  return code < 0 ? 1 : a.last[code] - a.first[code] + 1;
+  return code < 0 ? 1 : __float_as_int(a.ihi[code].w);
 }
 __device__ __forceinline__ int code_first(CollapseArgs const & a, int code) { return code < 0 ? ~code : a.first[code]; }
 
-__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
-  float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
-  return x * y + y * z + z * x;
-}
-
-// For each frontier binary node, choose the W binary subtrees that become the children of its wide node: starting from
-// the two children, repeatedly open the subtree with the largest surface area among those too big to be a leaf.
-// Frontier of the level being collapsed, kept on the device so that several levels run between host synchronisations:
-// its size, the wide index of its first node, and the number of levels emitted so far.
+// The level being collapsed, kept on the device so that all levels run between two host synchronisations: its frontier
+// size, the wide index of its first node, and the number of levels emitted so far.
 struct CollapseLevel {
   int64_t fsize;
   int64_t base;
   int64_t levels;
   int64_t overflow;  // set if a node would have landed past the node bound (never, by the bound's construction)
-  int64_t parity;    // which of the two frontier buffers holds the current frontier
 };
 
-// The W binary subtrees that become the children of frontier node f's wide node; returns how many are internal
+// The W binary subtrees that become the children of frontier node f's wide node: starting from its two children,
+// repeatedly open the subtree with the largest surface area among those too big to be a leaf. Returns how many are
+// internal.
 template <int W>
 __device__ __forceinline__ int collapse_decide_one(CollapseArgs const & a, int const * __restrict__ frontier, int64_t f,
                                                    int * __restrict__ chosen) {
   int b = frontier[f];
   int codes[W];
-  int ne = 2;
-  codes[0] = a.left[b];
-  codes[1] = a.right[b];
+  float area[W];  // of the subtrees too big to be a leaf; negative otherwise
+  auto put = [&](int e, int code) {
+    codes[e] = code;
+    bool big = code >= 0 && __float_as_int(a.ihi[code].w) > a.leaf_size;
+    area[e] = big ? a.ilo[code].w : -1.f;
+    if (big && !(area[e] >= 0.f)) area[e] = 0.f;  // (a NaN or negative area still opens, last)
+  };
 #pragma unroll
-  for (int e = 2; e < W; ++e) codes[e] = CHILD_EMPTY;
-  while (ne < W) {
-    int best = -1;
+  for (int e = 0; e < W; ++e) codes[e] = CHILD_EMPTY, area[e] = -1.f;
+  put(0, a.left[b]);
+  put(1, a.right[b]);
+#pragma unroll
+  for (int ne = 2; ne < W; ++ne) {
+    int best = -1, code = CHILD_EMPTY;
     float best_sa = -1.f;
-    for (int e = 0; e < ne; ++e) {
-      int c = codes[e];
-      if (c >= 0 && code_count(a, c) > a.leaf_size) {
-        float sa = half_area(a.ilo[c], a.ihi[c]);
-        if (sa > best_sa) { best_sa = sa; best = e; }
-      }
-    }
+#pragma unroll
+    for (int e = 0; e < W; ++e)
+      if (e < ne && area[e] > best_sa) best_sa = area[e], best = e, code = codes[e];
     if (best < 0) break;
-    int c = codes[best];
-    codes[best] = a.left[c];
-    codes[ne++] = a.right[c];
+    int l = a.left[code], r = a.right[code];
+#pragma unroll
+    for (int e = 0; e < W; ++e)
+      if (e == best) put(e, l);
+    put(ne, r);
   }
   int nint = 0;
+#pragma unroll
   for (int e = 0; e < W; ++e) {
     chosen[f * W + e] = codes[e];
-    if (codes[e] != CHILD_EMPTY && code_count(a, codes[e]) > a.leaf_size) ++nint;
+    nint += area[e] >= 0.f ? 1 : 0;
   }
   return nint;
 }
 
+// A level takes two launches: every frontier node's children decided, with the internal ones counted per block (offs: the
+// node's place among its block's, tot: the block's count); then the wide nodes written, the internal children placed
+// after those of the blocks before (summed here from tot, or read from `scanned` when there are too many blocks). The
+// numbering is the frontier's order, whatever order the blocks run in. The state for the next level goes to `next`.
 template <int W>
-__global__ void collapse_decide_kernel(CollapseArgs a, int const * __restrict__ fa, int const * __restrict__ fb,
-                                       CollapseLevel const * __restrict__ lv, int64_t bound,
-                                       int * __restrict__ chosen, int * __restrict__ num_internal) {
-  int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= bound) return;
+__global__ void __launch_bounds__(BUILD_THREADS)
+collapse_decide_kernel(CollapseArgs a, int const * __restrict__ frontier, CollapseLevel const * __restrict__ lv,
+                       int * __restrict__ chosen, int * __restrict__ offs, int * __restrict__ tot) {
   int64_t fsize = lv->fsize;
-  num_internal[f] = f < fsize ? collapse_decide_one<W>(a, lv->parity ? fb : fa, f, chosen) : 0;  // the scan covers
-                                                                                                   // the host's bound
+  int64_t f0 = (int64_t)blockIdx.x * BUILD_THREADS;
+  if (f0 >= fsize) {
+    if (threadIdx.x == 0) tot[blockIdx.x] = 0;
+    return;
+  }
+  int64_t f = f0 + threadIdx.x;
+  int nint = f < fsize ? collapse_decide_one<W>(a, frontier, f, chosen) : 0;
+  int total;
+  int off = block_exclusive_scan<int>(nint, total);
+  if (f < fsize) offs[f] = off;
+  if (threadIdx.x == 0) tot[blockIdx.x] = total;
 }
 
 // Pad a box outwards by a relative margin of its coordinates' magnitude, so that rounding in element distances and hit
@@ -420,83 +467,45 @@ __device__ __forceinline__ bool collapse_emit_one(CollapseArgs const & a, int co
 }
 
 template <int W>
-__global__ void collapse_emit_kernel(CollapseArgs a, int * __restrict__ fa, int * __restrict__ fb,
-                                     CollapseLevel * __restrict__ lv, int64_t bound, int const * __restrict__ chosen,
-                                     int const * __restrict__ offsets, int64_t cap, WideNode<W> * __restrict__ nodes) {
-  int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(BUILD_THREADS)
+collapse_emit_kernel(CollapseArgs a, int const * __restrict__ frontier, int * __restrict__ next_frontier,
+                     CollapseLevel const * __restrict__ lv, CollapseLevel * __restrict__ next,
+                     int const * __restrict__ chosen, int const * __restrict__ offs, int const * __restrict__ tot,
+                     int const * __restrict__ scanned, int64_t cap, WideNode<W> * __restrict__ nodes) {
+  __shared__ int s_sum[BUILD_THREADS / 32];
   int64_t fsize = lv->fsize;
-  if (f >= fsize || f >= bound) return;
+  int64_t f0 = (int64_t)blockIdx.x * BUILD_THREADS;
+  if (f0 >= fsize && blockIdx.x > 0) return;
   int64_t level_base = lv->base;
-  bool par = lv->parity != 0;
-  if (!collapse_emit_one<W>(a, par ? fb : fa, f, chosen, offsets[f], level_base, level_base + fsize, cap, nodes,
-                            par ? fa : fb))
-    lv->overflow = 1;
-}
-
-// Levels whose frontier fits in one block, one after another in one launch (the top of the tree and its tail): thread f
-// decides and emits frontier node f, a block scan places the internal children. Returns when the frontier is empty or
-// outgrows the block.
-constexpr int COLLAPSE_BLOCK = 1024;
-
-template <int W>
-__global__ void __launch_bounds__(COLLAPSE_BLOCK)
-collapse_small_levels_kernel(CollapseArgs a, int * __restrict__ fa, int * __restrict__ fb,
-                             CollapseLevel * __restrict__ lv, int * __restrict__ chosen, int64_t cap,
-                             WideNode<W> * __restrict__ nodes) {
-  __shared__ int64_t s_fsize, s_base, s_parity;
-  __shared__ int s_bad;
-  int t = threadIdx.x;
-  if (t == 0) {
-    s_fsize = lv->fsize;
-    s_base = lv->base;
-    s_parity = lv->parity;
-    s_bad = 0;
+  int nb = (int)ceil_div(fsize, BUILD_THREADS);
+  // internal children of the blocks before this one; block 0 sums all of them instead, for the next level's size
+  int sum = 0;
+  if (scanned) {
+    if (threadIdx.x == 0) sum = blockIdx.x > 0 ? scanned[blockIdx.x] : (nb > 0 ? scanned[nb - 1] + tot[nb - 1] : 0);
+  } else {
+    int upto = blockIdx.x > 0 ? (int)blockIdx.x : nb;
+    for (int i = threadIdx.x; i < upto; i += BUILD_THREADS) sum += tot[i];
   }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
   __syncthreads();
-  int64_t levels = 0;
-  while (true) {
-    int64_t fsize = s_fsize;
-    if (fsize <= 0 || fsize > COLLAPSE_BLOCK || s_bad) break;
-    bool par = s_parity != 0;
-    int * cur = par ? fb : fa;
-    int * nxt = par ? fa : fb;
-    int nint = t < fsize ? collapse_decide_one<W>(a, cur, t, chosen) : 0;
-    int total = 0;
-    int off = block_exclusive_scan<int>(nint, total);
-    if (t < fsize && !collapse_emit_one<W>(a, cur, t, chosen, off, s_base, s_base + fsize, cap, nodes, nxt))
-      s_bad = 1;
-    __syncthreads();
-    if (t == 0) {
-      s_base += fsize;
-      s_fsize = total;
-      s_parity = !par;
+  sum = 0;
+#pragma unroll
+  for (int w = 0; w < BUILD_THREADS / 32; ++w) sum += s_sum[w];
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      next->fsize = sum;
+      next->base = level_base + fsize;
+      next->levels = lv->levels + (fsize > 0 ? 1 : 0);
+      if (lv->overflow) atomicOr((unsigned long long *)&next->overflow, 1ull);
     }
-    ++levels;
-    __syncthreads();
+    sum = 0;
   }
-  if (t == 0) {
-    lv->fsize = s_bad ? 0 : s_fsize;
-    lv->base = s_base;
-    lv->parity = s_parity;
-    lv->levels += levels;
-    if (s_bad) lv->overflow = 1;
-  }
-}
-
-// Moves the device state to the next level: the emitted children form the next frontier
-__global__ void collapse_advance_kernel(CollapseLevel * __restrict__ lv, int64_t bound, int const * __restrict__ offsets,
-                                        int const * __restrict__ num_internal) {
-  int64_t fsize = lv->fsize;
-  if (fsize <= 0) return;
-  if (fsize > bound) {  // the host's bound did not hold: stop, reported as an overflow
-    lv->overflow = 1;
-    lv->fsize = 0;
-    return;
-  }
-  lv->base += fsize;
-  lv->fsize = (int64_t)offsets[fsize - 1] + num_internal[fsize - 1];
-  lv->levels += 1;
-  lv->parity = !lv->parity;
+  int64_t f = f0 + threadIdx.x;
+  if (f >= fsize) return;
+  if (!collapse_emit_one<W>(a, frontier, f, chosen, sum + offs[f], level_base, level_base + fsize, cap, nodes,
+                            next_frontier))
+    atomicOr((unsigned long long *)&next->overflow, 1ull);
 }
 
 // Segment roots: big segments (more elements than a leaf) become level-0 frontier entries; small non-empty segments get
@@ -512,28 +521,51 @@ __global__ void segment_flags_kernel(int64_t const * __restrict__ seg_start, int
 }
 
 template <int W>
+__device__ __forceinline__ void write_leaf_root(WideNode<W> & out, int const * __restrict__ bounds, int count) {
+  WideNode<W> node;
+  clear_node(node);
+  float4 lo = make_float4(ord2f(bounds[6]), ord2f(bounds[7]), ord2f(bounds[8]), 0.f);
+  float4 hi = make_float4(ord2f(bounds[9]), ord2f(bounds[10]), ord2f(bounds[11]), 0.f);
+  pad_box(lo, hi);
+  node.lox[0] = lo.x; node.loy[0] = lo.y; node.loz[0] = lo.z;
+  node.hix[0] = hi.x; node.hiy[0] = hi.y; node.hiz[0] = hi.z;
+  node.child[0] = encode_leaf(0, count);
+  out = node;
+}
+
+// Level 0 of one segment: its root, or the only node when everything fits in a leaf
+template <int W>
+__global__ void single_root_kernel(int64_t n, int leaf_size, int const * __restrict__ bounds,
+                                   WideNode<W> * __restrict__ nodes, int * __restrict__ frontier,
+                                   int * __restrict__ seg_root, CollapseLevel * __restrict__ lv) {
+  bool big = n > leaf_size;
+  if (!big) write_leaf_root<W>(nodes[0], bounds, (int)n);
+  frontier[0] = 0;  // the binary root
+  seg_root[0] = 0;
+  lv[0] = CollapseLevel{big ? 1 : 0, big ? 0 : 1, 0, 0};
+  lv[1].overflow = 0;
+}
+
+template <int W>
 __global__ void segment_roots_kernel(CollapseArgs a, int64_t n, int const * __restrict__ is_small,
                                      int const * __restrict__ small_rank, int const * __restrict__ is_big,
-                                     int const * __restrict__ big_rank, int num_small, int const * __restrict__ bounds,
+                                     int const * __restrict__ big_rank, int const * __restrict__ bounds,
                                      WideNode<W> * __restrict__ nodes, int * __restrict__ frontier,
-                                     int * __restrict__ seg_root) {
+                                     int * __restrict__ seg_root, CollapseLevel * __restrict__ lv) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.M) return;
-  int64_t sa = a.seg_start ? a.seg_start[s] : 0, sb = a.seg_start ? a.seg_start[s + 1] : n;
+  int num_small = small_rank[a.M - 1] + is_small[a.M - 1];
+  if (s == 0) {
+    lv[0] = CollapseLevel{big_rank[a.M - 1] + is_big[a.M - 1], num_small, 0, 0};
+    lv[1].overflow = 0;
+  }
+  int64_t sa = a.seg_start[s], sb = a.seg_start[s + 1];
   if (is_big[s]) {
     // the Karras root of the segment is the internal node at its first position, slot sa - s
     frontier[big_rank[s]] = (int)(sa - s);
     seg_root[s] = num_small + big_rank[s];
   } else if (is_small[s]) {
-    WideNode<W> node;
-    clear_node(node);
-    float4 lo = make_float4(ord2f(bounds[12 * s + 6]), ord2f(bounds[12 * s + 7]), ord2f(bounds[12 * s + 8]), 0.f);
-    float4 hi = make_float4(ord2f(bounds[12 * s + 9]), ord2f(bounds[12 * s + 10]), ord2f(bounds[12 * s + 11]), 0.f);
-    pad_box(lo, hi);
-    node.lox[0] = lo.x; node.loy[0] = lo.y; node.loz[0] = lo.z;
-    node.hix[0] = hi.x; node.hiy[0] = hi.y; node.hiz[0] = hi.z;
-    node.child[0] = encode_leaf(0, (int)(sb - sa));
-    nodes[small_rank[s]] = node;
+    write_leaf_root<W>(nodes[small_rank[s]], bounds + 12 * (int64_t)s, (int)(sb - sa));
     seg_root[s] = small_rank[s];
   } else {
     seg_root[s] = -1;  // empty segment
@@ -549,7 +581,7 @@ __global__ void count_big_kernel(int const * __restrict__ first, int const * __r
 }
 
 // Element records in sorted order; the stored index is the element's index within its segment.
-__global__ void mesh_records_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t n,
+__global__ void mesh_records_kernel(float const * __restrict__ V, int64_t nv, int32_t const * __restrict__ F, int64_t n,
                                     int64_t const * __restrict__ seg_start, int M, uint32_t const * __restrict__ sorted,
                                     float4 * __restrict__ cp_rec, float4 * __restrict__ ray_rec,
                                     int32_t * __restrict__ leaf_to_elem) {
@@ -558,9 +590,10 @@ __global__ void mesh_records_kernel(float const * __restrict__ V, int32_t const 
   int64_t ge = (int64_t)sorted[s];
   int e = (int)(M > 1 ? ge - seg_start[segment_of(seg_start, M, ge)] : ge);
   leaf_to_elem[s] = e;
-  V3 v0 = load_v3(V + 3 * (int64_t)F[3 * ge]);
-  V3 v1 = load_v3(V + 3 * (int64_t)F[3 * ge + 1]);
-  V3 v2 = load_v3(V + 3 * (int64_t)F[3 * ge + 2]);
+  bool out = false;  // (reported by elem_box_kernel)
+  V3 v0 = load_v3(V + 3 * face_vertex(F, 3 * ge, nv, out));
+  V3 v1 = load_v3(V + 3 * face_vertex(F, 3 * ge + 1, nv, out));
+  V3 v2 = load_v3(V + 3 * face_vertex(F, 3 * ge + 2, nv, out));
   if (cp_rec) {
     TriPlane pl = tri_plane(v0, v1, v2);
     V3 d0, d1, d2;
@@ -599,80 +632,106 @@ __global__ void point_records_kernel(float const * __restrict__ P, int64_t n, in
   pt_rec[s] = make_float4(p.x, p.y, p.z, __int_as_float(e));
 }
 
-constexpr int COLLAPSE_LEVELS_PER_SYNC = 6;
+// Blocks of a level up to which the emitting kernel sums the counts of the blocks before it by itself
+constexpr int64_t COLLAPSE_SUM_BLOCKS = 1024;
+// Elements up to which the node array is first sized by the worst case; larger builds count their nodes first
+constexpr int64_t COLLAPSE_BOUND_MAX = 1 << 22;
+
+// What the build reads back, in one copy: the collapse's two alternating levels, whether a face index was out of range,
+// and the bounds of every segment (12 ordered ints each, see elem_box_kernel)
+struct BuildState {
+  CollapseLevel level[2];
+  int bad;
+  int pad[3];
+  __host__ __device__ int * bounds() { return reinterpret_cast<int *>(this + 1); }
+  static size_t bytes(int M) { return sizeof(BuildState) + (size_t)12 * M * sizeof(int); }
+};
 
 template <int W>
-void collapse(thea_bvh * b, CollapseArgs const & a, int64_t n, int const * d_bounds, cudaStream_t stream) {
+void collapse(thea_bvh * b, CollapseArgs const & a, int64_t n, BuildState * state, std::vector<char> & h_state,
+              cudaStream_t stream) {
   int M = a.M;
-  // segment roots
-  Scratch is_small((size_t)M * sizeof(int), stream), is_big((size_t)M * sizeof(int), stream);
-  Scratch small_rank((size_t)M * sizeof(int), stream), big_rank((size_t)M * sizeof(int), stream);
-  THEA_LAUNCH(segment_flags_kernel, (unsigned)ceil_div(M, BUILD_THREADS), BUILD_THREADS, 0, stream, a.seg_start, M, n,
-              a.leaf_size, is_small.as<int>(), is_big.as<int>());
-  exclusive_scan<int>(is_small.as<int>(), small_rank.as<int>(), M, stream);
-  exclusive_scan<int>(is_big.as<int>(), big_rank.as<int>(), M, stream);
-  int tails[4];
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&tails[0], small_rank.as<int>() + M - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&tails[1], is_small.as<int>() + M - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&tails[2], big_rank.as<int>() + M - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&tails[3], is_big.as<int>() + M - 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  // every other wide node corresponds to a distinct binary node with more elements than a leaf holds
-  int64_t m = n - M;  // binary internal nodes in the forest (segments are non-empty)
-  Scratch cnt(sizeof(unsigned long long), stream);
-  THEA_CUDA_CHECK(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes, stream));
-  if (m > 0)
-    THEA_LAUNCH(count_big_kernel, (unsigned)ceil_div(m, BUILD_THREADS), BUILD_THREADS, 0, stream, a.first, a.last, m,
-                a.leaf_size, cnt.as<unsigned long long>());
-  unsigned long long nbig = 0;
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&nbig, cnt.ptr, sizeof(nbig), cudaMemcpyDeviceToHost, stream));
-  THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
-  int num_small = tails[0] + tails[1], num_big = tails[2] + tails[3];
-  int64_t cap = (int64_t)num_small + (int64_t)std::max<unsigned long long>(nbig, 1);
-
-  WideNode<W> * nodes = nullptr;
-  THEA_CUDA_CHECK(thea_malloc_async((void **)&nodes, (size_t)cap * sizeof(WideNode<W>), stream));
-  THEA_CUDA_CHECK(thea_malloc_async((void **)&b->seg_root, (size_t)M * sizeof(int32_t), stream));
-  Scratch fa((size_t)std::max<int64_t>(cap, 1) * sizeof(int), stream), fb((size_t)std::max<int64_t>(cap, 1) * sizeof(int), stream);
-  THEA_LAUNCH((segment_roots_kernel<W>), (unsigned)ceil_div(M, BUILD_THREADS), BUILD_THREADS, 0, stream, a, n,
-              is_small.as<int>(), small_rank.as<int>(), is_big.as<int>(), big_rank.as<int>(), num_small, d_bounds,
-              nodes, fa.as<int>(), b->seg_root);
-  Scratch chosen((size_t)std::max<int64_t>(cap, 1) * W * sizeof(int), stream);
-  Scratch nint((size_t)std::max<int64_t>(cap, 1) * sizeof(int), stream);
-  Scratch offs((size_t)std::max<int64_t>(cap, 1) * sizeof(int), stream);
-  int depth = num_small > 0 ? 1 : 0;
-  // Levels whose frontier fits in one block run in one launch (collapse_small_levels_kernel); larger ones run
-  // COLLAPSE_LEVELS_PER_SYNC at a time, a few launches each, on the device state, with the host bounding each frontier
-  // (a frontier node has at most W internal children, and no level holds more than the nbig wide internal nodes) to
-  // size the launches and the scan. Levels past the last one find an empty frontier and do nothing.
-  CollapseLevel h{num_big, num_small, 0, 0, 0};
-  Scratch lv(sizeof(CollapseLevel), stream);
-  THEA_CUDA_CHECK(cudaMemcpyAsync(lv.ptr, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
-  int64_t limit = std::max<int64_t>((int64_t)nbig, 1);
-  while (h.fsize > 0) {
-    int64_t bound = h.fsize;
-    if (bound <= COLLAPSE_BLOCK) {
-      THEA_LAUNCH(collapse_small_levels_kernel<W>, 1, COLLAPSE_BLOCK, 0, stream, a, fa.as<int>(), fb.as<int>(),
-                  lv.as<CollapseLevel>(), chosen.as<int>(), cap, nodes);
-      bound = 0;  // read the state back before choosing the next step
-    }
-    for (int l = 0; l < COLLAPSE_LEVELS_PER_SYNC && bound > 0; ++l) {
-      unsigned grid = (unsigned)ceil_div(bound, BUILD_THREADS);
-      THEA_LAUNCH(collapse_decide_kernel<W>, grid, BUILD_THREADS, 0, stream, a, fa.as<int>(), fb.as<int>(),
-                  lv.as<CollapseLevel>(), bound, chosen.as<int>(), nint.as<int>());
-      exclusive_scan<int>(nint.as<int>(), offs.as<int>(), bound, stream);
-      THEA_LAUNCH(collapse_emit_kernel<W>, grid, BUILD_THREADS, 0, stream, a, fa.as<int>(), fb.as<int>(),
-                  lv.as<CollapseLevel>(), bound, chosen.as<int>(), offs.as<int>(), cap, nodes);
-      THEA_LAUNCH(collapse_advance_kernel, 1, 1, 0, stream, lv.as<CollapseLevel>(), bound, offs.as<int>(),
-                  nint.as<int>());
-      bound = std::min<int64_t>(bound * W, limit);
-    }
-    THEA_CUDA_CHECK(cudaMemcpyAsync(&h, lv.ptr, sizeof(h), cudaMemcpyDeviceToHost, stream));
+  // Wide nodes: every one but a small segment's root stands for a binary node with more elements than a leaf holds. At
+  // most one per leaf + 1 elements has fewer than W children, all of them leaves; the others have W, so there are at most
+  // (n - 1) / (W - 1) of them.
+  int64_t cap = (n - 1) / (W - 1) + n / (a.leaf_size + 1) + M + 1;
+  bool exact = n > COLLAPSE_BOUND_MAX;
+  if (exact) {
+    int64_t m = n - M;  // binary internal nodes in the forest (segments are non-empty)
+    Scratch cnt(sizeof(unsigned long long), stream);
+    THEA_CUDA_CHECK(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes, stream));
+    if (m > 0)
+      THEA_LAUNCH(count_big_kernel, (unsigned)ceil_div(m, BUILD_THREADS), BUILD_THREADS, 0, stream, a.first, a.last, m,
+                  a.leaf_size, cnt.as<unsigned long long>());
+    unsigned long long nbig = 0;
+    THEA_CUDA_CHECK(cudaMemcpyAsync(&nbig, cnt.ptr, sizeof(nbig), cudaMemcpyDeviceToHost, stream));
     THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
-    THEA_REQUIRE(!h.overflow, "BVH collapse exceeded its node bound");
+    cap = std::min<int64_t>(cap, (int64_t)nbig + M);
   }
-  b->nodes = nodes;
+  Scratch bound_nodes;
+  WideNode<W> * nodes = nullptr;
+  if (exact) {
+    THEA_CUDA_CHECK(thea_malloc_async((void **)&nodes, (size_t)cap * sizeof(WideNode<W>), stream));
+    b->nodes = nodes;
+  } else {
+    bound_nodes = Scratch((size_t)cap * sizeof(WideNode<W>), stream);
+    nodes = bound_nodes.as<WideNode<W>>();
+  }
+  THEA_CUDA_CHECK(thea_malloc_async((void **)&b->seg_root, (size_t)M * sizeof(int32_t), stream));
+  int64_t blocks_cap = ceil_div(cap, BUILD_THREADS);
+  Scratch fr((size_t)cap * 2 * sizeof(int), stream), chosen((size_t)cap * W * sizeof(int), stream);
+  Scratch offs((size_t)cap * sizeof(int), stream), tot((size_t)blocks_cap * 2 * sizeof(int), stream);
+  int * frontier[2] = {fr.as<int>(), fr.as<int>() + cap};
+  CollapseLevel * level = state->level;  // (device addresses)
+  int const * d_bounds = state->bounds();
+  if (M == 1) {
+    THEA_LAUNCH(single_root_kernel<W>, 1, 1, 0, stream, n, a.leaf_size, d_bounds, nodes, frontier[0], b->seg_root, level);
+  } else {
+    Scratch is_small((size_t)M * sizeof(int), stream), is_big((size_t)M * sizeof(int), stream);
+    Scratch small_rank((size_t)M * sizeof(int), stream), big_rank((size_t)M * sizeof(int), stream);
+    THEA_LAUNCH(segment_flags_kernel, (unsigned)ceil_div(M, BUILD_THREADS), BUILD_THREADS, 0, stream, a.seg_start, M, n,
+                a.leaf_size, is_small.as<int>(), is_big.as<int>());
+    exclusive_scan<int>(is_small.as<int>(), small_rank.as<int>(), M, stream);
+    exclusive_scan<int>(is_big.as<int>(), big_rank.as<int>(), M, stream);
+    THEA_LAUNCH((segment_roots_kernel<W>), (unsigned)ceil_div(M, BUILD_THREADS), BUILD_THREADS, 0, stream, a, n,
+                is_small.as<int>(), small_rank.as<int>(), is_big.as<int>(), big_rank.as<int>(), d_bounds, nodes,
+                frontier[0], b->seg_root, level);
+  }
+  // As many levels as a balanced tree and a few more, then the state is read; a deeper tree takes further rounds. Levels
+  // past the last one find an empty frontier and do nothing.
+  int64_t bound = M;
+  int run = 4;
+  for (int64_t m = n / M; m > a.leaf_size; m /= W) ++run;
+  CollapseLevel h{0, 0, 0, 0};
+  int par = 0;
+  do {
+    for (int l = 0; l < run; ++l) {
+      unsigned grid = (unsigned)ceil_div(bound, BUILD_THREADS);
+      int * scanned = grid > COLLAPSE_SUM_BLOCKS ? tot.as<int>() + blocks_cap : nullptr;
+      THEA_LAUNCH(collapse_decide_kernel<W>, grid, BUILD_THREADS, 0, stream, a, frontier[par], level + par,
+                  chosen.as<int>(), offs.as<int>(), tot.as<int>());
+      if (scanned) exclusive_scan<int>(tot.as<int>(), scanned, grid, stream);
+      THEA_LAUNCH(collapse_emit_kernel<W>, grid, BUILD_THREADS, 0, stream, a, frontier[par], frontier[par ^ 1],
+                  level + par, level + (par ^ 1), chosen.as<int>(), offs.as<int>(), tot.as<int>(), scanned, cap, nodes);
+      bound = std::min<int64_t>(bound * W, cap);
+      par ^= 1;
+    }
+    THEA_CUDA_CHECK(cudaMemcpyAsync(h_state.data(), state, h_state.size(), cudaMemcpyDeviceToHost, stream));
+    THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
+    BuildState hs;
+    memcpy(&hs, h_state.data(), sizeof(hs));
+    h = hs.level[par];
+    THEA_REQUIRE(!hs.bad, "build: a face index lies outside [0, num_vertices)");
+    THEA_REQUIRE(!h.overflow, "BVH collapse exceeded its node bound");
+    run = 8;
+  } while (h.fsize > 0);
+  if (!exact) {
+    THEA_CUDA_CHECK(thea_malloc_async(&b->nodes, (size_t)h.base * sizeof(WideNode<W>), stream));
+    THEA_CUDA_CHECK(cudaMemcpyAsync(b->nodes, nodes, (size_t)h.base * sizeof(WideNode<W>), cudaMemcpyDeviceToDevice,
+                                    stream));
+  }
   b->num_nodes = h.base;
-  b->depth = std::max<int>(depth, (int)h.levels);
+  b->depth = (int)std::max<int64_t>(1, h.levels);
 }
 
 }  // namespace
@@ -703,7 +762,7 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
     starts = {0, n};
   }
 
-  if (is_mesh) check_face_indices(F, n_elems, nv, "build", stream);
+  THEA_REQUIRE(!is_mesh || nv > 0, "build: a face index lies outside [0, num_vertices)");
 
   thea_bvh * b = new thea_bvh;
   try {
@@ -718,17 +777,22 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
     b->seg_start_host = starts;
 
     THEA_CUDA_CHECK(thea_malloc_async((void **)&b->seg_start, (size_t)(M + 1) * sizeof(int64_t), stream));
-    THEA_CUDA_CHECK(cudaMemcpyAsync(b->seg_start, starts.data(), (size_t)(M + 1) * sizeof(int64_t),
-                                    cudaMemcpyHostToDevice, stream));
+    THEA_CUDA_CHECK(thea_malloc_async((void **)&b->err, sizeof(unsigned), stream));
+    b->err_host = take_host_word();
+    if (M > 1)
+      THEA_CUDA_CHECK(cudaMemcpyAsync(b->seg_start, starts.data(), (size_t)(M + 1) * sizeof(int64_t),
+                                      cudaMemcpyHostToDevice, stream));
     int64_t const * seg = b->seg_start;
 
     Scratch elo((size_t)n * sizeof(float4), stream), ehi((size_t)n * sizeof(float4), stream);
-    Scratch bounds((size_t)12 * M * sizeof(int), stream);
-    THEA_LAUNCH(init_bounds_kernel, (unsigned)ceil_div(12 * (int64_t)M, BUILD_THREADS), BUILD_THREADS, 0, stream,
-                bounds.as<int>(), M);
+    Scratch state_buf(BuildState::bytes(M), stream);
+    BuildState * state = state_buf.as<BuildState>();
+    int * bounds = state->bounds();
+    THEA_LAUNCH(build_init_kernel, (unsigned)ceil_div(12 * (int64_t)M, BUILD_THREADS), BUILD_THREADS, 0, stream,
+                bounds, M, &state->bad, b->err, b->seg_start, n);
     unsigned grid = (unsigned)ceil_div(n, BUILD_THREADS);
-    THEA_LAUNCH(elem_box_kernel, grid, BUILD_THREADS, 0, stream, V, F, n, is_mesh ? 1 : 0, seg, M, elo.as<float4>(),
-                ehi.as<float4>(), bounds.as<int>());
+    THEA_LAUNCH(elem_box_kernel, grid, BUILD_THREADS, 0, stream, V, nv, F, n, is_mesh ? 1 : 0, seg, M, elo.as<float4>(),
+                ehi.as<float4>(), bounds, &state->bad);
 
     int segbits = 0;
     while ((int64_t(1) << segbits) < M) ++segbits;
@@ -736,8 +800,8 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
     int mbits = 3 * bpa;
     Scratch keys((size_t)n * sizeof(uint64_t), stream), vals((size_t)n * sizeof(uint32_t), stream);
     THEA_LAUNCH(morton_kernel, grid, BUILD_THREADS, 0, stream, elo.as<float4>(), ehi.as<float4>(), n, seg, M,
-                bounds.as<int>(), bpa, keys.as<uint64_t>(), vals.as<uint32_t>());
-    radix_sort_pairs(keys.as<uint64_t>(), vals.as<uint32_t>(), n, mbits + segbits, stream);
+                bounds, bpa, keys.as<uint64_t>(), vals.as<uint32_t>());
+    radix_sort_pairs(keys.as<uint64_t>(), vals.as<uint32_t>(), n, mbits + segbits, stream, /*probe_passes=*/false);
 
     int64_t m = n - M;  // binary internal nodes
     size_t mm = (size_t)std::max<int64_t>(m, 1);
@@ -747,31 +811,27 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
     Scratch ilo(mm * sizeof(float4), stream), ihi(mm * sizeof(float4), stream);
     Scratch visits(mm * sizeof(unsigned), stream);
     if (m >= 1) {
-      THEA_CUDA_CHECK(cudaMemsetAsync(parent.ptr, 0xff, (size_t)m * sizeof(int), stream));
-      THEA_CUDA_CHECK(cudaMemsetAsync(leaf_parent.ptr, 0xff, (size_t)n * sizeof(int), stream));
-      THEA_CUDA_CHECK(cudaMemsetAsync(visits.ptr, 0, (size_t)m * sizeof(unsigned), stream));
       THEA_LAUNCH(karras_kernel, grid, BUILD_THREADS, 0, stream, keys.as<uint64_t>(), n, seg, M, mbits,
                   left.as<int>(), right.as<int>(), first.as<int>(), last.as<int>(), parent.as<int>(),
-                  leaf_parent.as<int>());
-      THEA_LAUNCH(refit_kernel, grid, BUILD_THREADS, 0, stream, n, left.as<int>(), right.as<int>(), parent.as<int>(),
-                  leaf_parent.as<int>(), elo.as<float4>(), ehi.as<float4>(), vals.as<uint32_t>(), ilo.as<float4>(),
+                  leaf_parent.as<int>(), visits.as<unsigned>());
+      THEA_LAUNCH(refit_kernel, grid, BUILD_THREADS, 0, stream, n, left.as<int>(), right.as<int>(), first.as<int>(),
+                  last.as<int>(), parent.as<int>(), leaf_parent.as<int>(), elo.as<float4>(), ehi.as<float4>(), vals.as<uint32_t>(), ilo.as<float4>(),
                   ihi.as<float4>(), visits.as<unsigned>());
     }
     CollapseArgs a{left.as<int>(), right.as<int>(), first.as<int>(), last.as<int>(), elo.as<float4>(),
                    ehi.as<float4>(), vals.as<uint32_t>(), ilo.as<float4>(), ihi.as<float4>(),
                    M > 1 ? seg : nullptr, M, leaf};
-    if (width == 4) collapse<4>(b, a, n, bounds.as<int>(), stream);
-    else collapse<8>(b, a, n, bounds.as<int>(), stream);
+    std::vector<char> h_state(BuildState::bytes(M));
+    if (width == 4) collapse<4>(b, a, n, state, h_state, stream);
+    else collapse<8>(b, a, n, state, h_state, stream);
+    std::vector<int> hb((size_t)12 * M);
+    memcpy(hb.data(), h_state.data() + sizeof(BuildState), hb.size() * sizeof(int));
     int64_t node_bytes = b->num_nodes * (width == 4 ? (int64_t)sizeof(WideNode<4>) : (int64_t)sizeof(WideNode<8>));
 
     int need = b->depth * (width - 1) + 1;
     if (need > (width == 4 ? 256 : 512))
       throw Error(THEA_ERR_NOT_SUPPORTED, "build: tree too deep for the traversal stack (depth " +
                                               std::to_string(b->depth) + ")");
-    THEA_CUDA_CHECK(thea_malloc_async((void **)&b->err, sizeof(unsigned), stream));
-    THEA_CUDA_CHECK(cudaMemsetAsync(b->err, 0, sizeof(unsigned), stream));
-    THEA_CUDA_CHECK(thea_malloc_host(&b->err_host, sizeof(unsigned)));
-    *b->err_host = 0;
     THEA_CUDA_CHECK(thea_malloc_async((void **)&b->leaf_to_elem, (size_t)n * sizeof(int32_t), stream));
     int64_t rec_bytes = n * (int64_t)sizeof(int32_t);
     if (is_mesh) {
@@ -784,7 +844,7 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
                                           stream));
         rec_bytes += n * RAY_REC_F4 * (int64_t)sizeof(float4);
       }
-      THEA_LAUNCH(mesh_records_kernel, grid, BUILD_THREADS, 0, stream, V, F, n, seg, M, vals.as<uint32_t>(),
+      THEA_LAUNCH(mesh_records_kernel, grid, BUILD_THREADS, 0, stream, V, nv, F, n, seg, M, vals.as<uint32_t>(),
                   b->cp_rec, b->ray_rec, b->leaf_to_elem);
     } else {
       THEA_CUDA_CHECK(thea_malloc_async((void **)&b->pt_rec, (size_t)n * sizeof(float4), stream));
@@ -792,9 +852,6 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
       THEA_LAUNCH(point_records_kernel, grid, BUILD_THREADS, 0, stream, V, n, seg, M, vals.as<uint32_t>(), b->pt_rec,
                   b->leaf_to_elem);
     }
-    std::vector<int> hb((size_t)12 * M);
-    THEA_CUDA_CHECK(cudaMemcpyAsync(hb.data(), bounds.ptr, hb.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
-    THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
     b->seg_lo.resize((size_t)3 * M);
     b->seg_hi.resize((size_t)3 * M);
     for (int s = 0; s < M; ++s)
@@ -813,6 +870,7 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
     b->device_bytes = node_bytes + rec_bytes;
     init_segment_roots(b, stream);
     init_slabs(b, stream);
+    THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
     if (b->slabs) b->device_bytes += b->num_nodes * width * (int64_t)sizeof(float4);
     return b;
   } catch (...) {
@@ -1039,7 +1097,7 @@ static void build_slabs(thea_bvh * b, cudaStream_t stream) {
   THEA_CUDA_CHECK(cudaMemcpyAsync(&h, bad.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream));
   THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
   if (h) {
-    cudaFree(b->slabs);
+    cudaFreeAsync(b->slabs, stream);
     b->slabs = nullptr;  // searches use boxes alone
   }
 }
@@ -1060,11 +1118,9 @@ void init_segment_roots(thea_bvh * b, cudaStream_t stream) {
   int M = b->num_segments;
   std::vector<RootCut> h((size_t)M);
   for (int s = 0; s < M; ++s) h[(size_t)s] = root_cut_of(&b->seg_lo[3 * (size_t)s], &b->seg_hi[3 * (size_t)s], nullptr);
-  if (b->seg_roots) cudaFree(b->seg_roots);
-  b->seg_roots = nullptr;
-  THEA_CUDA_CHECK(thea_malloc(&b->seg_roots, (size_t)M * sizeof(RootCut)));
+  if (!b->seg_roots) THEA_CUDA_CHECK(thea_malloc_async(&b->seg_roots, (size_t)M * sizeof(RootCut), stream));
+  // (pageable memory: the copy has read h when the call returns)
   THEA_CUDA_CHECK(cudaMemcpyAsync(b->seg_roots, h.data(), (size_t)M * sizeof(RootCut), cudaMemcpyHostToDevice, stream));
-  THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
 }
 
 void check_face_indices(int32_t const * F, int64_t nf, int64_t nv, char const * what, cudaStream_t stream) {
@@ -1096,17 +1152,12 @@ void destroy_bvh(thea_bvh * b) {
   cudaGetDevice(&prev);
   cudaSetDevice(b->device);
   cudaDeviceSynchronize();
-  if (b->nodes) cudaFree(b->nodes);
-  if (b->cp_rec) cudaFree(b->cp_rec);
-  if (b->slabs) cudaFree(b->slabs);
-  if (b->ray_rec) cudaFree(b->ray_rec);
-  if (b->pt_rec) cudaFree(b->pt_rec);
-  if (b->leaf_to_elem) cudaFree(b->leaf_to_elem);
-  if (b->err) cudaFree(b->err);
-  if (b->err_host) cudaFreeHost(b->err_host);
-  if (b->seg_start) cudaFree(b->seg_start);
-  if (b->seg_root) cudaFree(b->seg_root);
-  if (b->seg_roots) cudaFree(b->seg_roots);
+  // the device is idle: the arrays go back to the library's pool for the next handle
+  for (void * p : {b->nodes, (void *)b->cp_rec, (void *)b->slabs, (void *)b->ray_rec, (void *)b->pt_rec,
+                   (void *)b->leaf_to_elem, (void *)b->err, (void *)b->seg_start, (void *)b->seg_root,
+                   (void *)b->seg_roots})
+    if (p) cudaFreeAsync(p, (cudaStream_t)0);
+  if (b->err_host) release_host_word(b->err_host);
   if (prev >= 0) cudaSetDevice(prev);
   delete b;
 }

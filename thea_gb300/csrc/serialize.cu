@@ -158,12 +158,12 @@ thea_bvh * deserialize_bvh(void const * in, int64_t bytes, cudaStream_t s) {
     std::memcpy(b->seg_hi.data(), p, (size_t)M * 12);
     THEA_CUDA_CHECK(thea_malloc_async((void **)&b->err, sizeof(unsigned), s));
     THEA_CUDA_CHECK(cudaMemsetAsync(b->err, 0, sizeof(unsigned), s));
-    THEA_CUDA_CHECK(thea_malloc_host(&b->err_host, sizeof(unsigned)));
-    *b->err_host = 0;
+    b->err_host = take_host_word();
     // the host image may be reused by the caller as soon as this returns
     THEA_CUDA_CHECK(cudaStreamSynchronize(s));
     init_segment_roots(b, s);
     init_slabs(b, s);
+    THEA_CUDA_CHECK(cudaStreamSynchronize(s));
     if (h.has_transform) set_transform(b, h.xf, s);
     return b;
   } catch (...) {
