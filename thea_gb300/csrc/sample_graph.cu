@@ -451,108 +451,144 @@ void run_sample_graph_oversampled(float const * positions, float const * normals
 namespace thea {
 namespace {
 
+// The running sum in three launches. The terms are cut into windows of RSUM_WINDOW. All SMs first sum each window roughly
+// (rsum_parts_kernel), which locates the running sum at every window to within a few rounding errors, then add up each
+// window's units in the one or two binades it can lie in (rsum_units_kernel). One block then walks the windows
+// (rsum_walk_kernel): a block scan over 1,024 windows finds how far the sum can move in whole windows, and a window that
+// it cannot take whole (a binade crossing, a tie, a term to be taken alone, an estimate that was off) is added one
+// fl(s + x) at a time by one thread, from shared memory. A sequence has one crossing and about one tie per binade, so some
+// twenty windows of 2,048 terms at 4 us each, and as many scans; what bounds it is that chain of dependent additions. (One
+// block walking 16,384-term windows with a scan each: 862 us for 1.96 M terms; this form 120 us for the walk and 12 before
+// it. A warp walking 256-term sub-windows was slower than that block.)
 constexpr int RSUM_THREADS = 1024;
-constexpr int RSUM_ITEMS = 16;  // consecutive terms per thread; the cursor moves in multiples of it
-constexpr int64_t RSUM_WINDOW = (int64_t)RSUM_THREADS * RSUM_ITEMS;
+constexpr int RSUM_UNIT_THREADS = 256;
+constexpr int RSUM_WINDOW = 2048;
 
-// Units of a thread's 16 terms in binade e; false if one of them has to be taken on its own
-__device__ __forceinline__ bool rsum_group_units(float4 const (&v)[RSUM_ITEMS / 4], int e, long long & units) {
-  bool ok = true;
-  units = 0;
+// Units of a window's terms in binade e and in binade e + 1 (negative: a term has to be taken on its own)
+struct RsumWindow {
+  long long units[2];
+  int e;
+  int pad;
+};
+
+__device__ __forceinline__ int64_t rsum_count(int64_t const * count, int64_t n_host) { return count ? *count : n_host; }
+
+__global__ void __launch_bounds__(RSUM_UNIT_THREADS)
+rsum_parts_kernel(float const * __restrict__ x, int64_t const * __restrict__ count, int64_t n_host,
+                  float * __restrict__ part) {
+  __shared__ float s_sum[RSUM_UNIT_THREADS / 32];
+  int64_t n = rsum_count(count, n_host);
+  int64_t w0 = (int64_t)blockIdx.x * RSUM_WINDOW;
+  float sum = 0.f;
+  for (int64_t j = w0 + threadIdx.x; j < w0 + RSUM_WINDOW && j < n; j += RSUM_UNIT_THREADS) sum += x[j];
 #pragma unroll
-  for (int i = 0; i < RSUM_ITEMS / 4; ++i) {
-    long long d0 = 0, d1 = 0, d2 = 0, d3 = 0;
-    ok = ok && running_sum_step_units(e, v[i].x, d0) && running_sum_step_units(e, v[i].y, d1) &&
-         running_sum_step_units(e, v[i].z, d2) && running_sum_step_units(e, v[i].w, d3);
-    units += d0 + d1 + d2 + d3;
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sum = 0.f;
+    for (int w = 0; w < RSUM_UNIT_THREADS / 32; ++w) sum += s_sum[w];
+    part[blockIdx.x] = sum;
   }
-  return ok;
 }
 
-// One block walks the terms in windows of RSUM_THREADS x RSUM_ITEMS. Each thread sums the units of its 16 terms in the
-// binade of the sum at the window's start; a block scan over the threads finds the first group that cannot be added in
-// bulk (a term to be taken alone, or a total past RUNNING_SUM_MAX_UNITS). Every group before it is added as one integer
-// sum, that group's 16 terms one fl(s + x) at a time, and the next window starts after it. Each thread loads its
-// group of the following window while the current one is scanned, and keeps it when the window was taken whole.
+__global__ void __launch_bounds__(RSUM_UNIT_THREADS)
+rsum_units_kernel(float const * __restrict__ x, int64_t const * __restrict__ count, int64_t n_host, float s0,
+                  float const * __restrict__ before, RsumWindow * __restrict__ out) {
+  __shared__ long long s_u[2][RSUM_UNIT_THREADS / 32];
+  int64_t n = rsum_count(count, n_host);
+  int64_t w0 = (int64_t)blockIdx.x * RSUM_WINDOW;
+  if (w0 >= n) return;
+  // the lower of the two binades: that of the estimate less what rounding may have taken off the sum
+  int e = 0;
+  bool known = running_sum_binade((s0 + before[blockIdx.x]) * (63.0f / 64.0f), e);
+  long long u[2] = {0, 0};
+  bool ok[2] = {known, known};
+  if (known) {
+    for (int64_t j = w0 + threadIdx.x; j < w0 + RSUM_WINDOW && j < n; j += RSUM_UNIT_THREADS) {
+      float v = x[j];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        long long d = 0;
+        ok[c] = running_sum_step_units(e + c, v, d) && ok[c];
+        u[c] += d;
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    bool all = __syncthreads_and(ok[c]);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
+    if ((threadIdx.x & 31) == 0) s_u[c][threadIdx.x >> 5] = u[c];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      long long sum = 0;
+      for (int w = 0; w < RSUM_UNIT_THREADS / 32; ++w) sum += s_u[c][w];
+      out[blockIdx.x].units[c] = all ? sum : -1;
+      out[blockIdx.x].e = e;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(RSUM_THREADS)
-running_sum_kernel(float const * __restrict__ x, int64_t const * __restrict__ count, int64_t n_host, float s0,
-                   float * __restrict__ out) {
+rsum_walk_kernel(float const * __restrict__ x, int64_t const * __restrict__ count, int64_t n_host, float s0,
+                 RsumWindow const * __restrict__ win, float * __restrict__ out) {
   __shared__ float s_sum;
-  __shared__ int64_t s_cursor;
   __shared__ int s_first;
-  int64_t n = count ? *count : n_host;
+  __shared__ long long s_units;
+  __shared__ float4 s_x[RSUM_WINDOW / 4];
+  int64_t n = rsum_count(count, n_host);
+  int64_t windows = (n + RSUM_WINDOW - 1) / RSUM_WINDOW;
   int t = threadIdx.x;
-  if (t == 0) {
-    s_sum = s0;
-    s_cursor = 0;
-  }
-  __syncthreads();
-  float4 v[RSUM_ITEMS / 4], nv[RSUM_ITEMS / 4];
-  int64_t have = -1;  // window start whose group is in v
-  while (true) {
-    int64_t cur = s_cursor;
-    float s = s_sum;
-    if (cur >= n) break;
+  float s = s0;
+  for (int64_t w = 0; w < windows;) {
+    // whole windows, as far as they go
     int e = 0;
-    bool bulk = running_sum_binade(s, e);
-    int64_t g0 = cur + (int64_t)t * RSUM_ITEMS;
-    bool full = g0 + RSUM_ITEMS <= n;
-    if (full && have != cur) {
-      float4 const * p = reinterpret_cast<float4 const *>(x + g0);
-#pragma unroll
-      for (int i = 0; i < RSUM_ITEMS / 4; ++i) v[i] = p[i];
-    }
-    int64_t g1 = g0 + RSUM_WINDOW;
-    bool next_full = g1 + RSUM_ITEMS <= n;
-    if (next_full) {
-      float4 const * p = reinterpret_cast<float4 const *>(x + g1);
-#pragma unroll
-      for (int i = 0; i < RSUM_ITEMS / 4; ++i) nv[i] = p[i];
-    }
-    long long units = 0;
-    bool ok = bulk;
-    if (bulk && g0 < n) {
-      if (full) {
-        ok = rsum_group_units(v, e, units);
-      } else {
-        for (int64_t j = g0; j < n; ++j) {
-          long long d = 0;
-          ok = ok && running_sum_step_units(e, x[j], d);
-          units += d;
-        }
+    bool bulk = running_sum_binade(s, e);  // (the same for every thread)
+    if (bulk) {
+      long long units = -1;
+      if (w + t < windows) {
+        RsumWindow const & q = win[w + t];
+        int c = e - q.e;
+        if (c == 0 || c == 1) units = q.units[c];
       }
+      if (t == 0) s_first = RSUM_THREADS;
+      long long total;
+      long long before = block_exclusive_scan<long long>(units < 0 ? 0 : units, total);
+      long long base = running_sum_units_of(s, e);
+      if (units < 0 || base + before + units > RUNNING_SUM_MAX_UNITS) atomicMin(&s_first, t);
+      __syncthreads();
+      int g = s_first;
+      if (g == RSUM_THREADS ? t == RSUM_THREADS - 1 : t == g) s_units = base + before + (g == RSUM_THREADS ? units : 0);
+      __syncthreads();
+      if (g > 0) s = running_sum_from_units(s_units, e);
+      w += g;
+      if (g == RSUM_THREADS) continue;
+      if (w >= windows) break;
     }
-    long long total = 0;
-    long long before = block_exclusive_scan<long long>(units, total);
-    long long base = bulk ? running_sum_units_of(s, e) : 0;
-    bool fits = ok && base + before + units <= RUNNING_SUM_MAX_UNITS;
-    if (t == 0) s_first = RSUM_THREADS;
+    // the window that stopped it, term by term
+    int64_t w0 = w * RSUM_WINDOW;
+    int m = (int)(n - w0 < RSUM_WINDOW ? n - w0 : RSUM_WINDOW);
+    float * sx = reinterpret_cast<float *>(s_x);
+    for (int j = t; j < RSUM_WINDOW; j += RSUM_THREADS) sx[j] = j < m ? x[w0 + j] : 0.f;
     __syncthreads();
-    if (!fits && g0 < n) atomicMin(&s_first, t);
-    __syncthreads();
-    int g = s_first;
-    if (t == (g < RSUM_THREADS ? g : RSUM_THREADS - 1)) {
-      if (g < RSUM_THREADS) {
-        if (bulk && before > 0) s = running_sum_from_units(base + before, e);
-        int64_t end = g0 + RSUM_ITEMS < n ? g0 + RSUM_ITEMS : n;
-        for (int64_t j = g0; j < end; ++j) s = __fadd_rn(s, x[j]);
-        s_cursor = end;
-      } else {
-        s = running_sum_from_units(base + before + units, e);
-        s_cursor = cur + RSUM_WINDOW;
+    if (t == 0) {
+      float r = s;
+      int j = 0;
+#pragma unroll 8
+      for (; j + 4 <= m; j += 4) {
+        float4 v = s_x[j / 4];
+        r = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(r, v.x), v.y), v.z), v.w);
       }
-      s_sum = s;
-    }
-    if (g == RSUM_THREADS && next_full) {
-#pragma unroll
-      for (int i = 0; i < RSUM_ITEMS / 4; ++i) v[i] = nv[i];
-      have = cur + RSUM_WINDOW;
-    } else {
-      have = -1;
+      for (; j < m; ++j) r = __fadd_rn(r, sx[j]);
+      s_sum = r;
     }
     __syncthreads();
+    s = s_sum;
+    ++w;
   }
-  if (t == 0) *out = s_sum;
+  if (t == 0) *out = s;
 }
 
 // Offsets of each sample's separations in the compact sequence (exclusive scan of the degrees, done before) -> the
@@ -576,9 +612,16 @@ __global__ void mean_of_sum_kernel(float * __restrict__ sum, int64_t const * __r
 
 }  // namespace
 
+// n: the number of terms, or with `count` (device) a bound on it
 void run_running_sum(float const * x, int64_t const * count, int64_t n, float s0, float * out, cudaStream_t s) {
   THEA_REQUIRE(((uintptr_t)x & 15) == 0, "running_sum: terms must be 16-byte aligned");
-  THEA_LAUNCH(running_sum_kernel, 1, RSUM_THREADS, 0, s, x, count, n, s0, out);
+  int64_t windows = std::max<int64_t>(1, ceil_div(n, RSUM_WINDOW));
+  Scratch part((size_t)windows * sizeof(float), s), win((size_t)windows * sizeof(RsumWindow), s);
+  THEA_LAUNCH(rsum_parts_kernel, (unsigned)windows, RSUM_UNIT_THREADS, 0, s, x, count, n, part.as<float>());
+  exclusive_scan<float>(part.as<float>(), part.as<float>(), windows, s);
+  THEA_LAUNCH(rsum_units_kernel, (unsigned)windows, RSUM_UNIT_THREADS, 0, s, x, count, n, s0, part.as<float>(),
+              win.as<RsumWindow>());
+  THEA_LAUNCH(rsum_walk_kernel, 1, RSUM_THREADS, 0, s, x, count, n, s0, win.as<RsumWindow>(), out);
 }
 
 void run_mean_separation(float const * separations, int32_t const * degree, int64_t n, int max_degree, float * out,
@@ -588,7 +631,7 @@ void run_mean_separation(float const * separations, int32_t const * degree, int6
   exclusive_scan<int32_t>(degree, off.as<int32_t>(), n, s);
   THEA_LAUNCH(compact_separations_kernel, (unsigned)ceil_div(n, GRAPH_THREADS), GRAPH_THREADS, 0, s, separations,
               degree, off.as<int32_t>(), n, max_degree, vals.as<float>(), count.as<int64_t>());
-  run_running_sum(vals.as<float>(), count.as<int64_t>(), 0, 0.f, out, s);
+  run_running_sum(vals.as<float>(), count.as<int64_t>(), n * max_degree, 0.f, out, s);
   THEA_LAUNCH(mean_of_sum_kernel, 1, 1, 0, s, out, count.as<int64_t>());
 }
 
