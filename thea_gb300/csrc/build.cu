@@ -151,16 +151,6 @@ __global__ void elem_box_kernel(float const * __restrict__ V, int64_t nv, int32_
   }
 }
 
-// Sets *bad when any of the 3 * nf face indices lies outside [0, nv).
-__global__ void face_range_kernel(int32_t const * __restrict__ F, int64_t count, int64_t nv, int * __restrict__ bad) {
-  bool out = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t f = F[i];
-    out |= f < 0 || (int64_t)f >= nv;
-  }
-  if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
-}
-
 // Start values: bounds, the error words and, for one segment, its start, its root and the collapse's first level
 __global__ void build_init_kernel(int * __restrict__ bounds, int M, int * __restrict__ bad, unsigned * __restrict__ err,
                                   int64_t * __restrict__ seg_start, int64_t n) {
@@ -1121,19 +1111,6 @@ void init_segment_roots(thea_bvh * b, cudaStream_t stream) {
   if (!b->seg_roots) THEA_CUDA_CHECK(thea_malloc_async(&b->seg_roots, (size_t)M * sizeof(RootCut), stream));
   // (pageable memory: the copy has read h when the call returns)
   THEA_CUDA_CHECK(cudaMemcpyAsync(b->seg_roots, h.data(), (size_t)M * sizeof(RootCut), cudaMemcpyHostToDevice, stream));
-}
-
-void check_face_indices(int32_t const * F, int64_t nf, int64_t nv, char const * what, cudaStream_t stream) {
-  if (nf <= 0) return;
-  Scratch bad(sizeof(int), stream);
-  THEA_CUDA_CHECK(cudaMemsetAsync(bad.ptr, 0, sizeof(int), stream));
-  int64_t count = 3 * nf;
-  unsigned grid = (unsigned)std::min<int64_t>(ceil_div(count, BUILD_THREADS), 152 * 8);
-  THEA_LAUNCH(face_range_kernel, grid, BUILD_THREADS, 0, stream, F, count, nv, bad.as<int>());
-  int h = 0;
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&h, bad.ptr, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  THEA_CUDA_CHECK(cudaStreamSynchronize(stream));
-  THEA_REQUIRE(h == 0, std::string(what) + ": a face index lies outside [0, num_vertices)");
 }
 
 thea_bvh * build_bvh(bool is_mesh, float const * V, int64_t nv, int32_t const * F, int64_t nf,

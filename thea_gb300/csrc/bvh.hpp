@@ -65,8 +65,4 @@ void init_segment_roots(thea_bvh * b, cudaStream_t stream);
 // loading an image); other handles, and node arrays that do not follow the build's layout, get none.
 void init_slabs(thea_bvh * b, cudaStream_t stream);
 
-// Throws INVALID_ARGUMENT unless every face index lies in [0, nv): checked on the device before any kernel loads a
-// vertex through the faces (one pass over F and one 4-byte read back, which synchronizes `stream`).
-void check_face_indices(int32_t const * F, int64_t nf, int64_t nv, char const * what, cudaStream_t stream);
-
 }  // namespace thea

@@ -11,6 +11,7 @@
 // so word N - M keeps its value), then all 624 words are tempered and written out. The counter mode draws the three
 // words of sample i from Philox-4x32-10 (Salmon et al., SC'11) keyed by the seed, which is fully parallel.
 #include "device_util.cuh"
+#include "traverse.cuh"
 #include "bvh.hpp"
 #include "query.hpp"
 
@@ -66,28 +67,85 @@ __device__ __forceinline__ void mt_seed_state(uint32_t seed, uint32_t * st) {
   for (int i = 1; i < MT_N; ++i) st[i] = 1812433253u * (st[i - 1] ^ (st[i - 1] >> 30)) + (uint32_t)i;
 }
 
-// Writes `count` tempered words of Random(seed): Random::Random(seed) then bits() repeatedly.
-__global__ void __launch_bounds__(MT_THREADS) thea_mt_stream_kernel(uint32_t seed, int64_t count, uint32_t * __restrict__ out) {
-  __shared__ uint32_t buf[2][MT_N];
-  int t = threadIdx.x;
-  if (t == 0) mt_seed_state(seed, buf[0]);
+// The same twist by a block of 2 * MT_THREADS threads with one barrier. Thread t of the first half has words t, 228 + t
+// and 454 + t. Word 228 + t needs the new word t + 1 and word 454 + t the new word 227 + t, which the threads one to the
+// right and one to the left have just computed, so each of eight warps takes 30 values of t and one more on either side,
+// computed twice, and passes them on by shuffles. The second half meanwhile writes the words of X (the previous twist's
+// result, stream positions from `base`; base < 0: none). A twist's chain is then one shared-memory read, three mixes, two
+// shuffles and the barrier (0.45 us with a barrier after each third and the words written in between, 0.41 now).
+constexpr int MT_LANES = 30;  // words of a third that a warp owns
+static_assert(MT_THREADS / 32 * MT_LANES >= MT_N - MT_M, "eight warps cover a third of the state");
+
+__device__ __forceinline__ void mt_twist_emit_block(uint32_t const * X, uint32_t * Y, int64_t base, int64_t count,
+                                                    uint32_t * __restrict__ out) {
+  constexpr int R = MT_N - MT_M;  // 227
+  if (threadIdx.x < MT_THREADS) {
+    int lane = threadIdx.x & 31;
+    int t = (int)(threadIdx.x >> 5) * MT_LANES + lane - 1;
+    bool own = lane >= 1 && lane <= MT_LANES && t < R;
+    // clamped reads feed words that nobody owns
+    int c = t < 0 ? 0 : (t < R ? t : R - 1);
+    uint32_t y1 = mt_mix(X[c], X[c + 1], X[c + MT_M]);
+    uint32_t right = __shfl_down_sync(0xffffffffu, y1, 1);  // word t + 1
+    int c2 = c < R - 1 ? c : R - 2;                         // t <= 225
+    uint32_t y2 = mt_mix(X[R + 1 + c2], X[R + 2 + c2], right);
+    uint32_t left = __shfl_up_sync(0xffffffffu, y2, 1);  // word 227 + t
+    if (t == 0) left = X[R];                             // the word that the twist leaves alone
+    int i = 2 * R + c;
+    if (own) {
+      Y[t] = y1;
+      if (t == 0) Y[R] = X[R];
+      if (t < R - 1) Y[R + 1 + t] = y2;
+      if (i < MT_N - 1) Y[i] = mt_mix(X[i], X[i + 1], left);
+      else if (i == MT_N - 1) Y[i] = mt_mix(X[i], mt_mix(X[0], X[1], X[MT_M]), left);
+    }
+  } else if (base >= 0) {
+    // three words per thread, their loads and mixes side by side
+    int k = threadIdx.x - MT_THREADS;
+    bool third = k + 2 * MT_THREADS < MT_N;
+    uint32_t a = mt_temper(X[k]), b = mt_temper(X[k + MT_THREADS]), c = mt_temper(X[third ? k + 2 * MT_THREADS : k]);
+    uint32_t * o = out + base + k;
+    int64_t left = count - base - k;  // words from o on
+    if (left > 2 * MT_THREADS) {
+      o[0] = a;
+      o[MT_THREADS] = b;
+      if (third) o[2 * MT_THREADS] = c;
+    } else {
+      if (left > 0) o[0] = a;
+      if (left > MT_THREADS) o[MT_THREADS] = b;
+    }
+  }
   __syncthreads();
-  int64_t twists = ceil_div(count, MT_N);
+}
+
+// Twists [k0, k1) from the state in buf[0] (shared memory, set by the block beforehand), the tempered words of each
+// written at their stream positions
+__device__ __forceinline__ void mt_run_block(uint32_t (*buf)[MT_N], int64_t k0, int64_t k1, int64_t count,
+                                             uint32_t * __restrict__ out) {
   int cur = 0;
-  for (int64_t k = 0; k < twists; ++k) {
-    mt_twist_block(buf[cur], buf[cur ^ 1]);
-    uint32_t const * Y = buf[cur ^ 1];
-    int64_t base = k * MT_N;
-    for (int j = t; j < MT_N; j += MT_THREADS)
-      if (base + j < count) out[base + j] = mt_temper(Y[j]);
-    // the next twist reads Y and writes the other buffer, whose last readers finished before the barrier above
+  for (int64_t k = k0; k < k1; ++k) {
+    mt_twist_emit_block(buf[cur], buf[cur ^ 1], k > k0 ? (k - 1) * MT_N : -1, count, out);
+    // the next twist reads the new state and writes the other buffer, whose last readers finished before the barrier above
     cur ^= 1;
   }
+  int64_t base = (k1 - 1) * MT_N;
+  for (int j = threadIdx.x; j < MT_N; j += blockDim.x)
+    if (base + j < count) out[base + j] = mt_temper(buf[cur][j]);
+}
+
+// Writes `count` tempered words of Random(seed): Random::Random(seed) then bits() repeatedly.
+__global__ void __launch_bounds__(2 * MT_THREADS) thea_mt_stream_kernel(uint32_t seed, int64_t count,
+                                                                        uint32_t * __restrict__ out) {
+  __shared__ uint32_t buf[2][MT_N];
+  if (threadIdx.x == 0) mt_seed_state(seed, buf[0]);
+  __syncthreads();
+  mt_run_block(buf, 0, ceil_div(count, MT_N), count, out);
 }
 
 // Jump-ahead (the twist is linear over GF(2) in the 19,968 state bits, MT_A entering only through the low bit of each
 // mixed word): P = T^L as a bit matrix, column j the state reached from the unit state e_j after L twists. Then the
 // state before twist cL is P^c applied to the seeded state; chunks of L twists run in parallel from those states.
+// L balances the chain of jumps against a chunk's chain of twists
 constexpr int MT_JUMP_TWISTS = 512;  // L
 constexpr int MT_STATE_BITS = MT_N * 32;
 constexpr int MT_VEC_THREADS = 640;  // one output word per thread (>= MT_N)
@@ -105,17 +163,31 @@ __global__ void __launch_bounds__(MT_THREADS) mt_jump_columns_kernel(uint32_t * 
   for (int w = t; w < MT_N; w += MT_THREADS) P[(int64_t)j * MT_N + w] = buf[cur][w];
 }
 
-// out ^= P v over the columns [blockIdx.x * per, ...) of P (out zeroed beforehand; partial sums combined by atomicXor)
+// out ^= P v over the columns of MT_JUMP_WORDS words of v (out zeroed beforehand; partial sums combined by atomicXor). A
+// thread's loads, one word of each column whose bit is set, are in flight together; about one block per SM, since all
+// blocks add to the same 624 words. (One load at a time behind its bit test: 22 us a jump; one word of v per block, four
+// times the atomics: 11 us; this form 9.2, for the 25 MB of columns it reads.)
+constexpr int MT_JUMP_WORDS = 4;
+static_assert(MT_N % MT_JUMP_WORDS == 0, "whole blocks");
 __global__ void __launch_bounds__(MT_VEC_THREADS) mt_jump_apply_kernel(uint32_t const * __restrict__ P,
-                                                                       uint32_t const * __restrict__ v, int per,
+                                                                       uint32_t const * __restrict__ v,
                                                                        uint32_t * __restrict__ out) {
   int w = threadIdx.x;
-  int j0 = blockIdx.x * per, j1 = min(j0 + per, MT_STATE_BITS);
+  if (w >= MT_N) return;
   uint32_t acc = 0;
-  for (int j = j0; j < j1; ++j)
-    if ((__ldg(v + (j >> 5)) >> (j & 31)) & 1u)
-      if (w < MT_N) acc ^= __ldg(P + (int64_t)j * MT_N + w);
-  if (w < MT_N && acc) atomicXor(out + w, acc);
+#pragma unroll
+  for (int u = 0; u < MT_JUMP_WORDS; ++u) {
+    int word = blockIdx.x * MT_JUMP_WORDS + u;
+    uint32_t bits = __ldg(v + word);
+    uint32_t const * col = P + (int64_t)word * 32 * MT_N + w;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      uint32_t x = 0;
+      if ((bits >> j) & 1u) x = __ldg(col + (int64_t)j * MT_N);
+      acc ^= x;
+    }
+  }
+  if (acc) atomicXor(out + w, acc);
 }
 
 __global__ void mt_seed_kernel(uint32_t seed, uint32_t * __restrict__ st) {
@@ -123,33 +195,31 @@ __global__ void mt_seed_kernel(uint32_t seed, uint32_t * __restrict__ st) {
 }
 
 // Chunk c: L twists (fewer for the last) from its start state, tempered words written at their stream positions
-__global__ void __launch_bounds__(MT_THREADS) mt_chunk_kernel(uint32_t const * __restrict__ starts, int64_t count,
-                                                              uint32_t * __restrict__ out) {
+__global__ void __launch_bounds__(2 * MT_THREADS) mt_chunk_kernel(uint32_t const * __restrict__ starts, int64_t count,
+                                                                  uint32_t * __restrict__ out) {
   __shared__ uint32_t buf[2][MT_N];
-  int t = threadIdx.x;
   int64_t c = blockIdx.x;
-  for (int w = t; w < MT_N; w += MT_THREADS) buf[0][w] = starts[c * MT_N + w];
+  for (int w = threadIdx.x; w < MT_N; w += blockDim.x) buf[0][w] = starts[c * MT_N + w];
   __syncthreads();
   int64_t twists = ceil_div(count, MT_N);
   int64_t k0 = c * MT_JUMP_TWISTS, k1 = k0 + MT_JUMP_TWISTS < twists ? k0 + MT_JUMP_TWISTS : twists;
-  int cur = 0;
-  for (int64_t k = k0; k < k1; ++k) {
-    mt_twist_block(buf[cur], buf[cur ^ 1]);
-    uint32_t const * Y = buf[cur ^ 1];
-    int64_t base = k * MT_N;
-    for (int j = t; j < MT_N; j += MT_THREADS)
-      if (base + j < count) out[base + j] = mt_temper(Y[j]);
-    cur ^= 1;
-  }
+  mt_run_block(buf, k0, k1, count, out);
 }
 
-__global__ void tri_area_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t nf,
-                                float * __restrict__ area) {
+// A face with an index outside [0, nv) is not loaded: it sets *bad (the host then refuses the call) and counts as zero.
+__global__ void tri_area_kernel(float const * __restrict__ V, int64_t nv, int32_t const * __restrict__ F, int64_t nf,
+                                float * __restrict__ area, int * __restrict__ bad) {
   int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
-  V3 v0 = load_v3(V + 3 * (int64_t)F[3 * f]);
-  V3 v1 = load_v3(V + 3 * (int64_t)F[3 * f + 1]);
-  V3 v2 = load_v3(V + 3 * (int64_t)F[3 * f + 2]);
+  int32_t i0 = F[3 * f], i1 = F[3 * f + 1], i2 = F[3 * f + 2];
+  if (i0 < 0 || i1 < 0 || i2 < 0 || (int64_t)i0 >= nv || (int64_t)i1 >= nv || (int64_t)i2 >= nv) {
+    *bad = 1;
+    area[f] = 0.f;
+    return;
+  }
+  V3 v0 = load_v3(V + 3 * (int64_t)i0);
+  V3 v1 = load_v3(V + 3 * (int64_t)i1);
+  V3 v2 = load_v3(V + 3 * (int64_t)i2);
   area[f] = tri_plane(v0, v1, v2).area;
 }
 
@@ -221,11 +291,17 @@ __device__ __forceinline__ void float_parts(float a, uint32_t & m, int & e) {
   }
 }
 
-// st[0] = smallest exponent of a nonzero area, st[1] = largest, st[2] = 1 if an area is negative, infinite or NaN
+// st[0] = smallest exponent of a nonzero area, st[1] = largest, st[2] = 1 if an area is negative, infinite or NaN,
+// st[3] = 1 if a face index is out of range; then the total area (double), for the host's one read
 __global__ void cdf_init_kernel(int * st) {
   st[0] = INT_MAX;
   st[1] = INT_MIN;
   st[2] = 0;
+  st[3] = 0;
+}
+
+__global__ void cdf_total_kernel(double const * __restrict__ cum, int64_t nf, int * st) {
+  *reinterpret_cast<double *>(st + 4) = cum[nf - 1];
 }
 
 __global__ void cdf_range_kernel(float const * __restrict__ area, int64_t nf, int * st) {
@@ -322,53 +398,123 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 ctr, uint2 key) {
   return ctr;
 }
 
-__global__ void sample_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t nf,
-                              double const * __restrict__ cum, uint32_t const * __restrict__ words, uint32_t seed,
-                              int64_t n, float * __restrict__ pos, float * __restrict__ nrm, int32_t * __restrict__ face) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t w0, w1, w2;
-  if (words) {
-    w0 = words[3 * i];
-    w1 = words[3 * i + 1];
-    w2 = words[3 * i + 2];
-  } else {
-    uint4 r = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)(i >> 32), 0u, 0u), make_uint2(seed, 0x5EEDu));
-    w0 = r.x; w1 = r.y; w2 = r.z;
-  }
-  // Random::uniform01(): (float)bits() * (1.0f / (float)0xFFFFFFFF), the factor being 2^-32
-  float const NORM = 2.3283064365386963e-10f;
-  double total = cum[nf - 1];
-  double t = (double)(__uint2float_rn(w0) * NORM) * total;
-  // std::lower_bound: first position whose value is not less than t, clamped to the last triangle
-  int64_t lo = 0, len = nf;
-  while (len > 0) {
-    int64_t half = len >> 1;
-    if (cum[lo + half] < t) { lo = lo + half + 1; len = len - half - 1; }
-    else len = half;
-  }
-  int64_t tri = lo < nf - 1 ? lo : nf - 1;
-  V3 v0 = load_v3(V + 3 * (int64_t)F[3 * tri]);
-  V3 v1 = load_v3(V + 3 * (int64_t)F[3 * tri + 1]);
-  V3 v2 = load_v3(V + 3 * (int64_t)F[3 * tri + 2]);
+// One triangle as the samples use it: v0, the edges e01 and e02, and the unit normal, 64 bytes (two 32-byte loads in place
+// of twelve 4-byte ones through the face's indices). Written when there are enough samples to pay for all triangles.
+struct alignas(32) SampleRec {
+  float4 a, b, c, d;  // (v0, n.x) (e01, n.y) (e02, n.z) unused
+};
+
+__global__ void sample_records_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t nf,
+                                      SampleRec * __restrict__ out) {
+  int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= nf) return;
+  V3 v0 = load_v3(V + 3 * (int64_t)F[3 * f]);
+  V3 v1 = load_v3(V + 3 * (int64_t)F[3 * f + 1]);
+  V3 v2 = load_v3(V + 3 * (int64_t)F[3 * f + 2]);
   V3 e01 = v1 - v0, e02 = v2 - v0;
-  float s = __uint2float_rn(w1) * NORM;
-  float u = __uint2float_rn(w2) * NORM;
-  if (s + u > 1.f) {
-    u = 1.f - u;
-    s = 1.f - s;
+  V3 nn = normalized(cross(e01, e02));
+  out[f] = SampleRec{make_float4(v0.x, v0.y, v0.z, nn.x), make_float4(e01.x, e01.y, e01.z, nn.y),
+                     make_float4(e02.x, e02.y, e02.z, nn.z), make_float4(0.f, 0.f, 0.f, 0.f)};
+}
+
+// A block keeps every 2^k-th cumulative area (at most SAMPLE_COARSE of them) in shared memory, so that the first eleven of
+// a sample's 17 dependent probes (81,920 triangles) stay on the SM; blocks take samples in a grid-stride loop to share
+// the table's cost. Bound by the L1 data pipe: every probe and every load of a triangle is a wavefront per lane.
+// 1,048,576 samples: 70 us with all probes in global memory and the triangle through its indices, 53 now.
+constexpr int SAMPLE_COARSE = 2048;
+constexpr int SAMPLE_THREADS = 512;
+
+inline unsigned sample_grid(int64_t n) {
+  return (unsigned)std::min<int64_t>(ceil_div(n, SAMPLE_THREADS), (int64_t)sm_count() * 4);
+}
+
+// Shift of the coarse table: entry c is cum[((c + 1) << shift) - 1], the last of the c-th run of 2^shift
+__host__ __device__ inline int sample_shift(int64_t nf) {
+  int shift = 0;
+  while ((nf >> shift) > SAMPLE_COARSE) ++shift;
+  return shift;
+}
+
+__global__ void sample_coarse_kernel(double const * __restrict__ cum, int64_t nf, double * __restrict__ coarse) {
+  int c = blockIdx.x * blockDim.x + threadIdx.x, shift = sample_shift(nf);
+  if (c < (nf >> shift)) coarse[c] = cum[((int64_t)(c + 1) << shift) - 1];
+}
+
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(float const * __restrict__ V, int32_t const * __restrict__ F, int64_t nf,
+              SampleRec const * __restrict__ rec, double const * __restrict__ coarse_table,
+              double const * __restrict__ cum,
+              uint32_t const * __restrict__ words, uint32_t seed, int64_t n,
+              float * __restrict__ pos, float * __restrict__ nrm, int32_t * __restrict__ face) {
+  __shared__ double s_cum[SAMPLE_COARSE];
+  int shift = sample_shift(nf);
+  int coarse = (int)(nf >> shift);
+  for (int c = threadIdx.x; c < coarse; c += SAMPLE_THREADS)
+    s_cum[c] = coarse_table ? coarse_table[c] : cum[((int64_t)(c + 1) << shift) - 1];
+  __syncthreads();
+  double total = cum[nf - 1];
+  for (int64_t i = (int64_t)blockIdx.x * SAMPLE_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * SAMPLE_THREADS) {
+    uint32_t w0, w1, w2;
+    if (words) {
+      w0 = words[3 * i];
+      w1 = words[3 * i + 1];
+      w2 = words[3 * i + 2];
+    } else {
+      uint4 r = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)(i >> 32), 0u, 0u), make_uint2(seed, 0x5EEDu));
+      w0 = r.x; w1 = r.y; w2 = r.z;
+    }
+    // Random::uniform01(): (float)bits() * (1.0f / (float)0xFFFFFFFF), the factor being 2^-32
+    float const NORM = 2.3283064365386963e-10f;
+    double t = (double)(__uint2float_rn(w0) * NORM) * total;
+    // std::lower_bound: first position whose value is not less than t, clamped to the last triangle
+    int c0 = 0, cl = coarse;
+    while (cl > 0) {
+      int half = cl >> 1;
+      if (s_cum[c0 + half] < t) { c0 = c0 + half + 1; cl = cl - half - 1; }
+      else cl = half;
+    }
+    // every run before c0 ends below t, and run c0 does not (past the last run: the remaining nf - (coarse << shift))
+    int64_t lo = (int64_t)c0 << shift, len = c0 < coarse ? ((int64_t)1 << shift) - 1 : nf - lo;
+    while (len > 0) {
+      int64_t half = len >> 1;
+      if (cum[lo + half] < t) { lo = lo + half + 1; len = len - half - 1; }
+      else len = half;
+    }
+    int64_t tri = lo < nf - 1 ? lo : nf - 1;
+    V3 v0, e01, e02, nn;
+    if (rec) {
+      float4 a, b, c, unused;
+      ldg8(&rec[tri].a, a, b);
+      ldg8(&rec[tri].c, c, unused);
+      v0 = xyz(a);
+      e01 = xyz(b);
+      e02 = xyz(c);
+      nn = V3{a.w, b.w, c.w};
+    } else {
+      v0 = load_v3(V + 3 * (int64_t)F[3 * tri]);
+      V3 v1 = load_v3(V + 3 * (int64_t)F[3 * tri + 1]);
+      V3 v2 = load_v3(V + 3 * (int64_t)F[3 * tri + 2]);
+      e01 = v1 - v0;
+      e02 = v2 - v0;
+      nn = normalized(cross(e01, e02));
+    }
+    float s = __uint2float_rn(w1) * NORM;
+    float u = __uint2float_rn(w2) * NORM;
+    if (s + u > 1.f) {
+      u = 1.f - u;
+      s = 1.f - s;
+    }
+    V3 p = (s * e01 + u * e02) + v0;
+    pos[3 * i] = p.x;
+    pos[3 * i + 1] = p.y;
+    pos[3 * i + 2] = p.z;
+    if (nrm) {
+      nrm[3 * i] = nn.x;
+      nrm[3 * i + 1] = nn.y;
+      nrm[3 * i + 2] = nn.z;
+    }
+    if (face) face[i] = (int32_t)tri;
   }
-  V3 p = (s * e01 + u * e02) + v0;
-  pos[3 * i] = p.x;
-  pos[3 * i + 1] = p.y;
-  pos[3 * i + 2] = p.z;
-  if (nrm) {
-    V3 nn = normalized(cross(e01, e02));
-    nrm[3 * i] = nn.x;
-    nrm[3 * i + 1] = nn.y;
-    nrm[3 * i + 2] = nn.z;
-  }
-  if (face) face[i] = (int32_t)tri;
 }
 
 //============================================================================================================================
@@ -514,7 +660,8 @@ int64_t run_sample_by_area_noalloc(float const * V, int64_t nv, int32_t const * 
   THEA_REQUIRE(!bad, "sample_by_area_noalloc: a face index lies outside [0, num_vertices)");
   if (!(total > 0.0)) return 0;
   if (rng == THEA_RNG_COUNTER) {
-    THEA_LAUNCH(sample_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, V, F, nf, (double const *)scratch->cum,
+    THEA_LAUNCH(sample_kernel, sample_grid(n), SAMPLE_THREADS, 0, s, V, F, nf,
+                (SampleRec const *)nullptr, (double const *)nullptr, (double const *)scratch->cum,
                 (uint32_t const *)nullptr, seed, n, pos, nrm, face);
     return n;
   }
@@ -522,7 +669,8 @@ int64_t run_sample_by_area_noalloc(float const * V, int64_t nv, int32_t const * 
     int64_t cnt = n - begin < NOALLOC_CHUNK ? n - begin : NOALLOC_CHUNK;
     THEA_LAUNCH(noalloc_mt_kernel, 1, MT_THREADS, 0, s, seed, begin == 0 ? 1 : 0, scratch->mt_state, 3 * cnt,
                 scratch->words);
-    THEA_LAUNCH(sample_kernel, (unsigned)ceil_div(cnt, 256), 256, 0, s, V, F, nf, (double const *)scratch->cum,
+    THEA_LAUNCH(sample_kernel, sample_grid(cnt), SAMPLE_THREADS, 0, s, V, F, nf,
+                (SampleRec const *)nullptr, (double const *)nullptr, (double const *)scratch->cum,
                 (uint32_t const *)scratch->words, seed, cnt, pos + 3 * begin, nrm ? nrm + 3 * begin : nullptr,
                 face ? face + begin : nullptr);
   }
@@ -533,7 +681,6 @@ namespace {
 
 // Streams of at least this many twists run as parallel chunks (below it one block is faster than the jump chain)
 constexpr int64_t MT_PARALLEL_MIN_TWISTS = 2 * MT_JUMP_TWISTS;
-constexpr int MT_APPLY_BLOCKS = 156;  // column slices of one jump (128 columns each)
 
 // P = T^L per device, computed on the first long stream of the device (about 50 MB; kept for the process)
 std::mutex g_jump_mu;
@@ -563,7 +710,7 @@ void run_thea_random_words(uint32_t seed, int64_t count, uint32_t * out, cudaStr
   int64_t twists = ceil_div(count, MT_N);
   uint32_t const * P = twists >= MT_PARALLEL_MIN_TWISTS ? jump_matrix(s) : nullptr;
   if (!P) {
-    THEA_LAUNCH(thea_mt_stream_kernel, 1, MT_THREADS, 0, s, seed, count, out);
+    THEA_LAUNCH(thea_mt_stream_kernel, 1, 2 * MT_THREADS, 0, s, seed, count, out);
     return;
   }
   // start states of the chunks: the seeded state, then one jump (P times the previous start) per chunk
@@ -572,46 +719,55 @@ void run_thea_random_words(uint32_t seed, int64_t count, uint32_t * out, cudaStr
   uint32_t * st = starts.as<uint32_t>();
   THEA_CUDA_CHECK(cudaMemsetAsync(st, 0, starts.bytes, s));
   THEA_LAUNCH(mt_seed_kernel, 1, 32, 0, s, seed, st);
-  int per = (int)ceil_div(MT_STATE_BITS, MT_APPLY_BLOCKS);
   for (int64_t c = 1; c < chunks; ++c)
-    THEA_LAUNCH(mt_jump_apply_kernel, MT_APPLY_BLOCKS, MT_VEC_THREADS, 0, s, P, st + (c - 1) * MT_N, per,
-                st + c * MT_N);
-  THEA_LAUNCH(mt_chunk_kernel, (unsigned)chunks, MT_THREADS, 0, s, st, count, out);
+    THEA_LAUNCH(mt_jump_apply_kernel, MT_N / MT_JUMP_WORDS, MT_VEC_THREADS, 0, s, P, st + (c - 1) * MT_N, st + c * MT_N);
+  THEA_LAUNCH(mt_chunk_kernel, (unsigned)chunks, 2 * MT_THREADS, 0, s, st, count, out);
 }
 
 int64_t run_sample_by_area(float const * V, int64_t nv, int32_t const * F, int64_t nf, int64_t n, uint32_t seed, int rng,
                            float * pos, float * nrm, int32_t * face, cudaStream_t s) {
   if (n <= 0 || nf <= 0) return 0;
-  check_face_indices(F, nf, nv, "sample_by_area", s);
   Scratch area((size_t)nf * sizeof(float), s);
   Scratch cum((size_t)nf * sizeof(double), s);
-  THEA_LAUNCH(tri_area_kernel, (unsigned)ceil_div(nf, 256), 256, 0, s, V, F, nf, area.as<float>());
+  struct {
+    int st[4];
+    double total;
+  } h;
   {
     // exact parallel cumulative areas; the serial kernel where they would not be exact
-    Scratch st(4 * sizeof(int), s), fixed((size_t)nf * sizeof(U128), s), excl((size_t)nf * sizeof(U128), s);
+    Scratch st(sizeof(h), s), fixed((size_t)nf * sizeof(U128), s), excl((size_t)nf * sizeof(U128), s);
+    int * d = st.as<int>();
     unsigned g = (unsigned)ceil_div(nf, 256);
-    THEA_LAUNCH(cdf_init_kernel, 1, 1, 0, s, st.as<int>());
-    THEA_LAUNCH(cdf_range_kernel, g, 256, 0, s, area.as<float>(), nf, st.as<int>());
-    THEA_LAUNCH(cdf_fixed_kernel, g, 256, 0, s, area.as<float>(), nf, st.as<int>(), fixed.as<U128>());
+    THEA_LAUNCH(cdf_init_kernel, 1, 1, 0, s, d);
+    THEA_LAUNCH(tri_area_kernel, g, 256, 0, s, V, nv, F, nf, area.as<float>(), d + 3);
+    THEA_LAUNCH(cdf_range_kernel, g, 256, 0, s, area.as<float>(), nf, d);
+    THEA_LAUNCH(cdf_fixed_kernel, g, 256, 0, s, area.as<float>(), nf, d, fixed.as<U128>());
     exclusive_scan<U128>(fixed.as<U128>(), excl.as<U128>(), nf, s);
-    THEA_LAUNCH(cdf_convert_kernel, g, 256, 0, s, excl.as<U128>(), fixed.as<U128>(), nf, st.as<int>(),
-                cum.as<double>());
-    int flag = 0;
-    THEA_CUDA_CHECK(cudaMemcpyAsync(&flag, st.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+    THEA_LAUNCH(cdf_convert_kernel, g, 256, 0, s, excl.as<U128>(), fixed.as<U128>(), nf, d, cum.as<double>());
+    THEA_LAUNCH(cdf_total_kernel, 1, 1, 0, s, cum.as<double>(), nf, d);
+    THEA_CUDA_CHECK(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
     THEA_CUDA_CHECK(cudaStreamSynchronize(s));
-    if (flag) THEA_LAUNCH(serial_cdf_kernel, 1, 256, 0, s, area.as<float>(), nf, cum.as<double>());
+    THEA_REQUIRE(h.st[3] == 0, "sample_by_area: a face index lies outside [0, num_vertices)");
+    if (h.st[2]) {
+      THEA_LAUNCH(serial_cdf_kernel, 1, 256, 0, s, area.as<float>(), nf, cum.as<double>());
+      THEA_CUDA_CHECK(cudaMemcpyAsync(&h.total, cum.as<double>() + nf - 1, sizeof(double), cudaMemcpyDeviceToHost, s));
+      THEA_CUDA_CHECK(cudaStreamSynchronize(s));
+    }
   }
-  double total = 0.0;
-  THEA_CUDA_CHECK(cudaMemcpyAsync(&total, cum.as<double>() + nf - 1, sizeof(double), cudaMemcpyDeviceToHost, s));
-  THEA_CUDA_CHECK(cudaStreamSynchronize(s));
-  if (!(total > 0.0)) return 0;  // MeshSampler returns no samples for a zero-area mesh
+  if (!(h.total > 0.0)) return 0;  // MeshSampler returns no samples for a zero-area mesh
   Scratch words;
   if (rng == THEA_RNG_THEA_MT) {
     words = Scratch((size_t)n * 3 * sizeof(uint32_t), s);
     run_thea_random_words(seed, 3 * n, words.as<uint32_t>(), s);
   }
-  THEA_LAUNCH(sample_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, V, F, nf, cum.as<double>(), words.as<uint32_t>(),
-              seed, n, pos, nrm, face);
+  // records for every triangle pay from about one sample in two triangles on
+  Scratch rec(n >= nf / 2 ? (size_t)nf * sizeof(SampleRec) : 0, s);
+  if (rec.ptr)
+    THEA_LAUNCH(sample_records_kernel, (unsigned)ceil_div(nf, 256), 256, 0, s, V, F, nf, rec.as<SampleRec>());
+  Scratch coarse(SAMPLE_COARSE * sizeof(double), s);
+  THEA_LAUNCH(sample_coarse_kernel, SAMPLE_COARSE / 256, 256, 0, s, cum.as<double>(), nf, coarse.as<double>());
+  THEA_LAUNCH(sample_kernel, sample_grid(n), SAMPLE_THREADS, 0, s, V, F, nf, rec.as<SampleRec>(), coarse.as<double>(),
+              cum.as<double>(), words.as<uint32_t>(), seed, n, pos, nrm, face);
   return n;
 }
 
