@@ -90,54 +90,35 @@ __device__ __forceinline__ double bound2_of(ClosestArgs const & a, int m) {
 }
 
 // One round: lane query q when active. Called by all 32 lanes of the warp together.
-template <int W, int STACK, int PREC>
+template <int W, int STACK>
 __device__ __forceinline__ void closest_round(BatchForest const & f, ClosestArgs const & a, int64_t q, bool active,
-                                              int budget, HardQueue const & hq, F64WarpBuf * buf) {
+                                              int budget, HardQueue const & hq) {
   WideNode<W> const * nodes = (WideNode<W> const *)f.nodes;
-  int root = 0;
-  int64_t ebase = 0;
   V3 p = V3{0.f, 0.f, 0.f};
-  float thresh = a.thresh;
-  double bound2 = a.bound2;
-  if (active) {
-    int m = mesh_of_query(a.qoff, f.M, q);
-    root = __ldg(f.seg_root + m);
-    ebase = __ldg(f.seg_start + m);
-    p = load_v3(a.queries + 3 * q);
-    thresh = thresh_of(a, m);
-    bound2 = bound2_of(a, m);
-  }
   ClosestOut r;
   r.idx = INT_MAX;
   r.d2 = 0.f;
-  r.d2_64 = 0.0;
   r.slot = -1;
   r.best32 = INFINITY;
   r.done = true;
-  float dist = 0.f;
-  if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-    float scale = fmaxf(a.scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
-    F64Search s;
-    if (active) closest_search_f64<W, STACK>(nodes, f.cp_rec, root, ebase, p, bound2, scale, f.err, s, budget);
-    else f64_search_init(s);
-    f64_resolve_warp(s, active && s.done, f.cp_rec, ebase, p, bound2, *buf);
-    r = f64_result(s);
-    dist = (float)sqrt(r.d2_64);
-  } else {
-    if (active) r = closest_query<W, STACK>(nodes, f.cp_rec, root, ebase, p, thresh, f.err, budget);
-    dist = sqrtf(r.d2);
+  if (active) {
+    int m = mesh_of_query(a.qoff, f.M, q);
+    p = load_v3(a.queries + 3 * q);
+    r = closest_query<W, STACK>(nodes, f.cp_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m), p, thresh_of(a, m), f.err,
+                                budget);
   }
+  float dist = sqrtf(r.d2);
   if (active && !r.done) {
     unsigned long long pos = atomicAdd(hq.count, 1ull);
     hq.q[pos] = q;
     hq.bound[pos] = r.best32;
-    hq.idx[pos] = PREC == THEA_PRECISION_FP64_RECHECK ? INT_MAX : r.idx;
+    hq.idx[pos] = r.idx;
     hq.slot[pos] = r.slot;
   }
   bool fin = active && r.done;
   bool found = r.idx != INT_MAX;
-  double d64 = r.d2_64;
-  if (PREC != THEA_PRECISION_FP64_RECHECK && a.out_err) {
+  double d64 = 0.0;
+  if (a.out_err) {
     __syncwarp();
     if (fin && found) {
       D3 cp64;
@@ -147,21 +128,16 @@ __device__ __forceinline__ void closest_round(BatchForest const & f, ClosestArgs
   if (fin) write_closest(q, found, dist, r.cp, r.idx, d64, a.out_index, a.out_dist, a.out_cp, a.out_err);
 }
 
-template <int W, int STACK, int PREC>
+template <int W, int STACK>
 __global__ void __launch_bounds__(BATCH_THREADS)
 batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long long * counter, int chunk, int budget,
                      HardQueue hq) {
-  F64WarpBuf * buf = nullptr;
-  if constexpr (PREC == THEA_PRECISION_FP64_RECHECK) {
-    __shared__ F64WarpBuf s_buf[BATCH_THREADS / 32];
-    buf = &s_buf[threadIdx.x >> 5];
-  }
   int lane = threadIdx.x & 31;
   int64_t base;
   while (next_chunk(counter, chunk, nq, base)) {
     int64_t end = base + chunk < nq ? base + chunk : nq;
     for (int64_t r0 = base; r0 < end; r0 += 32)
-      closest_round<W, STACK, PREC>(f, a, r0 + lane, r0 + lane < end, budget, hq, buf);
+      closest_round<W, STACK>(f, a, r0 + lane, r0 + lane < end, budget, hq);
   }
 }
 
@@ -260,6 +236,214 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
   }
 }
 
+// The mixed-precision search in two kernels. closest_collect_kernel is the persistent-lane FP32 traversal above with the
+// band rule of closest_search_f64: it keeps the elements whose FP32 distance lies within the band of the best (in shared
+// memory, F64_CAND a lane) and leaves each query's final band entries in `cand`, -1 past the last. closest_resolve_kernel
+// evaluates them in FP64, 32 queries to a warp in full-warp rounds (f64_resolve_warp). Apart, the traversal runs at the
+// FP32 search's registers and refills its lanes, and the FP64 pipe sees nothing but full rounds; one kernel that does both
+// needs 128 registers, or idles lanes until their warp's next round. A query over the step budget, or with more band
+// entries than fit (rare), goes to the warp-per-query kernel with the FP32 best as its bound. Results do not depend on who
+// finishes a query.
+constexpr int F64_HARD = -2;  // cand[0] of a query left to the warp-per-query kernel
+
+template <int W, int STACK>
+__global__ void __launch_bounds__(BATCH_THREADS)
+closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long long * counter, int budget, HardQueue hq,
+                       int block, int32_t * __restrict__ cand) {
+  __shared__ int2 s_stk[CLOSEST_SHARED_STACK][BATCH_THREADS];
+  __shared__ float s_cd[F64_CAND][BATCH_THREADS];
+  __shared__ int s_ck[F64_CAND][BATCH_THREADS];
+  unsigned const FULL = 0xffffffffu;
+  float const REL = 1.0f + 1.0f / 16384.0f;
+  int lane = threadIdx.x & 31, t = threadIdx.x;
+  WideNode<W> const * nodes = (WideNode<W> const *)f.nodes;
+  int64_t qb = 0, qe = 0;  // warp-local block of query indices, warp-uniform
+  bool exhausted = false;  // warp-uniform
+  int64_t q = -1;          // this lane's query (-1: idle)
+  int64_t ebase = 0;
+  V3 p = V3{0.f, 0.f, 0.f};
+  SharedStack<STACK, CLOSEST_SHARED_STACK, BATCH_THREADS> stk(s_stk);
+  int sp = 0;
+  int next = CHILD_EMPTY;  // nearest child of the last node, visited next without a stack round trip
+  float lim = 0.f;         // band limit on FP32 squared distances
+  float best32 = INFINITY, abs_tol = 0.f;
+  int nc = 0;     // entries kept, some of them outside the band by now
+  int steps = 0;  // (two-phase form: budget > 0)
+  while (true) {
+    unsigned idle = __ballot_sync(FULL, q < 0);
+    if (idle && !exhausted) {
+      if (qb >= qe) {
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(counter, (unsigned long long)block);
+        b = __shfl_sync(FULL, b, 0);
+        qb = (int64_t)b;
+        qe = qb + block < nq ? qb + block : nq;
+        if (qb >= nq) exhausted = true;
+      }
+      if (!exhausted) {
+        int rank = __popc(idle & ((1u << lane) - 1));
+        int64_t avail = qe - qb;
+        int64_t take = __popc(idle);
+        if (q < 0 && rank < avail) {
+          q = qb + rank;
+          int m = mesh_of_query(a.qoff, f.M, q);
+          ebase = __ldg(f.seg_start + m);
+          p = load_v3(a.queries + 3 * q);
+          sp = 0;
+          next = __ldg(f.seg_root + m);
+          steps = 0;
+          nc = 0;
+          float scale = fmaxf(a.scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+          lim = f64_band_start(bound2_of(a, m), scale, abs_tol);
+          best32 = INFINITY;
+        }
+        qb += take < avail ? take : avail;
+      }
+    }
+    if (__ballot_sync(FULL, q >= 0) == 0) break;
+    if (q < 0) continue;
+    bool hard = budget > 0 && ++steps > budget;
+    if (!hard && next == CHILD_EMPTY && sp == 0) {
+      // finished: the entries still in the band
+      int out[F64_CAND];
+      int c = 0;
+#pragma unroll
+      for (int j = 0; j < F64_CAND; ++j) out[j] = -1;
+      for (int j = 0; j < nc; ++j) {
+        if (s_cd[j][t] <= lim) {
+          int k = s_ck[j][t];
+#pragma unroll
+          for (int u = 0; u < F64_CAND; ++u) out[u] = u == c ? k : out[u];
+          ++c;
+        }
+      }
+      int4 * o = reinterpret_cast<int4 *>(cand + q * F64_CAND);
+#pragma unroll
+      for (int j = 0; j < F64_CAND; j += 4) o[j / 4] = make_int4(out[j], out[j + 1], out[j + 2], out[j + 3]);
+      q = -1;
+      continue;
+    }
+    if (!hard) {
+      int code = next;
+      if (code == CHILD_EMPTY) {
+        --sp;
+        int2 top = stk.get(sp);
+        code = top.x;
+        if (__int_as_float(top.y) > lim * PRUNE_SLACK) continue;
+      }
+      next = CHILD_EMPTY;
+      int first = 0, count = 0;
+      if (code < 0) decode_leaf(code, first, count);
+      auto children = [&](NodeRegs<W> const & nd) {
+        float lb[W];
+        point_child_bounds<W>(nd, p, lb);
+        push_children_next<W>(nd, lb, lim * PRUNE_SLACK, stk, sp, next, f.err);
+      };
+      auto take = [&](float d2, int kr) {
+        if (!(d2 <= lim)) return;
+        if (d2 < best32) {
+          best32 = d2;
+          float lb1 = sqrtf(best32) * REL + abs_tol;
+          lim = fminf(lim, lb1 * lb1);
+        }
+        if (nc == F64_CAND) {
+          // drop the entries that have left the band
+          int m = 0;
+          for (int j = 0; j < F64_CAND; ++j) {
+            float d = s_cd[j][t];
+            int k = s_ck[j][t];
+            if (d <= lim) {
+              s_cd[m][t] = d;
+              s_ck[m][t] = k;
+              ++m;
+            }
+          }
+          nc = m;
+        }
+        if (nc < F64_CAND) {
+          s_cd[nc][t] = d2;
+          s_ck[nc][t] = kr;
+          ++nc;
+        } else {
+          hard = true;  // more entries in the band than fit
+        }
+      };
+      if constexpr (W == 4) {
+        int64_t k = ebase + first;
+        float4 r[8];
+        load_line(code >= 0 ? reinterpret_cast<float4 const *>(nodes + code) : f.cp_rec + k * CP_REC_F4, r);
+        if (code >= 0) {
+          NodeRegs<W> nd;
+          node_from_line(r, nd);
+          children(nd);
+        } else {
+          V3 cp;
+          take(cp_record_eval(r, p, cp), first);
+          if (count > 1) next = encode_leaf(first + 1, count - 1);
+        }
+      } else {
+        if (code >= 0) {
+          NodeRegs<W> nd;
+          load_node(nodes, code, nd);
+          children(nd);
+        } else {
+          for (int kr = first; kr < first + count; ++kr) {
+            V3 cp;
+            take(cp_record_test(f.cp_rec, ebase + kr, p, cp), kr);
+          }
+        }
+      }
+    }
+    if (hard) {
+      unsigned long long pos = atomicAdd(hq.count, 1ull);
+      hq.q[pos] = q;
+      hq.bound[pos] = best32;
+      hq.idx[pos] = INT_MAX;
+      hq.slot[pos] = -1;
+      cand[q * F64_CAND] = F64_HARD;
+      q = -1;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(BATCH_THREADS)
+closest_resolve_kernel(BatchForest f, ClosestArgs a, int64_t nq, int32_t const * __restrict__ cand) {
+  __shared__ F64WarpBuf s_buf[BATCH_THREADS / 32];
+  int64_t q = (int64_t)blockIdx.x * BATCH_THREADS + threadIdx.x;
+  bool active = q < nq;
+  F64Search s;
+  f64_search_init(s);
+  int64_t ebase = 0;
+  double bound2 = -1.0;
+  V3 p = V3{0.f, 0.f, 0.f};
+  if (active) {
+    int4 const * c = reinterpret_cast<int4 const *>(cand + q * F64_CAND);
+#pragma unroll
+    for (int j = 0; j < F64_CAND; j += 4) {
+      int4 v = __ldg(c + j / 4);
+      s.cand_k[j] = v.x;
+      s.cand_k[j + 1] = v.y;
+      s.cand_k[j + 2] = v.z;
+      s.cand_k[j + 3] = v.w;
+    }
+    if (s.cand_k[0] == F64_HARD) {
+      active = false;
+    } else {
+#pragma unroll
+      for (int j = 0; j < F64_CAND; ++j) s.cand_d[j] = 0.f;  // all of them lie in the band
+      int m = mesh_of_query(a.qoff, f.M, q);
+      ebase = __ldg(f.seg_start + m);
+      bound2 = bound2_of(a, m);
+      p = load_v3(a.queries + 3 * q);
+    }
+  }
+  f64_resolve_warp(s, active, f.cp_rec, ebase, p, bound2, s_buf[threadIdx.x >> 5]);
+  if (!active) return;
+  ClosestOut r = f64_result(s);
+  write_closest(q, r.idx != INT_MAX, (float)sqrt(r.d2_64), r.cp, r.idx, r.d2_64, a.out_index, a.out_dist, a.out_cp,
+                a.out_err);
+}
+
 constexpr int PHASE2_WARPS = BATCH_THREADS / 32;
 
 template <int W, int PREC>
@@ -285,7 +469,7 @@ batch_closest_phase2_kernel(BatchForest f, ClosestArgs a, HardQueue hq, unsigned
     if (PREC == THEA_PRECISION_FP64_RECHECK) {
       float scale = fmaxf(a.scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
       WarpBest64 b = closest_warp_query_f64<W>(nodes, f.cp_rec, root, ebase, p, bound2_of(a, m), scale, hq.bound[j],
-                                               s_code[warp], s_lb[warp], s_cd[warp], s_ck[warp], f.err);
+                                               s_code[warp], s_lb[warp], s_cd[warp], s_ck[warp], f.err, f.slabs);
       if (lane == 0) {
         bool found = b.idx != INT_MAX;
         V3 cp = V3{0.f, 0.f, 0.f};
@@ -320,6 +504,34 @@ batch_closest_phase2_kernel(BatchForest f, ClosestArgs a, HardQueue hq, unsigned
       }
     }
     __syncwarp();
+  }
+}
+
+// A warp per query from the root, FP64 re-check, one BVH: the small-batch form of the mixed-precision search
+template <int W>
+__global__ void __launch_bounds__(BATCH_THREADS)
+closest_warp_f64_kernel(BatchForest f, ClosestArgs a, int64_t nq) {
+  __shared__ int s_code[PHASE2_WARPS][WARP_STACK];
+  __shared__ float s_lb[PHASE2_WARPS][WARP_STACK];
+  __shared__ float s_cd[PHASE2_WARPS][WARP_CAND];
+  __shared__ int64_t s_ck[PHASE2_WARPS][WARP_CAND];
+  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int64_t q = (int64_t)blockIdx.x * PHASE2_WARPS + warp;
+  if (q >= nq) return;  // the whole warp
+  V3 p = load_v3(a.queries + 3 * q);
+  float scale = fmaxf(a.scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+  WarpBest64 b = closest_warp_query_f64<W>((WideNode<W> const *)f.nodes, f.cp_rec, 0, 0, p, a.bound2, scale, INFINITY,
+                                           s_code[warp], s_lb[warp], s_cd[warp], s_ck[warp], f.err, f.slabs);
+  if (lane == 0) {
+    bool found = b.idx != INT_MAX;
+    V3 cp = V3{0.f, 0.f, 0.f};
+    if (found) {
+      D3 cp64;
+      double d64;
+      cp_record_f64(f.cp_rec, b.slot, p, cp64, d64);
+      cp = V3{(float)cp64.x, (float)cp64.y, (float)cp64.z};
+    }
+    write_closest(q, found, (float)sqrt(b.d2), cp, b.idx, b.d2, a.out_index, a.out_dist, a.out_cp, a.out_err);
   }
 }
 
@@ -549,41 +761,45 @@ int persistent_grid(void const * kernel) {
   return std::max(1, per_sm) * sms;
 }
 
-template <int W, int STACK, int PREC>
-void launch_closest_prec(BatchForest const & f, ClosestArgs const & a, int64_t nq, int budget,
-                         unsigned long long * counters, int chunk, HardQueue const & hq, cudaStream_t s) {
-  auto k1 = batch_closest_kernel<W, STACK, PREC>;
-  int phase1_budget = budget > 0 ? budget : 0;
-  char const * name = budget > 0                             ? "batch_closest_phase1_kernel"
-                      : PREC == THEA_PRECISION_FP64_RECHECK ? "batch_closest_kernel_fp64"
-                                                            : "batch_closest_kernel_fp32";
-  // FP32 without error estimates: persistent lanes (1.5x on the 256-mesh case), also as the first phase of the
-  // two-phase form
-  bool refill = PREC != THEA_PRECISION_FP64_RECHECK && !a.out_err;
-  if (refill) {
-    auto kr = batch_closest_refill_kernel<W, STACK>;
-    // a block of indices no larger than a warp's share: a small batch keeps every warp busy
-    int pg = persistent_grid((void const *)kr);
-    int64_t per = ceil_div(nq, (int64_t)pg * (BATCH_THREADS / 32));
-    THEA_LAUNCH_NAMED(name, kr, pg, BATCH_THREADS, 0, s, f, a, nq, counters, phase1_budget, hq,
-                      (int)std::min<int64_t>(REFILL_BLOCK, std::max<int64_t>(1, per)));
-  } else {
-    THEA_LAUNCH_NAMED(name, k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk,
-                      phase1_budget, hq);
-  }
-  if (budget <= 0) return;
-  auto k2 = batch_closest_phase2_kernel<W, PREC>;
-  THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, persistent_grid((void const *)k2), BATCH_THREADS, 0, s, f, a, hq,
-                    counters + 1);
+// Blocks of query indices a warp takes at a time: no larger than a warp's share, so that a small batch keeps every warp
+// busy
+int refill_block(int64_t nq, int grid) {
+  int64_t per = ceil_div(nq, (int64_t)grid * (BATCH_THREADS / 32));
+  return (int)std::min<int64_t>(REFILL_BLOCK, std::max<int64_t>(1, per));
 }
 
 template <int W, int STACK>
 void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t nq, int prec, int budget,
                           unsigned long long * counters, int chunk, HardQueue const & hq, cudaStream_t s) {
-  if (prec == THEA_PRECISION_FP64_RECHECK)
-    launch_closest_prec<W, STACK, THEA_PRECISION_FP64_RECHECK>(f, a, nq, budget, counters, chunk, hq, s);
-  else
-    launch_closest_prec<W, STACK, THEA_PRECISION_FP32_REFERENCE>(f, a, nq, budget, counters, chunk, hq, s);
+  int first_budget = budget > 0 ? budget : 0;
+  if (prec == THEA_PRECISION_FP64_RECHECK) {
+    Scratch cand((size_t)nq * F64_CAND * sizeof(int32_t), s);
+    auto k1 = closest_collect_kernel<W, STACK>;
+    int grid = persistent_grid((void const *)k1);
+    THEA_LAUNCH_NAMED("batch_closest_kernel_fp64", k1, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq,
+                      refill_block(nq, grid), cand.as<int32_t>());
+    THEA_LAUNCH_NAMED("closest_resolve_kernel", closest_resolve_kernel, (unsigned)ceil_div(nq, BATCH_THREADS),
+                      BATCH_THREADS, 0, s, f, a, nq, cand.as<int32_t>());
+    auto k2 = batch_closest_phase2_kernel<W, THEA_PRECISION_FP64_RECHECK>;
+    THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, persistent_grid((void const *)k2), BATCH_THREADS, 0, s, f, a, hq,
+                      counters + 1);
+    return;
+  }
+  char const * name = budget > 0 ? "batch_closest_phase1_kernel" : "batch_closest_kernel_fp32";
+  // without error estimates: persistent lanes (1.5x on the 256-mesh case), also as the first phase of the two-phase form
+  if (!a.out_err) {
+    auto kr = batch_closest_refill_kernel<W, STACK>;
+    int grid = persistent_grid((void const *)kr);
+    THEA_LAUNCH_NAMED(name, kr, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq, refill_block(nq, grid));
+  } else {
+    auto k1 = batch_closest_kernel<W, STACK>;
+    THEA_LAUNCH_NAMED(name, k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk,
+                      first_budget, hq);
+  }
+  if (budget <= 0) return;
+  auto k2 = batch_closest_phase2_kernel<W, THEA_PRECISION_FP32_REFERENCE>;
+  THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, persistent_grid((void const *)k2), BATCH_THREADS, 0, s, f, a, hq,
+                    counters + 1);
 }
 
 template <int W, int STACK>
@@ -632,65 +848,6 @@ BatchForest forest_view(thea_bvh const * b) {
 
 namespace {
 
-// FP64 re-check batches take their queries in (mesh, Morton code) order: a warp's round of 32 queries then holds
-// neighbours, whose searches take similar paths and share band candidates (256 config-3 meshes: 24.9 -> 20.8 ms). The
-// FP32 kernels refill lanes one query at a time and ran slower on sorted queries (11.2 -> 12.4 ms), so they keep the
-// caller's order. Results do not depend on the order.
-constexpr int64_t SORTED_QUERIES_MIN = 1 << 15;
-
-__device__ __forceinline__ uint32_t spread10(uint32_t x) {
-  x &= 0x3ffu;
-  x = (x | (x << 16)) & 0x030000ffu;
-  x = (x | (x << 8)) & 0x0300f00fu;
-  x = (x | (x << 4)) & 0x030c30c3u;
-  x = (x | (x << 2)) & 0x09249249u;
-  return x;
-}
-
-__global__ void sorted_query_keys_kernel(float const * __restrict__ q, int64_t const * __restrict__ qoff, int M,
-                                         int64_t nq, float lx, float ly, float lz, float sx, float sy, float sz,
-                                         uint64_t * __restrict__ keys, uint32_t * __restrict__ vals) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  int m = mesh_of_query(qoff, M, i);
-  float c[3] = {(q[3 * i] - lx) * sx, (q[3 * i + 1] - ly) * sy, (q[3 * i + 2] - lz) * sz};
-  uint32_t g[3];
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    float u = fminf(fmaxf(c[t], 0.f), 1.f);  // NaN-safe: fminf/fmaxf drop a NaN operand
-    g[t] = min((uint32_t)(u * 1024.f), 1023u);
-  }
-  keys[i] = ((uint64_t)m << 30) | (spread10(g[0]) << 2) | (spread10(g[1]) << 1) | spread10(g[2]);
-  vals[i] = (uint32_t)i;
-}
-
-__global__ void gather_queries_kernel(float const * __restrict__ q, uint32_t const * __restrict__ order, int64_t nq,
-                                      float * __restrict__ out) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  int64_t j = order[i];
-  out[3 * i] = q[3 * j];
-  out[3 * i + 1] = q[3 * j + 1];
-  out[3 * i + 2] = q[3 * j + 2];
-}
-
-__global__ void scatter_closest_kernel(uint32_t const * __restrict__ order, int64_t nq, int32_t const * __restrict__ si,
-                                       float const * __restrict__ sd, float const * __restrict__ sc,
-                                       float const * __restrict__ se, int32_t * __restrict__ idx,
-                                       float * __restrict__ dist, float * __restrict__ cpt, float * __restrict__ err) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  int64_t j = order[i];
-  idx[j] = si[i];
-  if (dist) dist[j] = sd[i];
-  if (cpt) {
-    cpt[3 * j] = sc[3 * i];
-    cpt[3 * j + 1] = sc[3 * i + 1];
-    cpt[3 * j + 2] = sc[3 * i + 2];
-  }
-  if (err) err[j] = se[i];
-}
-
 // One batched closest-point search of `a` (queries, offsets, outputs) over the forest
 void batch_closest_core(thea_bvh const * b, ClosestArgs const & a, int64_t nq, ClosestParams const & cp, int chunk,
                         cudaStream_t s) {
@@ -700,7 +857,8 @@ void batch_closest_core(thea_bvh const * b, ClosestArgs const & a, int64_t nq, C
   Scratch counters(3 * sizeof(unsigned long long), s);
   THEA_CUDA_CHECK(cudaMemsetAsync(counters.ptr, 0, 3 * sizeof(unsigned long long), s));
   auto * c = counters.as<unsigned long long>();
-  size_t hq_n = budget > 0 ? (size_t)nq : 0;
+  // (the mixed-precision search may hand over queries at any budget)
+  size_t hq_n = budget > 0 || cp.precision == THEA_PRECISION_FP64_RECHECK ? (size_t)nq : 0;
   Scratch hq_q(hq_n * sizeof(int64_t), s), hq_b(hq_n * sizeof(float), s);
   Scratch hq_i(hq_n * sizeof(int32_t), s), hq_s(hq_n * sizeof(int64_t), s);
   HardQueue hq{hq_q.as<int64_t>(), hq_b.as<float>(), hq_i.as<int32_t>(), hq_s.as<int64_t>(), c + 2};
@@ -710,46 +868,11 @@ void batch_closest_core(thea_bvh const * b, ClosestArgs const & a, int64_t nq, C
           : launch_batch_closest<8, 512>(f, a, nq, cp.precision, budget, c, chunk, hq, s);
 }
 
-// batch_closest_core on the queries in (mesh, Morton code) order: keys, a stable radix sort, the permuted copy, the
-// search into scratch outputs, then the results scattered back to the caller's order
-void batch_closest_sorted(thea_bvh const * b, float const * q, int64_t const * qoff, int64_t nq,
-                          ClosestParams const & cp, int chunk, int32_t * idx, float * dist, float * cpt, float * err,
-                          cudaStream_t s) {
-  float sc[3];
-  for (int t = 0; t < 3; ++t) {
-    float ext = b->hi[t] - b->lo[t];
-    sc[t] = ext > 0.f ? 1.0f / ext : 0.f;
-  }
-  Scratch keys((size_t)nq * sizeof(uint64_t), s), order((size_t)nq * sizeof(uint32_t), s);
-  unsigned grid = (unsigned)ceil_div(nq, 256);
-  THEA_LAUNCH(sorted_query_keys_kernel, grid, 256, 0, s, q, qoff, b->num_segments, nq, b->lo[0], b->lo[1], b->lo[2],
-              sc[0], sc[1], sc[2], keys.as<uint64_t>(), order.as<uint32_t>());
-  int seg_bits = 0;
-  while ((1 << seg_bits) < b->num_segments) ++seg_bits;
-  radix_sort_pairs(keys.as<uint64_t>(), order.as<uint32_t>(), nq, 30 + seg_bits, s, /*probe_passes=*/false);
-  keys = Scratch();
-  Scratch qs((size_t)nq * 12, s), si((size_t)nq * 4, s), sd(dist ? (size_t)nq * 4 : 0, s);
-  Scratch scp(cpt ? (size_t)nq * 12 : 0, s), se(err ? (size_t)nq * 4 : 0, s);
-  THEA_LAUNCH(gather_queries_kernel, grid, 256, 0, s, q, order.as<uint32_t>(), nq, qs.as<float>());
-  ClosestArgs a{qs.as<float>(), qoff, cp.thresh, cp.bound2, cp.scene_scale, si.as<int32_t>(),
-                dist ? sd.as<float>() : nullptr, cpt ? scp.as<float>() : nullptr, err ? se.as<float>() : nullptr,
-                cp.seg_cut};
-  batch_closest_core(b, a, nq, cp, chunk, s);
-  THEA_LAUNCH(scatter_closest_kernel, grid, 256, 0, s, order.as<uint32_t>(), nq, si.as<int32_t>(),
-              dist ? sd.as<float>() : nullptr, cpt ? scp.as<float>() : nullptr, err ? se.as<float>() : nullptr, idx,
-              dist, cpt, err);
-}
-
 }  // namespace
 
 void run_batch_closest(thea_bvh const * b, float const * q, int64_t const * qoff, int64_t nq, ClosestParams const & cp,
                        int chunk, int32_t * idx, float * dist, float * cpt, float * err, cudaStream_t s) {
   if (nq <= 0) return;
-  if (cp.precision == THEA_PRECISION_FP64_RECHECK && nq >= SORTED_QUERIES_MIN && nq < ((int64_t)1 << 32) &&
-      b->num_segments <= (1 << 20)) {
-    batch_closest_sorted(b, q, qoff, nq, cp, chunk, idx, dist, cpt, err, s);
-    return;
-  }
   ClosestArgs a{q, qoff, cp.thresh, cp.bound2, cp.scene_scale, idx, dist, cpt, err, cp.seg_cut};
   batch_closest_core(b, a, nq, cp, chunk, s);
 }
@@ -768,6 +891,16 @@ void run_closest_teams(thea_bvh const * b, float const * q, int64_t nq, ClosestP
   bool whole = nq < CLOSEST_WHOLE_WARP_MAX;
   if (b->width == 4) whole ? launch_closest_team<4, 32>(f, a, nq, s) : launch_closest_team<4, 16>(f, a, nq, s);
   else whole ? launch_closest_team<8, 32>(f, a, nq, s) : launch_closest_team<8, 16>(f, a, nq, s);
+}
+
+void run_closest_warps_f64(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,
+                           float * dist, float * cpt, float * err, cudaStream_t s) {
+  if (nq <= 0) return;
+  BatchForest f = forest_view(b);
+  ClosestArgs a{q, nullptr, cp.thresh, cp.bound2, cp.scene_scale, idx, dist, cpt, err};
+  unsigned grid = (unsigned)ceil_div(nq, PHASE2_WARPS);
+  if (b->width == 4) THEA_LAUNCH(closest_warp_f64_kernel<4>, grid, BATCH_THREADS, 0, s, f, a, nq);
+  else THEA_LAUNCH(closest_warp_f64_kernel<8>, grid, BATCH_THREADS, 0, s, f, a, nq);
 }
 
 template <int W, int STACK>

@@ -38,6 +38,9 @@ void run_batch_closest(thea_bvh const * b, float const * q, int64_t const * qoff
 constexpr int64_t CLOSEST_WHOLE_WARP_MAX = 3072;
 void run_closest_teams(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,
                        float * dist, float * cpt, cudaStream_t s);
+// FP64 re-check of a small batch on one BVH (num_segments == 1, small_stack_ok), a warp per query.
+void run_closest_warps_f64(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,
+                           float * dist, float * cpt, float * err, cudaStream_t s);
 // FP32 closest point of one BVH with queries and results in pinned host memory accessed by the kernels in place
 // (device-usable pointers); cp.budget > 0 enables the warp-per-query second phase.
 void run_closest_stream(thea_bvh const * b, float const * q, int64_t nq, ClosestParams const & cp, int32_t * idx,

@@ -572,6 +572,22 @@ constexpr int CLOSEST_WARP_BUDGET = 16;
 constexpr int64_t CLOSEST_TWO_PHASE_MIN = 98304;
 constexpr int CLOSEST_TWO_PHASE_BUDGET = 256;
 
+// FP64 re-check calls on one BVH. Call times in ms, queries near the surface / uniform in the box grown by half:
+//  * fewer than F64_WARP_MAX queries (F64_WARP_MAX_SMALL on small meshes): a warp per query. 1,000 queries on 20,480
+//    triangles: 0.066 / 0.075, against 0.143 / 0.491 one query per thread.
+//  * otherwise the collecting and resolving kernels with a step budget of 64, 128 from 8,192 queries and 256 from 32,768:
+//    20,480 triangles, 12,000 queries 0.162 / 0.602 -> 0.136 / 0.383, 100,000: 0.436 / 1.23 -> 0.361 / 0.934, 250,000:
+//    0.691 / 1.95 -> 0.665 / 1.70; 81,920 triangles, 250,000: 0.983 / 2.53 -> 0.881 / 1.85.
+//  * on small meshes (F64_SMALL_MESH triangles; four times as many from F64_SMALL_LARGE_BATCH queries on) one query per
+//    thread, in Morton order, with slabs, the form compared with above: nodes and records stay in L1 or nearly, and a
+//    warp of neighbours reads them together. 1,280 triangles, 100,000 queries: 0.254 / 0.511 against 0.215 / 0.670 collected
+//    and resolved; 5,120 triangles: 0.323 / 0.769 against 0.269 / 0.937, but 50,000 queries 0.245 / 0.608 against 0.173 /
+//    0.597.
+constexpr int64_t F64_WARP_MAX = 3072;
+constexpr int64_t F64_WARP_MAX_SMALL = 2048;
+constexpr int64_t F64_SMALL_MESH = 2048;
+constexpr int64_t F64_SMALL_LARGE_BATCH = 65536;
+
 __global__ void query_range_kernel(int64_t * qoff, int64_t n) {
   qoff[0] = 0;
   qoff[1] = n;
@@ -1049,6 +1065,20 @@ bool small_stack_ok(thea_bvh const * b) {
 void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams const & cp, int32_t * idx, float * dist,
                  float * cpt, float * errout, unsigned * err, cudaStream_t s) {
   if (n <= 0) return;
+  bool f64_small = b->n <= F64_SMALL_MESH || (b->n <= 4 * F64_SMALL_MESH && n >= F64_SMALL_LARGE_BATCH);
+  if (cp.precision == THEA_PRECISION_FP64_RECHECK && n < (f64_small ? F64_WARP_MAX_SMALL : F64_WARP_MAX) &&
+      small_stack_ok(b)) {
+    run_closest_warps_f64(b, q, n, cp, idx, dist, cpt, errout, s);
+    return;
+  }
+  if (cp.precision == THEA_PRECISION_FP64_RECHECK && !f64_small) {
+    Scratch qoff(2 * sizeof(int64_t), s);
+    THEA_LAUNCH(query_range_kernel, 1, 1, 0, s, qoff.as<int64_t>(), n);
+    ClosestParams c2 = cp;
+    c2.budget = n < 8192 ? 64 : (n < 32768 ? 128 : CLOSEST_TWO_PHASE_BUDGET);
+    run_batch_closest(b, q, qoff.as<int64_t>(), n, c2, 64, idx, dist, cpt, errout, s);
+    return;
+  }
   if (cp.precision == THEA_PRECISION_FP32_REFERENCE && !errout && !b->query_order &&
       (n < CLOSEST_WARP_MAX || n >= CLOSEST_TWO_PHASE_MIN)) {
     if (n < CLOSEST_WARP_MAX && small_stack_ok(b)) {

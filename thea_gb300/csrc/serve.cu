@@ -176,7 +176,7 @@ serve_closest_phase2_kernel(ServeTask const * __restrict__ tasks, int64_t const 
     if (PREC == THEA_PRECISION_FP64_RECHECK) {
       float scale = fmaxf(t->scene_scale, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
       WarpBest64 b = closest_warp_query_f64<W>(nodes, t->rec, 0, 0, p, t->bound2, scale, hq.bound[j], s_code[warp],
-                                               s_lb[warp], s_cd[warp], s_ck[warp], t->err);
+                                               s_lb[warp], s_cd[warp], s_ck[warp], t->err, t->slabs);
       found = b.idx != INT_MAX;
       idx = b.idx;
       dist = (float)sqrt(b.d2);

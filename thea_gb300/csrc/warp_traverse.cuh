@@ -293,8 +293,9 @@ template <int W>
 __device__ WarpBest64 closest_warp_query_f64(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ rec,
                                              int root, int64_t elem_base, V3 p, double bound2, float scale,
                                              float init_best32, int * s_code, float * s_lb, float * s_cd,
-                                             int64_t * s_ck, unsigned * err) {
+                                             int64_t * s_ck, unsigned * err, float4 const * __restrict__ slabs) {
   constexpr int NPOP = 32 / W;
+  float q1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
   float const REL = 1.0f + 1.0f / 16384.0f;
   float abs_tol = scale * (1.0f / 262144.0f);
   int lane = threadIdx.x & 31;
@@ -352,6 +353,10 @@ __device__ WarpBest64 closest_warp_query_f64(WideNode<W> const * __restrict__ no
       int child;
       load_child<W>(nodes, code, c, lx, hx, ly, hy, lz, hz, child);
       float d2b = point_box_d2(p.x, p.y, p.z, lx, ly, lz, hx, hy, hz);
+      if (slabs && child != CHILD_EMPTY) {
+        float d;
+        d2b = fmaxf(d2b, slab_lower_bound(__ldg(slabs + (int64_t)code * W + c), p, q1, d));
+      }
       if (child != CHILD_EMPTY && d2b <= plim) {
         if (child >= 0) {
           key = __float_as_uint(d2b);
