@@ -15,24 +15,36 @@ import numpy as np
 from . import _native as N
 
 
+_torch = None  # the torch module, once a torch tensor has been seen
+
+
 def _is_torch(x):
     return type(x).__module__.startswith("torch")
 
 
+def _torch_module():
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
+
+
 def _cuda_ready():
-    import torch
+    torch = _torch_module()
     return torch.cuda.is_available() and torch.cuda.is_initialized()
 
 
 def _stream_of(on_device):
     if not on_device:
         return None
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_torch_module().cuda.current_stream().cuda_stream)
 
 
 class _Arrays:
-    """Normalises inputs to contiguous float32/int32 arrays on one side (host or device) and allocates outputs there."""
+    """Normalises inputs to contiguous float32/int32 arrays on one side (host or device) and allocates outputs there. A
+    tensor that is already what the library reads goes through untouched: the conversions that change nothing took a
+    third of a small call's time on the host."""
 
     def __init__(self, like):
         self.device = _is_torch(like) and like.is_cuda
@@ -42,13 +54,13 @@ class _Arrays:
         if a is None:
             return None, 0
         if self.device:
-            import torch
-            tdt = torch.float32 if dtype == np.float32 else torch.int32
-            t = a.to(dtype=tdt).contiguous()
-            if cols:
+            torch = _torch_module()
+            tdt = torch.float32 if dtype is np.float32 else torch.int32
+            t = a if a.dtype is tdt and a.is_contiguous() else a.to(dtype=tdt).contiguous()
+            if cols and (t.dim() != 2 or t.shape[1] != cols):
                 t = t.reshape(-1, cols)
             self.keep.append(t)
-            return ctypes.c_void_p(t.data_ptr()), t.shape[0]
+            return t.data_ptr(), t.shape[0]
         if _is_torch(a):
             a = a.detach().cpu().numpy()
         arr = np.ascontiguousarray(a, dtype=dtype)
@@ -59,10 +71,9 @@ class _Arrays:
 
     def output(self, shape, dtype):
         if self.device:
-            import torch
-            tdt = torch.float32 if dtype == np.float32 else torch.int32
-            t = torch.empty(shape, dtype=tdt, device="cuda")
-            return t, ctypes.c_void_p(t.data_ptr() if t.numel() else 0)
+            torch = _torch_module()
+            t = torch.empty(shape, dtype=torch.float32 if dtype is np.float32 else torch.int32, device="cuda")
+            return t, t.data_ptr()
         arr = np.empty(shape, dtype=dtype)
         return arr, ctypes.c_void_p(arr.ctypes.data if arr.size else 0)
 
