@@ -141,7 +141,7 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
   }
 }
 
-// Persistent-lane form of batch_closest_kernel: each lane takes a new query as soon as its query is done, instead of
+// Persistent-lane form of batch_closest_kernel: lanes take new queries as theirs end, instead of
 // idling until the slowest query of its warp's round (the queries deep inside a mesh take ten times the steps of the
 // others). Every loop iteration advances each busy lane by one stack entry; idle lanes are refilled from a warp-local
 // block of up to 64 query indices. FP32 search only (the mixed-precision search is bound by the FP64 pipe, and rounds of 32
@@ -150,8 +150,14 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
 // and record loads (a third of the lanes active: a warp mixes lanes at nodes, at leaves and between queries). One
 // 128-byte line per lane and step through 32-byte loads, issued before node and leaf lanes part ways (closest_step), and
 // the first 24 stack entries in shared memory (SharedStack): 262,144 queries on 81,920 triangles 1.41 -> 1.13 ms, 256
-// meshes with 5.2 M queries 12.4 -> 9.85 ms. Blocks of 16 or 32 indices: within 3 % of 64. A lower step budget once the
+// meshes with 5.2 M queries 12.4 -> 9.85 ms, 9.01 with the refill below. Blocks of 16 or 32 indices: within 3 % of 64. A lower step budget once the
 // indices run out: slower (1.27 -> 1.74 ms at 128). Queries in Morton order: 1.18 -> 1.21 ms before the sort's own time.
+// Lanes without a query wait until this many of their warp's do (or all of them), so that results are written and queries
+// fetched for several lanes at a time. FP32, refilled at 1 / 2 / 4 / 8 lanes: 262,144 queries near 81,920 triangles 0.270 /
+// 0.270 / 0.270 / 0.289 ms (0.296 with each result written as it ends), 256 meshes with 5.2 M queries 9.62 / 9.25 / 9.01 /
+// 8.99 (9.81). The collecting kernel, whose lanes also pack their band entries: 100,003 queries 0.934 / 0.934 / 0.933 /
+// 0.783 (0.951); 12 and 16 lanes as 8.
+constexpr int CLOSEST_REFILL_AT = 4, COLLECT_REFILL_AT = 8;
 constexpr int REFILL_BLOCK = 64;
 
 template <int W, int STACK>
@@ -176,8 +182,18 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
   V3 best_cp = V3{0.f, 0.f, 0.f};
   int pops = 0;  // stack entries taken by this lane's query (two-phase form: budget > 0)
   while (true) {
-    unsigned idle = __ballot_sync(FULL, q < 0);
-    if (idle && !exhausted) {
+    // lanes whose query is done, or that have none
+    bool done = next == CHILD_EMPTY && sp == 0;
+    unsigned idle = __ballot_sync(FULL, done);
+    if (__popc(idle) >= CLOSEST_REFILL_AT || idle == FULL) {
+      if (done && q >= 0) {
+        write_closest(q, best_idx != INT_MAX, sqrtf(best), best_cp, best_idx, 0.0, a.out_index, a.out_dist, a.out_cp,
+                      nullptr);
+        q = -1;
+      }
+      if (exhausted && idle == FULL) break;
+    }
+    if ((__popc(idle) >= CLOSEST_REFILL_AT || idle == FULL) && !exhausted) {
       if (qb >= qe) {
         unsigned long long b = 0;
         if (lane == 0) b = atomicAdd(counter, (unsigned long long)block);
@@ -190,7 +206,8 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
         int rank = __popc(idle & ((1u << lane) - 1));
         int64_t avail = qe - qb;
         int64_t take = __popc(idle);
-        if (q < 0 && rank < avail) {
+        if (done && rank < avail) {
+          done = false;
           q = qb + rank;
           int m = mesh_of_query(a.qoff, f.M, q);
           ebase = __ldg(f.seg_start + m);
@@ -205,14 +222,7 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
         qb += take < avail ? take : avail;
       }
     }
-    if (__ballot_sync(FULL, q >= 0) == 0) break;
-    if (q < 0) continue;
-    if (next == CHILD_EMPTY && sp == 0) {
-      write_closest(q, best_idx != INT_MAX, sqrtf(best), best_cp, best_idx, 0.0, a.out_index, a.out_dist, a.out_cp,
-                    nullptr);
-      q = -1;
-      continue;
-    }
+    if (done) continue;
     if (budget > 0 && ++pops > budget) {
       // over budget (steps taken, the register-held child included): queued with the best element so far, finished
       // by a warp of its own in the second kernel
@@ -222,6 +232,8 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
       hq.idx[pos] = best_idx;
       hq.slot[pos] = best_slot;
       q = -1;
+      next = CHILD_EMPTY;
+      sp = 0;
       continue;
     }
     int code = next;
@@ -270,8 +282,32 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
   int nc = 0;     // entries kept, some of them outside the band by now
   int steps = 0;  // (two-phase form: budget > 0)
   while (true) {
-    unsigned idle = __ballot_sync(FULL, q < 0);
-    if (idle && !exhausted) {
+    // lanes whose query is done, or that have none
+    bool done = next == CHILD_EMPTY && sp == 0;
+    unsigned idle = __ballot_sync(FULL, done);
+    if (__popc(idle) >= COLLECT_REFILL_AT || idle == FULL) {
+      if (done && q >= 0) {
+        // finished: the entries still in the band
+        int out[F64_CAND];
+        int c = 0;
+  #pragma unroll
+        for (int j = 0; j < F64_CAND; ++j) out[j] = -1;
+        for (int j = 0; j < nc; ++j) {
+          if (s_cd[j][t] <= lim) {
+            int k = s_ck[j][t];
+  #pragma unroll
+            for (int u = 0; u < F64_CAND; ++u) out[u] = u == c ? k : out[u];
+            ++c;
+          }
+        }
+        int4 * o = reinterpret_cast<int4 *>(cand + q * F64_CAND);
+  #pragma unroll
+        for (int j = 0; j < F64_CAND; j += 4) o[j / 4] = make_int4(out[j], out[j + 1], out[j + 2], out[j + 3]);
+        q = -1;
+      }
+      if (exhausted && idle == FULL) break;
+    }
+    if ((__popc(idle) >= COLLECT_REFILL_AT || idle == FULL) && !exhausted) {
       if (qb >= qe) {
         unsigned long long b = 0;
         if (lane == 0) b = atomicAdd(counter, (unsigned long long)block);
@@ -284,7 +320,8 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
         int rank = __popc(idle & ((1u << lane) - 1));
         int64_t avail = qe - qb;
         int64_t take = __popc(idle);
-        if (q < 0 && rank < avail) {
+        if (done && rank < avail) {
+          done = false;
           q = qb + rank;
           int m = mesh_of_query(a.qoff, f.M, q);
           ebase = __ldg(f.seg_start + m);
@@ -300,29 +337,8 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
         qb += take < avail ? take : avail;
       }
     }
-    if (__ballot_sync(FULL, q >= 0) == 0) break;
-    if (q < 0) continue;
+    if (done) continue;
     bool hard = budget > 0 && ++steps > budget;
-    if (!hard && next == CHILD_EMPTY && sp == 0) {
-      // finished: the entries still in the band
-      int out[F64_CAND];
-      int c = 0;
-#pragma unroll
-      for (int j = 0; j < F64_CAND; ++j) out[j] = -1;
-      for (int j = 0; j < nc; ++j) {
-        if (s_cd[j][t] <= lim) {
-          int k = s_ck[j][t];
-#pragma unroll
-          for (int u = 0; u < F64_CAND; ++u) out[u] = u == c ? k : out[u];
-          ++c;
-        }
-      }
-      int4 * o = reinterpret_cast<int4 *>(cand + q * F64_CAND);
-#pragma unroll
-      for (int j = 0; j < F64_CAND; j += 4) o[j / 4] = make_int4(out[j], out[j + 1], out[j + 2], out[j + 3]);
-      q = -1;
-      continue;
-    }
     if (!hard) {
       int code = next;
       if (code == CHILD_EMPTY) {
@@ -402,6 +418,8 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
       hq.slot[pos] = -1;
       cand[q * F64_CAND] = F64_HARD;
       q = -1;
+      next = CHILD_EMPTY;
+      sp = 0;
     }
   }
 }
@@ -614,7 +632,7 @@ closest_stream_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lo
     }
     __syncwarp();
     unsigned idle = __ballot_sync(FULL, q < 0);
-    if (idle && !exhausted) {
+    if ((__popc(idle) >= CLOSEST_REFILL_AT || idle == FULL) && !exhausted) {
       if (qb >= qe && taken - oldest < CP_STREAM_RING) {
         unsigned long long b = 0;
         if (lane == 0) b = atomicAdd(counter, (unsigned long long)REFILL_BLOCK);

@@ -184,17 +184,22 @@ ray_recheck_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __rest
 
 // Persistent form of ray_kernel for large batches (FP32 verdict only). Rays that leave the mesh after a few nodes and
 // rays that traverse deep share warps; with one ray per thread the finished lanes idle until their warp's last ray is
-// done. Here each lane takes a new ray as soon as its ray finishes: every loop iteration advances each busy lane by one
-// stack entry, and idle lanes are refilled from a warp-local block of 64 rays (one atomic per block). Results are the
+// done. Here lanes take new rays as theirs finish: every loop iteration advances each busy lane by one stack entry, and
+// idle lanes are refilled from a warp-local block of 64 rays (one atomic per block). Results are the
 // same as ray_kernel's: each ray's traversal is the same sequence of steps. (Measured on the 2 M-triangle heightfield:
 // skipping pruned entries in an inner loop, or postponing leaves so that node steps run converged, were both slower,
 // since a lane's extra steps then stall its whole warp; keeping the nearest child in a register and packing stack
 // entries into 8 bytes gained 4.5 %.) What bounds it: the L1 data pipe (81 % of its peak with 16-byte loads inside the
 // node and leaf branches, each lane's line a wavefront per load) and the latency of those loads. Node or leaf read
 // through one set of 32-byte loads (ray_step) and the first 16 stack entries in shared memory: 4.2 M rays on 2.1 M
-// triangles 1.011 -> 0.871 ms; from pinned host arrays (ray_stream_kernel, seven blocks per SM: eight would spill) 1.130
+// triangles 1.011 -> 0.871 ms, 0.771 with the refill above; from pinned host arrays (ray_stream_kernel, seven blocks per SM: eight would spill) 1.130
 // -> 1.006 ms.
 constexpr int RAY_WARP_BLOCK = 64;
+// Lanes without a ray wait until this many of their warp's do (or all of them): writing a ray's results, fetching the next
+// and its three divisions then run for eight or more lanes together instead of one or two. 4.2 M rays on 2.1 M triangles
+// (half of them done after two steps), refilled at 1 / 4 / 8 / 12 / 16 / 24 lanes: 0.817 / 0.789 / 0.771 / 0.781 / 0.821 /
+// 0.997 ms (0.869 with the results written as each ray ends).
+constexpr int RAY_REFILL_AT = 8;
 constexpr int64_t RAY_PERSISTENT_MIN = 1 << 16;
 
 template <int W, int STACK>
@@ -219,40 +224,12 @@ ray_persistent_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __r
   int sp = 0;
   int next = CHILD_EMPTY;  // the nearest child of the last node: visited next without a stack round trip
   while (true) {
-    unsigned idle = __ballot_sync(FULL, q < 0);
-    if (idle && !exhausted) {
-      if (qb >= qe) {
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(counter, (unsigned long long)RAY_WARP_BLOCK);
-        b = __shfl_sync(FULL, b, 0);
-        qb = (int64_t)b;
-        qe = qb + RAY_WARP_BLOCK < n ? qb + RAY_WARP_BLOCK : n;
-        if (qb >= n) exhausted = true;
-      }
-      if (!exhausted) {
-        int rank = __popc(idle & ((1u << lane) - 1));
-        int take = __popc(idle);
-        int64_t avail = qe - qb;
-        if (q < 0 && rank < avail) {
-          q = qb + rank;
-          int64_t r = order ? (int64_t)order[q] : q;
-          q = r;
-          ray_setup(ray, load_v3(origins + 3 * r), load_v3(dirs + 3 * r));
-          best = max_time >= 0.f ? max_time : INFINITY;
-          best_idx = INT_MAX;
-          best_slot = -1;
-          sp = 0;
-          next = 0;  // the root
-        }
-        qb += take < avail ? take : avail;
-      }
-    }
-    if (__ballot_sync(FULL, q >= 0) == 0) break;
-    if (q < 0) continue;
-    int code = next;
-    if (code == CHILD_EMPTY) {
-      if (sp == 0) {
-        // finished: the same outputs as ray_kernel
+    // lanes whose ray is done, or that have none
+    bool done = next == CHILD_EMPTY && sp == 0;
+    unsigned idle = __ballot_sync(FULL, done);
+    if (__popc(idle) >= RAY_REFILL_AT || idle == FULL) {
+      if (done && q >= 0) {
+        // the same outputs as ray_kernel
         bool found = best_idx != INT_MAX;
         out_time[q] = found ? best : -1.f;
         if (out_index) out_index[q] = found ? best_idx : -1;
@@ -267,8 +244,37 @@ ray_persistent_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __r
           out_normal[3 * q + 2] = nn.z;
         }
         q = -1;
-        continue;
       }
+      if (!exhausted && qb >= qe) {
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(counter, (unsigned long long)RAY_WARP_BLOCK);
+        b = __shfl_sync(FULL, b, 0);
+        qb = (int64_t)b;
+        qe = qb + RAY_WARP_BLOCK < n ? qb + RAY_WARP_BLOCK : n;
+        if (qb >= n) exhausted = true;
+      }
+      if (!exhausted) {
+        int rank = __popc(idle & ((1u << lane) - 1));
+        int take = __popc(idle);
+        int64_t avail = qe - qb;
+        if (done && rank < avail) {
+          q = qb + rank;
+          if (order) q = (int64_t)order[q];
+          ray_setup(ray, load_v3(origins + 3 * q), load_v3(dirs + 3 * q));
+          best = max_time >= 0.f ? max_time : INFINITY;
+          best_idx = INT_MAX;
+          best_slot = -1;
+          next = 0;  // the root
+          done = false;
+        }
+        qb += take < avail ? take : avail;
+      } else if (idle == FULL) {
+        break;
+      }
+    }
+    if (done) continue;
+    int code = next;
+    if (code == CHILD_EMPTY) {
       --sp;
       int2 top = stk.get(sp);
       code = top.x;
@@ -335,7 +341,7 @@ ray_stream_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restr
     }
     __syncwarp();
     unsigned idle = __ballot_sync(FULL, q < 0);
-    if (idle && !exhausted) {
+    if ((__popc(idle) >= RAY_REFILL_AT || idle == FULL) && !exhausted) {
       if (qb >= qe && taken - oldest < STREAM_RING) {
         unsigned long long b = 0;
         if (lane == 0) b = atomicAdd(counter, (unsigned long long)RAY_WARP_BLOCK);
