@@ -755,7 +755,8 @@ batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t cons
       int root = __ldg(f.seg_root + m);
       int64_t ebase = __ldg(f.seg_start + m);
       uint64_t keys[K];
-      if constexpr (K >= 8) {
+      // (K = 8 in registers: 200,000 queries over 100 sets of 2,000 points 0.322 -> 0.237 ms)
+      if constexpr (K >= 16) {
         __shared__ uint64_t s_list[K][BATCH_THREADS];
         SharedKnnList<K, BATCH_THREADS> list(s_list);
         list.init(entry);

@@ -430,9 +430,11 @@ void launch_ray_stream(thea_bvh const * b, float const * o, float const * d, int
 // BoundedSortedArrayN.hpp:137-214)
 //============================================================================================================================
 
-// The k-NN kernels keep lists of K >= 8 in shared memory: 48-56 registers for K = 16, and the
-// register allocator is asked for eight resident blocks of 128 threads (four for K = 32, whose lists take 32 KB)
-template <int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 8; }
+// The kernels over points keep lists of K >= 16 in shared memory, those over triangles from K = 8 on (their K = 8 spills in
+// registers). Points, shared memory against registers: K = 8, 262,144 queries of 50,000 points 0.266 / 0.251 ms; K = 16
+// 0.403 / 0.454 (five resident blocks). The register allocator is asked for eight resident blocks of 128 threads (four
+// for K = 32, whose lists take 32 KB).
+template <int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 16; }
 template <int K> constexpr int knn_point_min_blocks() { return knn_lists_shared<K>() ? (K <= 16 ? 8 : 4) : 8; }
 
 // Row `row` of the k-NN outputs from a K-entry list read through gd(j) / gi(j) (registers or shared memory): -1 for
@@ -540,7 +542,7 @@ knn_mesh_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restric
   if (order) q = order[q];
   V3 p = load_v3(queries + 3 * q);
   int excl = exclude ? exclude[q] : -1;
-  if constexpr (knn_lists_shared<K>()) {
+  if constexpr (K >= 8) {
     __shared__ float s_d[K][QUERY_THREADS];
     __shared__ int s_i[K][QUERY_THREADS];
     int t = threadIdx.x;
