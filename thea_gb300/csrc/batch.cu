@@ -141,17 +141,21 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
   }
 }
 
-// Persistent-lane form of batch_closest_kernel: lanes take new queries as theirs end, instead of
-// idling until the slowest query of its warp's round (the queries deep inside a mesh take ten times the steps of the
-// others). Every loop iteration advances each busy lane by one stack entry; idle lanes are refilled from a warp-local
-// block of up to 64 query indices. FP32 search only (the mixed-precision search is bound by the FP64 pipe, and rounds of 32
-// queries fill its FP64 step better: 25.7 against 27.5 ms on 256 meshes). Results are the round-based kernel's: each
-// query's search is the same sequence of steps. What bounds it: the L1 data pipe (65 % busy) and the latency of the node
-// and record loads (a third of the lanes active: a warp mixes lanes at nodes, at leaves and between queries). One
-// 128-byte line per lane and step through 32-byte loads, issued before node and leaf lanes part ways (closest_step), and
-// the first 24 stack entries in shared memory (SharedStack): 262,144 queries on 81,920 triangles 1.41 -> 1.13 ms, 256
-// meshes with 5.2 M queries 12.4 -> 9.85 ms, 9.01 with the refill below. Blocks of 16 or 32 indices: within 3 % of 64. A lower step budget once the
-// indices run out: slower (1.27 -> 1.74 ms at 128). Queries in Morton order: 1.18 -> 1.21 ms before the sort's own time.
+// Persistent-lane form of batch_closest_kernel: lanes take new queries as theirs end, instead of idling until the slowest
+// query of its warp's round (the queries deep inside a mesh take ten times the steps of the others). Every loop iteration
+// advances each busy lane by one stack entry; idle lanes are refilled from a warp-local block of up to 64 query indices.
+// FP32 search only; closest_collect_kernel below is the mixed-precision form. Results are the round-based kernel's: each
+// query's search is the same sequence of steps.
+//
+// What bounds it: the L1 data pipe (68 % busy), the issue slots (65 %) and the latency of the node and record loads, with
+// a third of the lanes active (a warp mixes lanes at nodes, at leaves and between queries). One 128-byte line per lane and
+// step through 32-byte loads, issued before node and leaf lanes part ways (closest_step), and the first 24 stack entries
+// in shared memory (SharedStack): 262,144 queries on 81,920 triangles 1.41 -> 1.13 ms, 256 meshes with 5.2 M queries 12.4
+// -> 9.85 ms; 1.04 and 9.01 with the refill below. Measured and not taken: blocks of 16 or 32 indices (within 3 %); a
+// lower step budget once the indices run out (1.27 -> 1.74 ms at 128); queries in Morton order (1.18 -> 1.21 ms before the
+// sort's own time); a line fetched by eight lanes with 16-byte asynchronous copies into shared memory (1.04 -> 1.47 ms:
+// fewer wavefronts, but every step waits for the copies and reads the line once more).
+//
 // Lanes without a query wait until this many of their warp's do (or all of them), so that results are written and queries
 // fetched for several lanes at a time. FP32, refilled at 1 / 2 / 4 / 8 lanes: 262,144 queries near 81,920 triangles 0.270 /
 // 0.270 / 0.270 / 0.289 ms (0.296 with each result written as it ends), 256 meshes with 5.2 M queries 9.62 / 9.25 / 9.01 /
@@ -755,8 +759,9 @@ batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t cons
       int root = __ldg(f.seg_root + m);
       int64_t ebase = __ldg(f.seg_start + m);
       uint64_t keys[K];
-      // (K = 8 in registers: 200,000 queries over 100 sets of 2,000 points 0.322 -> 0.237 ms)
-      if constexpr (K >= 16) {
+      // lists in shared memory as in knn_kernel (width 4, K = 8, 200,000 queries over 100 sets of 2,000 points: 0.322 ms, in
+      // registers 0.237)
+      if constexpr (K >= 16 || (W == 8 && K >= 8)) {
         __shared__ uint64_t s_list[K][BATCH_THREADS];
         SharedKnnList<K, BATCH_THREADS> list(s_list);
         list.init(entry);

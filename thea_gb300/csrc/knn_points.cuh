@@ -63,7 +63,7 @@ template <int K> struct RegisterKnnList {
   }
 };
 
-// Lists of 16 and more: unsorted in shared memory ([K][B], entry j of thread t at [j][t]: no bank conflicts), in groups of
+// Lists of 16 and more (knn_lists_shared): unsorted in shared memory ([K][B], entry j of thread t at [j][t]: no bank conflicts), in groups of
 // four with each group's largest key in a register. An insertion replaces the largest key of all and looks at its group
 // alone: one store, three loads and a fixed sequence of selects, where a sorted list shifts K / 2 entries on average and
 // a warp waits for the longest shift of its lanes. The row is sorted once, at the end, by a network all lanes run

@@ -190,10 +190,10 @@ ray_recheck_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __rest
 // skipping pruned entries in an inner loop, or postponing leaves so that node steps run converged, were both slower,
 // since a lane's extra steps then stall its whole warp; keeping the nearest child in a register and packing stack
 // entries into 8 bytes gained 4.5 %.) What bounds it: the L1 data pipe (81 % of its peak with 16-byte loads inside the
-// node and leaf branches, each lane's line a wavefront per load) and the latency of those loads. Node or leaf read
-// through one set of 32-byte loads (ray_step) and the first 16 stack entries in shared memory: 4.2 M rays on 2.1 M
-// triangles 1.011 -> 0.871 ms, 0.771 with the refill above; from pinned host arrays (ray_stream_kernel, seven blocks per SM: eight would spill) 1.130
-// -> 1.006 ms.
+// node and leaf branches, each lane's line a wavefront per load; 78 % now) and the latency of those loads. Node or leaf
+// read through one set of 32-byte loads (ray_step) and the first 16 stack entries in shared memory: 4.2 M rays on 2.1 M
+// triangles 1.011 -> 0.871 ms, 0.771 with the refill below; from pinned host arrays (ray_stream_kernel, seven blocks per
+// SM: eight would spill) 1.130 -> 1.006 ms. Lines fetched by eight lanes together into shared memory: 0.790 ms, not taken.
 constexpr int RAY_WARP_BLOCK = 64;
 // Lanes without a ray wait until this many of their warp's do (or all of them): writing a ray's results, fetching the next
 // and its three divisions then run for eight or more lanes together instead of one or two. 4.2 M rays on 2.1 M triangles
@@ -430,12 +430,13 @@ void launch_ray_stream(thea_bvh const * b, float const * o, float const * d, int
 // BoundedSortedArrayN.hpp:137-214)
 //============================================================================================================================
 
-// The kernels over points keep lists of K >= 16 in shared memory, those over triangles from K = 8 on (their K = 8 spills in
-// registers). Points, shared memory against registers: K = 8, 262,144 queries of 50,000 points 0.266 / 0.251 ms; K = 16
-// 0.403 / 0.454 (five resident blocks). The register allocator is asked for eight resident blocks of 128 threads (four
-// for K = 32, whose lists take 32 KB).
-template <int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 16; }
-template <int K> constexpr int knn_point_min_blocks() { return knn_lists_shared<K>() ? (K <= 16 ? 8 : 4) : 8; }
+// Kernels over points keep their K best in shared memory from K = 16 on (width-8 trees, whose 256-byte nodes leave fewer
+// registers, from K = 8 on), and in registers below. Shared memory against registers, 262,144 queries: K = 8, width 4,
+// 0.266 / 0.251 ms; K = 8, width 8, 0.408 / 0.420; K = 16, width 4, 0.403 / 0.454 (five resident blocks). The register
+// allocator is asked for eight resident blocks of 128 threads (four for K = 32, whose lists take 32 KB). The lists of
+// triangles (knn_mesh_kernel) are in shared memory from K = 8 on.
+template <int W, int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 16 || (W == 8 && K >= 8); }
+template <int K> constexpr int knn_point_min_blocks() { return K <= 16 ? 8 : 4; }
 
 // Row `row` of the k-NN outputs from a K-entry list read through gd(j) / gi(j) (registers or shared memory): -1 for
 // empty entries. Whole rows go out as 16-byte stores when they can: rows land at scattered element indices (self
@@ -515,7 +516,7 @@ knn_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restrict__ p
     return key < none ? key : none;
   };
   uint64_t keys[K];
-  if constexpr (knn_lists_shared<K>()) {
+  if constexpr (knn_lists_shared<W, K>()) {
     __shared__ uint64_t s_list[K][QUERY_THREADS];
     SharedKnnList<K, QUERY_THREADS> list(s_list);
     list.init(entry);
