@@ -52,3 +52,15 @@ def test_many_band_entries(width, leaf):
     rng = np.random.default_rng(2)
     Q = (rng.normal(size=(5000, 3)) * 0.01 + [0, 0, 1]).astype(np.float32)
     _check(bvh, V, F, Q, -1.0, 300)
+
+
+@pytest.mark.parametrize("width,leaf", [(4, 7), (4, 8), (4, 15), (8, 8)])
+@pytest.mark.parametrize("n", [32767, 32768])
+def test_leaf_sizes_at_the_budget_rule(n, width, leaf):
+    """Either side of the larger step budget of leaves of eight, queries around and deep inside the mesh."""
+    import torch
+    import thea_gb300 as T
+    from thea_gb300 import workloads as W
+    V, F = W.noisy_icosphere(5, 3)
+    bvh = T.MeshBvh(torch.from_numpy(V).cuda(), torch.from_numpy(F).cuda(), width=width, max_leaf_size=leaf)
+    _check(bvh, V, F, W.uniform_box_points(n, [-1.5] * 3, [1.5] * 3, n), -1.0, 200)

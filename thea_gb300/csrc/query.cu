@@ -592,6 +592,10 @@ constexpr int CLOSEST_TWO_PHASE_BUDGET = 256;
 //    warp of neighbours reads them together. 1,280 triangles, 100,000 queries: 0.254 / 0.511 against 0.215 / 0.670 collected
 //    and resolved; 5,120 triangles: 0.323 / 0.769 against 0.269 / 0.937, but 50,000 queries 0.245 / 0.608 against 0.173 /
 //    0.597.
+//  * a step tests one element of a width-4 leaf, so with leaves of 8 the budget is F64_BUDGET_BIG_LEAF: 81,920 triangles,
+//    queries in the box, 65,536: 1.34 ms at 256, 1.12 at 512, 1.45 at 1,024; 262,144: 4.20, 2.54, 2.80 (3.48 one query per
+//    thread); near the surface the same.
+constexpr int F64_BUDGET_BIG_LEAF = 512;
 constexpr int64_t F64_WARP_MAX = 3072;
 constexpr int64_t F64_WARP_MAX_SMALL = 2048;
 constexpr int64_t F64_SMALL_MESH = 2048;
@@ -1085,6 +1089,7 @@ void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams c
     THEA_LAUNCH(query_range_kernel, 1, 1, 0, s, qoff.as<int64_t>(), n);
     ClosestParams c2 = cp;
     c2.budget = n < 8192 ? 64 : (n < 32768 ? 128 : CLOSEST_TWO_PHASE_BUDGET);
+    if (b->width == 4 && b->leaf_size >= 8 && n >= 32768) c2.budget = F64_BUDGET_BIG_LEAF;
     run_batch_closest(b, q, qoff.as<int64_t>(), n, c2, 64, idx, dist, cpt, errout, s);
     return;
   }
