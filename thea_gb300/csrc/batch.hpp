@@ -23,10 +23,11 @@ BatchForest forest_view(thea_bvh const * b);
 
 // Step budget of a batched closest-point search whose caller names none. A query past its budget is finished by a whole
 // warp, which shortens the launch's longest chains but costs the GPU about five times a thread's search, so a batch that
-// fills the GPU hands over only its longest queries: 256 meshes of 320 to 327,680 triangles with 5.2 M queries, FP32:
-// 33.3 / 17.7 / 12.4 / 12.3 ms at budgets of 32 / 128 / 256 / 384, FP64 re-check: 72 / 31 / 22.5 / 22.7 ms; 64 meshes with
-// 210,677 queries: 1.30 / 1.20 / 1.28 / 1.43 and 3.0 / 1.79 / 2.02 / 2.25 ms. A small batch is bound by its longest chain
-// instead (config-0 mesh, 32,768 queries: 0.44 ms at 16 steps, 0.89 at 256; 131,072: 1.30 and 1.15 ms).
+// fills the GPU hands over only its longest queries. 256 meshes of 320 to 327,680 triangles with 5.2 M queries: FP32 9.0 /
+// 8.6 ms at budgets of 256 / 384 (with the searches as they were before: 33.3 / 17.7 / 12.4 / 12.3 at 32 / 128 / 256 / 384),
+// FP64 re-check 35.1 / 23.6 / 20.3 / 19.5 at 128 / 192 / 256 / 384; 64 meshes with 210,677 queries: FP32 1.28 / 0.80 / 0.80
+// / 0.89 at 32 / 160 / 256 / 384, FP64 1.60 / 1.42 / 1.40 / 1.48 at 128 / 192 / 256 / 384. A small batch is bound by its
+// longest chain instead (81,920 triangles, two kernels: 32,768 queries 0.44 ms at 16 steps, 0.89 at 256).
 inline int batch_closest_budget(int64_t nq) { return nq >= 98304 ? 256 : 32; }
 
 // qoff: device array of M + 1 query offsets (queries of segment m are [qoff[m], qoff[m+1])). chunk: queries a warp
