@@ -1106,10 +1106,11 @@ void init_slabs(thea_bvh * b, cudaStream_t stream) {
 
 void init_segment_roots(thea_bvh * b, cudaStream_t stream) {
   int M = b->num_segments;
-  std::vector<RootCut> h((size_t)M);
+  std::vector<RootCut> & h = b->seg_roots_host;
+  h.resize((size_t)M);
   for (int s = 0; s < M; ++s) h[(size_t)s] = root_cut_of(&b->seg_lo[3 * (size_t)s], &b->seg_hi[3 * (size_t)s], nullptr);
   if (!b->seg_roots) THEA_CUDA_CHECK(thea_malloc_async(&b->seg_roots, (size_t)M * sizeof(RootCut), stream));
-  // (pageable memory: the copy has read h when the call returns)
+  // (the handle keeps h: an asynchronous copy from pageable memory may read it late)
   THEA_CUDA_CHECK(cudaMemcpyAsync(b->seg_roots, h.data(), (size_t)M * sizeof(RootCut), cudaMemcpyHostToDevice, stream));
 }
 

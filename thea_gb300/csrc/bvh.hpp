@@ -41,6 +41,7 @@ struct thea_bvh {
   std::vector<int64_t> seg_start_host;
   std::vector<float> seg_lo, seg_hi;  // per-segment element bounds (3 floats each)
   RootCut * seg_roots = nullptr;      // device, num_segments: per-segment root cuts (distance bounds of closest queries)
+  std::vector<RootCut> seg_roots_host;  // what seg_roots is copied from: lives as long as the copy may be under way
   // affine transform (BvhN::setTransform): row-major 3x4 [L | t] and its FP32 inverse; `world` is the world-space copy
   // of the element records that closest-point, k-NN and radius queries read (it shares this handle's error word)
   int32_t has_transform = 0;
@@ -59,7 +60,8 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
                         int64_t const * seg_start_host, int M, thea_build_config const & cfg, cudaStream_t stream);
 void destroy_bvh(thea_bvh * b);
 
-// Fills seg_roots from seg_lo / seg_hi (allocates it; synchronizes the stream)
+// Fills seg_roots_host from seg_lo / seg_hi and copies it to seg_roots (allocated if need be) on the stream, which the
+// caller synchronizes before it hands out or destroys the handle
 void init_segment_roots(thea_bvh * b, cudaStream_t stream);
 // The oriented slabs of a single-mesh BVH with the closest layout, from its nodes and records (after a build, and after
 // loading an image); other handles, and node arrays that do not follow the build's layout, get none.
