@@ -14,6 +14,16 @@ namespace thea {
 
 constexpr int WARP_STACK = 1024;  // entries per warp (code + bound = 8 KB)
 
+// Nodes a warp's step pops from a stack of sp entries: 32 / W, but one at a time once the stack is nearly full. A step leaves
+// at most 31 entries more than it found, and one node at a time the stack grows by at most (W - 1) x depth more (depth-first),
+// which the build keeps below 256 (W = 4) or 512 (W = 8): so no tree that a build accepts overfills it. Trees of ordinary
+// depth stay far below the line (81,920 triangles, width 4: at most 8 x (3 x 10 + 1) entries).
+template <int W> __device__ __forceinline__ int warp_pops(int sp) {
+  constexpr int NEARLY_FULL = WARP_STACK - 32 - (W == 4 ? 256 : 512);
+  int most = sp > NEARLY_FULL ? 1 : 32 / W;
+  return sp < most ? sp : most;
+}
+
 // Lexicographic (d2, index) key: non-negative float bits order like unsigned integers.
 __device__ __forceinline__ unsigned long long best_key(float d2, int idx) {
   return ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)idx;
@@ -75,7 +85,6 @@ __device__ WarpBest closest_warp_query(WideNode<W> const * __restrict__ nodes, f
                                        int root, int64_t elem_base, V3 p, WarpBest best, int * s_code, float * s_lb,
                                        unsigned * err, float4 const * __restrict__ slabs = nullptr) {
   float q1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
-  constexpr int NPOP = 32 / W;
   int lane = threadIdx.x & 31;
   int e = lane / W, c = lane % W;
   int sp = 1;
@@ -86,7 +95,7 @@ __device__ WarpBest closest_warp_query(WideNode<W> const * __restrict__ nodes, f
   __syncwarp();
   unsigned long long bkey = best_key(best.d2, best.idx);
   while (sp > 0) {
-    int npop = sp < NPOP ? sp : NPOP;
+    int npop = warp_pops<W>(sp);
     int base = sp - npop;
     int code = CHILD_EMPTY;
     float lbe = 0.f;
@@ -294,7 +303,6 @@ __device__ WarpBest64 closest_warp_query_f64(WideNode<W> const * __restrict__ no
                                              int root, int64_t elem_base, V3 p, double bound2, float scale,
                                              float init_best32, int * s_code, float * s_lb, float * s_cd,
                                              int64_t * s_ck, unsigned * err, float4 const * __restrict__ slabs) {
-  constexpr int NPOP = 32 / W;
   float q1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
   float const REL = 1.0f + 1.0f / 16384.0f;
   float abs_tol = scale * (1.0f / 262144.0f);
@@ -330,7 +338,7 @@ __device__ WarpBest64 closest_warp_query_f64(WideNode<W> const * __restrict__ no
   }
   __syncwarp();
   while (sp > 0) {
-    int npop = sp < NPOP ? sp : NPOP;
+    int npop = warp_pops<W>(sp);
     int base = sp - npop;
     int code = CHILD_EMPTY;
     float lbe = 0.f;
