@@ -365,12 +365,13 @@ THEA_API thea_status thea_point_forest_build(const float * points, const int64_t
  * [query_offsets[m], query_offsets[m+1]) (num_meshes + 1 entries). Every array must be device memory; the calls are
  * asynchronous on `stream`, allocate only from the library's stream-ordered pool and never synchronize, so a sequence of
  * them can be captured with thea_graph_capture_begin/end. queries_per_warp: queries a warp takes per work fetch
- * (multiple of 32; 0 = 64). Per-query results as the single-BVH calls; the loop of closestElement calls over many meshes
+ * (multiple of 32; 0 = 64; fewer where a batch is too small to give every warp as many). Per-query results as the single-BVH calls; the loop of closestElement calls over many meshes
  * that this replaces is the reference's only form.
  * hard_query_budget (closest element only): each query first runs on one thread for at most this many traversal steps;
  * queries that need more (points deep inside a closed mesh, where thousands of nodes lie within the bound) are then
- * finished by a whole warp each, 32 lanes expanding nodes together. 0 = default (32; 256 from 98,304 queries on), negative = one thread per query
- * throughout. Results do not depend on it. */
+ * finished by a whole warp each, 32 lanes expanding nodes together. 0 = default (32; 256 from 98,304 queries on),
+ * negative = one thread per query throughout (THEA_PRECISION_FP64_RECHECK: but for a query with more than eight elements
+ * within its error band, which goes to a warp at any budget). Results do not depend on it. */
 THEA_API thea_status thea_batch_closest_element(const thea_bvh * mesh_forest, const float * queries,
                                                 const int64_t * query_offsets, int64_t num_queries, float dist_bound,
                                                 int32_t precision, int32_t queries_per_warp, int32_t hard_query_budget,
@@ -411,8 +412,8 @@ typedef struct thea_tuning {
 
 /* Times batched closest-point queries on a sample workload (a mesh forest's inputs plus device queries grouped by
  * mesh) for every BVH width (4, 8) and leaf size (1, 2, 4): queries-per-warp (32, 64, 128) with one thread per query
- * throughout, then step budgets (12, 32, 128) at the best queries-per-warp; returns the fastest (36 candidates).
- * Synchronizes the stream. */
+ * throughout, then step budgets (12, 32, 128; also 256 and 384 from 98,304 queries on) at the best queries-per-warp;
+ * returns the fastest (36 or 48 candidates). Synchronizes the stream. */
 THEA_API thea_status thea_autotune_batch_closest(const float * vertices, int64_t num_vertices, const int32_t * faces,
                                                  const int64_t * mesh_face_offsets, int32_t num_meshes,
                                                  const float * queries, const int64_t * query_offsets,

@@ -29,6 +29,7 @@ struct State {
   std::vector<std::function<void()>> queue;  // work not yet done
   std::map<void const *, std::string> names; // kernels by host entry point
   std::vector<std::string> launches;         // mangled names, in order
+  std::function<void(std::string const &, void **)> on_launch;  // sees each launch's name and arguments
 };
 inline State & state() {
   static State s;
@@ -130,8 +131,10 @@ cudaError_t __cudaPopCallConfiguration(dim3 * g, dim3 * b, size_t * m, void * s)
   return cudaSuccess;
 }
 cudaError_t __cudaGetKernel(cudaKernel_t * k, void const * host) { *k = (cudaKernel_t)host; return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **, size_t, cudaStream_t) {
-  fake::state().launches.push_back(fake::state().names[(void const *)k]);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void ** args, size_t, cudaStream_t) {
+  std::string const & name = fake::state().names[(void const *)k];
+  fake::state().launches.push_back(name);
+  if (fake::state().on_launch) fake::state().on_launch(name, args);
   return cudaSuccess;
 }
 

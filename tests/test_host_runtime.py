@@ -18,7 +18,7 @@ def run():
     objects = sorted(glob.glob(os.path.join(B.BUILD, "*.o")))
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(B.nvcc())))
 
-    def go(name):
+    def go(name, *args):
         src = os.path.join(ROOT, "tests", "cpp", name + ".cpp")
         out = os.path.join(ROOT, "tests", "cpp", "_build", name)
         os.makedirs(os.path.dirname(out), exist_ok=True)
@@ -26,7 +26,7 @@ def run():
                            ["-o", out, "-lpthread", "-ldl", "-Wl,--unresolved-symbols=ignore-all"],
                            capture_output=True, text=True)
         assert r.returncode == 0, r.stderr[-4000:]
-        r = subprocess.run([out], capture_output=True, text=True, timeout=600)
+        r = subprocess.run([out] + list(args), capture_output=True, text=True, timeout=600)
         assert r.returncode == 0, r.stdout + r.stderr
         return r.stdout
 
@@ -35,3 +35,7 @@ def run():
 
 def test_segment_cuts_outlive_their_copy(run):
     assert "segment cuts whole" in run("segment_cuts_check")
+
+
+def test_batches_fetch_work_as_asked(run):
+    assert "fetches as asked" in run("batch_fetch_check")

@@ -1263,7 +1263,10 @@ THEA_API thea_status thea_autotune_batch_closest(const float * vertices, int64_t
     thea_tuning best{};
     best.milliseconds = INFINITY;
     int tried = 0;
-    int const widths[2] = {4, 8}, leaves[3] = {1, 2, 4}, chunks[3] = {32, 64, 128}, budgets[3] = {12, 32, 128};
+    int const widths[2] = {4, 8}, leaves[3] = {1, 2, 4}, chunks[3] = {32, 64, 128};
+    // step budgets around the default of the sample's size (batch_closest_budget)
+    std::vector<int> budgets = {12, 32, 128};
+    if (batch_closest_budget(num_queries) > 128) budgets.insert(budgets.end(), {256, 384});
     for (int w : widths)
       for (int l : leaves) {
         thea_build_config cfg{};

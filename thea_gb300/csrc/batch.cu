@@ -143,7 +143,7 @@ batch_closest_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lon
 
 // Persistent-lane form of batch_closest_kernel: lanes take new queries as theirs end, instead of idling until the slowest
 // query of its warp's round (the queries deep inside a mesh take ten times the steps of the others). Every loop iteration
-// advances each busy lane by one stack entry; idle lanes are refilled from a warp-local block of up to 64 query indices.
+// advances each busy lane by one stack entry; idle lanes are refilled from a warp-local block of query indices (`block`).
 // FP32 search only; closest_collect_kernel below is the mixed-precision form. Results are the round-based kernel's: each
 // query's search is the same sequence of steps.
 //
@@ -785,11 +785,11 @@ int persistent_grid(void const * kernel) {
   return std::max(1, per_sm) * sms;
 }
 
-// Blocks of query indices a warp takes at a time: no larger than a warp's share, so that a small batch keeps every warp
-// busy
-int refill_block(int64_t nq, int grid) {
+// Blocks of query indices a warp takes at a time: the caller's `chunk`, but no larger than a warp's share, so that a small
+// batch keeps every warp busy
+int refill_block(int64_t nq, int grid, int chunk) {
   int64_t per = ceil_div(nq, (int64_t)grid * (BATCH_THREADS / 32));
-  return (int)std::min<int64_t>(REFILL_BLOCK, std::max<int64_t>(1, per));
+  return (int)std::min<int64_t>(chunk, std::max<int64_t>(1, per));
 }
 
 template <int W, int STACK>
@@ -801,7 +801,7 @@ void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t 
     auto k1 = closest_collect_kernel<W, STACK>;
     int grid = persistent_grid((void const *)k1);
     THEA_LAUNCH_NAMED("batch_closest_kernel_fp64", k1, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq,
-                      refill_block(nq, grid), cand.as<int32_t>());
+                      refill_block(nq, grid, chunk), cand.as<int32_t>());
     THEA_LAUNCH_NAMED("closest_resolve_kernel", closest_resolve_kernel, (unsigned)ceil_div(nq, BATCH_THREADS),
                       BATCH_THREADS, 0, s, f, a, nq, cand.as<int32_t>());
     auto k2 = batch_closest_phase2_kernel<W, THEA_PRECISION_FP64_RECHECK>;
@@ -814,7 +814,8 @@ void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t 
   if (!a.out_err) {
     auto kr = batch_closest_refill_kernel<W, STACK>;
     int grid = persistent_grid((void const *)kr);
-    THEA_LAUNCH_NAMED(name, kr, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq, refill_block(nq, grid));
+    THEA_LAUNCH_NAMED(name, kr, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq,
+                      refill_block(nq, grid, chunk));
   } else {
     auto k1 = batch_closest_kernel<W, STACK>;
     THEA_LAUNCH_NAMED(name, k1, persistent_grid((void const *)k1), BATCH_THREADS, 0, s, f, a, nq, counters, chunk,
