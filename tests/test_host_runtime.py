@@ -39,3 +39,7 @@ def test_segment_cuts_outlive_their_copy(run):
 
 def test_batches_fetch_work_as_asked(run):
     assert "fetches as asked" in run("batch_fetch_check")
+
+
+def test_mixed_precision_scratch_is_bounded(run):
+    assert "batches bounded" in run("scratch_check")

@@ -429,9 +429,9 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS)
-closest_resolve_kernel(BatchForest f, ClosestArgs a, int64_t nq, int32_t const * __restrict__ cand) {
+closest_resolve_kernel(BatchForest f, ClosestArgs a, int64_t q0, int64_t nq, int32_t const * __restrict__ cand) {
   __shared__ F64WarpBuf s_buf[BATCH_THREADS / 32];
-  int64_t q = (int64_t)blockIdx.x * BATCH_THREADS + threadIdx.x;
+  int64_t q = q0 + (int64_t)blockIdx.x * BATCH_THREADS + threadIdx.x;
   bool active = q < nq;
   F64Search s;
   f64_search_init(s);
@@ -792,21 +792,38 @@ int refill_block(int64_t nq, int grid, int chunk) {
   return (int)std::min<int64_t>(chunk, std::max<int64_t>(1, per));
 }
 
+// Queries of a mixed-precision batch that are collected and resolved at a time: the candidates and the queue of unfinished
+// queries take 56 bytes each, 5 GB for the 90 million of 4,096 meshes at once, 235 MB in slices.
+constexpr int64_t F64_SLICE = int64_t(1) << 22;
+
+__global__ void slice_counters_kernel(unsigned long long * counters, int64_t q0) {
+  counters[0] = (unsigned long long)q0;  // next query
+  counters[1] = 0;                       // next queued query
+  counters[2] = 0;                       // queued queries
+}
+
 template <int W, int STACK>
 void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t nq, int prec, int budget,
                           unsigned long long * counters, int chunk, HardQueue const & hq, cudaStream_t s) {
   int first_budget = budget > 0 ? budget : 0;
   if (prec == THEA_PRECISION_FP64_RECHECK) {
-    Scratch cand((size_t)nq * F64_CAND * sizeof(int32_t), s);
+    // slice by slice, each from its first query on in the arrays of the whole batch
+    Scratch cand((size_t)std::min(nq, F64_SLICE) * F64_CAND * sizeof(int32_t), s);
     auto k1 = closest_collect_kernel<W, STACK>;
-    int grid = persistent_grid((void const *)k1);
-    THEA_LAUNCH_NAMED("batch_closest_kernel_fp64", k1, grid, BATCH_THREADS, 0, s, f, a, nq, counters, first_budget, hq,
-                      refill_block(nq, grid, chunk), cand.as<int32_t>());
-    THEA_LAUNCH_NAMED("closest_resolve_kernel", closest_resolve_kernel, (unsigned)ceil_div(nq, BATCH_THREADS),
-                      BATCH_THREADS, 0, s, f, a, nq, cand.as<int32_t>());
     auto k2 = batch_closest_phase2_kernel<W, THEA_PRECISION_FP64_RECHECK>;
-    THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, persistent_grid((void const *)k2), BATCH_THREADS, 0, s, f, a, hq,
-                      counters + 1);
+    int grid = persistent_grid((void const *)k1), grid2 = persistent_grid((void const *)k2);
+    for (int64_t q0 = 0; q0 < nq; q0 += F64_SLICE) {
+      int64_t end = std::min(nq, q0 + F64_SLICE);
+      // (its entries are found at 8 q: as if the array began with query 0's)
+      int32_t * c = reinterpret_cast<int32_t *>(reinterpret_cast<uintptr_t>(cand.ptr) -
+                                                (uintptr_t)q0 * (F64_CAND * sizeof(int32_t)));
+      if (q0 > 0) THEA_LAUNCH(slice_counters_kernel, 1, 1, 0, s, counters, q0);
+      THEA_LAUNCH_NAMED("batch_closest_kernel_fp64", k1, grid, BATCH_THREADS, 0, s, f, a, end, counters, first_budget, hq,
+                        refill_block(end - q0, grid, chunk), c);
+      THEA_LAUNCH_NAMED("closest_resolve_kernel", closest_resolve_kernel, (unsigned)ceil_div(end - q0, BATCH_THREADS),
+                        BATCH_THREADS, 0, s, f, a, q0, end, c);
+      THEA_LAUNCH_NAMED("batch_closest_phase2_kernel", k2, grid2, BATCH_THREADS, 0, s, f, a, hq, counters + 1);
+    }
     return;
   }
   char const * name = budget > 0 ? "batch_closest_phase1_kernel" : "batch_closest_kernel_fp32";
@@ -882,8 +899,9 @@ void batch_closest_core(thea_bvh const * b, ClosestArgs const & a, int64_t nq, C
   Scratch counters(3 * sizeof(unsigned long long), s);
   THEA_CUDA_CHECK(cudaMemsetAsync(counters.ptr, 0, 3 * sizeof(unsigned long long), s));
   auto * c = counters.as<unsigned long long>();
-  // (the mixed-precision search may hand over queries at any budget)
-  size_t hq_n = budget > 0 || cp.precision == THEA_PRECISION_FP64_RECHECK ? (size_t)nq : 0;
+  // (the mixed-precision search may hand over queries at any budget, a slice of the batch at a time)
+  size_t hq_n = budget > 0 ? (size_t)nq : 0;
+  if (cp.precision == THEA_PRECISION_FP64_RECHECK) hq_n = (size_t)std::min(nq, F64_SLICE);
   Scratch hq_q(hq_n * sizeof(int64_t), s), hq_b(hq_n * sizeof(float), s);
   Scratch hq_i(hq_n * sizeof(int32_t), s), hq_s(hq_n * sizeof(int64_t), s);
   HardQueue hq{hq_q.as<int64_t>(), hq_b.as<float>(), hq_i.as<int32_t>(), hq_s.as<int64_t>(), c + 2};
