@@ -1,5 +1,5 @@
-// Scratch memory the library asks for: a batch in the mixed-precision mode takes no more than one slice's, however large it
-// is.
+// Scratch memory the library asks for: what a build takes an element does not jump with its size, and a batch in the
+// mixed-precision mode takes no more than one slice's, however large it is.
 #include "fake_cuda.hpp"
 
 #include "../../thea_gb300/csrc/common.cuh"
@@ -9,7 +9,37 @@
 
 using namespace thea;
 
-int main() {
+static size_t build_peak(int64_t n, int width) {
+  fake::State & s = fake::state();
+  thea_build_config cfg{};
+  cfg.width = width;
+  cfg.max_leaf_size = 1;
+  std::vector<float> p(3);  // (no kernel reads it)
+  s.peak = s.now;
+  size_t before = s.now;
+  thea_bvh * b = build_bvh(false, p.data(), n, nullptr, 0, cfg, nullptr);
+  size_t peak = s.peak - before;
+  destroy_bvh(b);
+  cudaDeviceSynchronize();
+  return peak;
+}
+
+int main(int argc, char ** argv) {
+  if (argc > 1 && std::string(argv[1]) == "build") {
+    for (int width : {4, 8}) {
+      double most = 1.05 * (double)build_peak(8 << 20, width) / (8 << 20);
+      for (int64_t n : {300000, 1 << 20, 1 << 22, (1 << 22) + 1}) {
+        double per = (double)build_peak(n, width) / (double)n;
+        if (per > most) {
+          std::printf("width %d, %lld elements: %.0f bytes each at the peak, %.0f in a larger build\n", width, (long long)n, per,
+                      most);
+          return 1;
+        }
+      }
+    }
+    std::printf("builds scale\n");
+    return 0;
+  }
   fake::State & s = fake::state();
   thea_bvh b;
   b.is_mesh = 1;

@@ -43,3 +43,7 @@ def test_batches_fetch_work_as_asked(run):
 
 def test_mixed_precision_scratch_is_bounded(run):
     assert "batches bounded" in run("scratch_check")
+
+
+def test_build_scratch_scales(run):
+    assert "builds scale" in run("scratch_check", "build")

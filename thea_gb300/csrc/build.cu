@@ -624,8 +624,10 @@ __global__ void point_records_kernel(float const * __restrict__ P, int64_t n, in
 
 // Blocks of a level up to which the emitting kernel sums the counts of the blocks before it by itself
 constexpr int64_t COLLAPSE_SUM_BLOCKS = 1024;
-// Elements up to which the node array is first sized by the worst case; larger builds count their nodes first
-constexpr int64_t COLLAPSE_BOUND_MAX = 1 << 22;
+// Elements up to which the node array is first sized by the worst case; larger builds count their nodes first, at the price
+// of one more synchronisation. The worst case takes 107 bytes an element at width 4 and 165 at width 8 (leaves of one): 28
+// and 43 MB of scratch at this line, which the scratch pool keeps mapped; at 4,194,304 elements 447 and 690.
+constexpr int64_t COLLAPSE_BOUND_MAX = 1 << 18;
 
 // What the build reads back, in one copy: the collapse's two alternating levels, whether a face index was out of range,
 // and the bounds of every segment (12 ordered ints each, see elem_box_kernel)
