@@ -462,8 +462,8 @@ __device__ WarpBest64 closest_warp_query_f64(WideNode<W> const * __restrict__ no
   WarpBest64 out;
   out.d2 = wmin;
   out.idx = (int)widx;
+  // (a query at infinity finds an element at infinite distance, as the one-thread search does; INT_MAX: none)
   out.slot = who ? __shfl_sync(0xffffffffu, my_slot, __ffs(who) - 1) : -1;
-  if (!(wmin < INFINITY)) out.idx = INT_MAX;
   return out;
 }
 
