@@ -44,7 +44,7 @@ __device__ __forceinline__ bool next_chunk(unsigned long long * counter, int chu
 // round (lanes past the end of the chunk carry no query), so the warp-wide FP64 step of the mixed-precision search and
 // the FP64 error estimate run with all lanes together.
 //
-// Two-phase form: with budget > 0, phase 1 stops a query after that many stack pops and queues it with the best
+// Two-phase form: with budget > 0, phase 1 stops a query after that many steps (nodes and leaves) and queues it with the best
 // element found so far (a valid upper bound); phase 2 finishes the queued queries with one warp per query.
 //============================================================================================================================
 
@@ -249,6 +249,7 @@ batch_closest_refill_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned l
     }
     closest_step<W>(nodes, f.cp_rec, ebase, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, f.err, nullptr,
                     0.f);
+    pops -= leaf_rest(code, next);
   }
 }
 
@@ -400,6 +401,7 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
           V3 cp;
           take(cp_record_eval(r, p, cp), first);
           if (count > 1) next = encode_leaf(first + 1, count - 1);
+          steps -= leaf_rest(code, next);
         }
       } else {
         if (code >= 0) {
@@ -715,7 +717,8 @@ closest_stream_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lo
       if (__int_as_float(top.y) > best * PRUNE_SLACK) continue;
     }
     closest_step<W>(nodes, f.cp_rec, 0, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, f.err, nullptr,
-                           0.f);
+                    0.f);
+    pops -= leaf_rest(code, next);
   }
 }
 

@@ -502,6 +502,10 @@ __device__ __forceinline__ void closest_step(WideNode<W> const * __restrict__ no
   }
 }
 
+// 1 where the step at `code` tested an element of a leaf and left the others to the next step, which a step budget then does
+// not count again: a budget counts nodes and leaves, however many steps a leaf takes.
+__device__ __forceinline__ int leaf_rest(int code, int next) { return code < 0 && next != CHILD_EMPTY ? 1 : 0; }
+
 // FP32 reference-arithmetic search: smallest (d2, index), accepting d2 <= thresh. With budget > 0 the search stops
 // after that many stack pops (done = false), leaving the best found so far. With the BVH's oriented slabs (single
 // mesh BVHs) the children's bounds are raised to their slab bounds; the result is the same, the search shorter.
@@ -538,6 +542,7 @@ __device__ __forceinline__ ClosestOut closest_query(WideNode<W> const * __restri
     }
     if constexpr (FUSED) {
       closest_step<W>(nodes, rec, elem_base, code, p, best, best_idx, best_slot, best_cp, stk, sp, next, err, slabs, q1);
+      pops -= leaf_rest(code, next);
     } else {
       next = CHILD_EMPTY;
       if (code >= 0) {
