@@ -25,6 +25,7 @@ namespace fake {
 
 struct State {
   size_t now = 0, peak = 0;                  // device bytes allocated
+  int allocations = 0;
   std::map<void *, size_t> sizes;            // live device allocations
   std::vector<std::function<void()>> queue;  // work not yet done
   std::map<void const *, std::string> names; // kernels by host entry point
@@ -44,6 +45,7 @@ inline cudaError_t allocate(void ** p, size_t n) {
   if (!*p) return cudaErrorMemoryAllocation;
   State & s = state();
   s.sizes[*p] = n;
+  ++s.allocations;
   s.now += n;
   s.peak = std::max(s.peak, s.now);
   return cudaSuccess;

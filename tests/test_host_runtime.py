@@ -47,3 +47,7 @@ def test_mixed_precision_scratch_is_bounded(run):
 
 def test_build_scratch_scales(run):
     assert "builds scale" in run("scratch_check", "build")
+
+
+def test_small_calls_ask_little_of_the_runtime(run):
+    assert "small calls are small" in run("small_call_check")

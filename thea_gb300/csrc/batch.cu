@@ -805,20 +805,45 @@ __global__ void slice_counters_kernel(unsigned long long * counters, int64_t q0)
   counters[2] = 0;                       // queued queries
 }
 
+// Scratch of one closest-point batch, in one allocation: the counters (zeroed on the stream), the queue of `queue` unfinished
+// queries and the band candidates of `cand` queries. (Six allocations and a kernel that wrote one BVH's query range, which
+// nothing reads, cost a small call 8 us of host time.)
+struct ClosestScratch {
+  Scratch all;
+  unsigned long long * counters;  // next query, next queued query, queued queries
+  HardQueue hq;
+  int32_t * cand;
+  ClosestScratch(int64_t queue, int64_t cands, cudaStream_t s)
+      : all((size_t)(64 + queue * (int64_t)(2 * sizeof(int64_t) + sizeof(float) + sizeof(int32_t)) +
+                     cands * (int64_t)(F64_CAND * sizeof(int32_t))), s) {
+    char * p = all.as<char>();
+    counters = reinterpret_cast<unsigned long long *>(p);
+    cand = reinterpret_cast<int32_t *>(p + 64);
+    p += 64 + cands * (int64_t)(F64_CAND * sizeof(int32_t));
+    hq.q = reinterpret_cast<int64_t *>(p);
+    hq.slot = hq.q + queue;
+    hq.bound = reinterpret_cast<float *>(hq.slot + queue);
+    hq.idx = reinterpret_cast<int32_t *>(hq.bound + queue);
+    hq.count = counters + 2;
+    THEA_CUDA_CHECK(cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), s));
+  }
+};
+
 template <int W, int STACK>
-void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t nq, int prec, int budget,
-                          unsigned long long * counters, int chunk, HardQueue const & hq, cudaStream_t s) {
+void launch_batch_closest(BatchForest const & f, ClosestArgs const & a, int64_t nq, int prec, int budget, int chunk,
+                          ClosestScratch const & w, cudaStream_t s) {
+  unsigned long long * counters = w.counters;
+  HardQueue const & hq = w.hq;
   int first_budget = budget > 0 ? budget : 0;
   if (prec == THEA_PRECISION_FP64_RECHECK) {
     // slice by slice, each from its first query on in the arrays of the whole batch
-    Scratch cand((size_t)std::min(nq, F64_SLICE) * F64_CAND * sizeof(int32_t), s);
     auto k1 = closest_collect_kernel<W, STACK>;
     auto k2 = batch_closest_phase2_kernel<W, THEA_PRECISION_FP64_RECHECK>;
     int grid = persistent_grid((void const *)k1), grid2 = persistent_grid((void const *)k2);
     for (int64_t q0 = 0; q0 < nq; q0 += F64_SLICE) {
       int64_t end = std::min(nq, q0 + F64_SLICE);
       // (its entries are found at 8 q: as if the array began with query 0's)
-      int32_t * c = reinterpret_cast<int32_t *>(reinterpret_cast<uintptr_t>(cand.ptr) -
+      int32_t * c = reinterpret_cast<int32_t *>(reinterpret_cast<uintptr_t>(w.cand) -
                                                 (uintptr_t)q0 * (F64_CAND * sizeof(int32_t)));
       if (q0 > 0) THEA_LAUNCH(slice_counters_kernel, 1, 1, 0, s, counters, q0);
       THEA_LAUNCH_NAMED("batch_closest_kernel_fp64", k1, grid, BATCH_THREADS, 0, s, f, a, end, counters, first_budget, hq,
@@ -899,19 +924,14 @@ void batch_closest_core(thea_bvh const * b, ClosestArgs const & a, int64_t nq, C
   BatchForest f = forest_view(b);
   bool sm = small_stack_ok(b);
   int budget = cp.budget > 0 ? cp.budget : 0;
-  Scratch counters(3 * sizeof(unsigned long long), s);
-  THEA_CUDA_CHECK(cudaMemsetAsync(counters.ptr, 0, 3 * sizeof(unsigned long long), s));
-  auto * c = counters.as<unsigned long long>();
   // (the mixed-precision search may hand over queries at any budget, a slice of the batch at a time)
-  size_t hq_n = budget > 0 ? (size_t)nq : 0;
-  if (cp.precision == THEA_PRECISION_FP64_RECHECK) hq_n = (size_t)std::min(nq, F64_SLICE);
-  Scratch hq_q(hq_n * sizeof(int64_t), s), hq_b(hq_n * sizeof(float), s);
-  Scratch hq_i(hq_n * sizeof(int32_t), s), hq_s(hq_n * sizeof(int64_t), s);
-  HardQueue hq{hq_q.as<int64_t>(), hq_b.as<float>(), hq_i.as<int32_t>(), hq_s.as<int64_t>(), c + 2};
-  if (b->width == 4) sm ? launch_batch_closest<4, 64>(f, a, nq, cp.precision, budget, c, chunk, hq, s)
-                        : launch_batch_closest<4, 256>(f, a, nq, cp.precision, budget, c, chunk, hq, s);
-  else sm ? launch_batch_closest<8, 128>(f, a, nq, cp.precision, budget, c, chunk, hq, s)
-          : launch_batch_closest<8, 512>(f, a, nq, cp.precision, budget, c, chunk, hq, s);
+  bool f64 = cp.precision == THEA_PRECISION_FP64_RECHECK;
+  int64_t slice = std::min(nq, F64_SLICE);
+  ClosestScratch w(f64 ? slice : (budget > 0 ? nq : 0), f64 ? slice : 0, s);
+  if (b->width == 4) sm ? launch_batch_closest<4, 64>(f, a, nq, cp.precision, budget, chunk, w, s)
+                        : launch_batch_closest<4, 256>(f, a, nq, cp.precision, budget, chunk, w, s);
+  else sm ? launch_batch_closest<8, 128>(f, a, nq, cp.precision, budget, chunk, w, s)
+          : launch_batch_closest<8, 512>(f, a, nq, cp.precision, budget, chunk, w, s);
 }
 
 }  // namespace
@@ -969,17 +989,11 @@ void run_closest_stream(thea_bvh const * b, float const * q, int64_t nq, Closest
   bool sm = small_stack_ok(b);
   ClosestArgs a{q, nullptr, cp.thresh, cp.bound2, cp.scene_scale, idx, dist, cpt, nullptr};
   int budget = cp.budget > 0 ? cp.budget : 0;
-  Scratch counters(3 * sizeof(unsigned long long), s);
-  THEA_CUDA_CHECK(cudaMemsetAsync(counters.ptr, 0, 3 * sizeof(unsigned long long), s));
-  auto * c = counters.as<unsigned long long>();
-  size_t hq_n = budget > 0 ? (size_t)nq : 1;
-  Scratch hq_q(hq_n * sizeof(int64_t), s), hq_b(hq_n * sizeof(float), s);
-  Scratch hq_i(hq_n * sizeof(int32_t), s), hq_s(hq_n * sizeof(int64_t), s);
-  HardQueue hq{hq_q.as<int64_t>(), hq_b.as<float>(), hq_i.as<int32_t>(), hq_s.as<int64_t>(), c + 2};
-  if (b->width == 4) sm ? launch_closest_stream<4, 64>(f, a, nq, budget, c, hq, s)
-                        : launch_closest_stream<4, 256>(f, a, nq, budget, c, hq, s);
-  else sm ? launch_closest_stream<8, 128>(f, a, nq, budget, c, hq, s)
-          : launch_closest_stream<8, 512>(f, a, nq, budget, c, hq, s);
+  ClosestScratch w(budget > 0 ? nq : 1, 0, s);
+  if (b->width == 4) sm ? launch_closest_stream<4, 64>(f, a, nq, budget, w.counters, w.hq, s)
+                        : launch_closest_stream<4, 256>(f, a, nq, budget, w.counters, w.hq, s);
+  else sm ? launch_closest_stream<8, 128>(f, a, nq, budget, w.counters, w.hq, s)
+          : launch_closest_stream<8, 512>(f, a, nq, budget, w.counters, w.hq, s);
 }
 
 void run_batch_ray(thea_bvh const * b, float const * o, float const * d, int64_t const * qoff, int64_t nq,

@@ -30,8 +30,8 @@ BatchForest forest_view(thea_bvh const * b);
 // longest chain instead (81,920 triangles, two kernels: 32,768 queries 0.44 ms at 16 steps, 0.89 at 256).
 inline int batch_closest_budget(int64_t nq) { return nq >= 98304 ? 256 : 32; }
 
-// qoff: device array of M + 1 query offsets (queries of segment m are [qoff[m], qoff[m+1])). chunk: queries a warp
-// takes per fetch (a multiple of 32).
+// qoff: device array of M + 1 query offsets (queries of segment m are [qoff[m], qoff[m+1])), or null for one segment, whose
+// queries are all of them. chunk: queries a warp takes per fetch (a multiple of 32).
 void run_batch_closest(thea_bvh const * b, float const * q, int64_t const * qoff, int64_t nq, ClosestParams const & cp,
                        int chunk, int32_t * idx, float * dist, float * cpt, float * err, cudaStream_t s);
 // FP32 closest point of a small batch on one BVH (num_segments == 1, small_stack_ok), a whole warp per query below

@@ -601,11 +601,6 @@ constexpr int64_t F64_WARP_MAX_SMALL = 2048;
 constexpr int64_t F64_SMALL_MESH = 2048;
 constexpr int64_t F64_SMALL_LARGE_BATCH = 65536;
 
-__global__ void query_range_kernel(int64_t * qoff, int64_t n) {
-  qoff[0] = 0;
-  qoff[1] = n;
-}
-
 //============================================================================================================================
 // Points within a radius (BvhN::rangeQueryIndices with a Ball3 range, BvhN.hpp:1208-1219, 2118-2171; BallN::contains,
 // BallN.hpp:83: (p - center).squaredNorm() <= radius * radius, inclusive, FP32). Counting pass, then a filling pass into
@@ -1085,12 +1080,10 @@ void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams c
     return;
   }
   if (cp.precision == THEA_PRECISION_FP64_RECHECK && !f64_small) {
-    Scratch qoff(2 * sizeof(int64_t), s);
-    THEA_LAUNCH(query_range_kernel, 1, 1, 0, s, qoff.as<int64_t>(), n);
     ClosestParams c2 = cp;
     c2.budget = n < 8192 ? 64 : (n < 32768 ? 128 : CLOSEST_TWO_PHASE_BUDGET);
     if (b->width == 4 && b->leaf_size >= 8 && n >= 32768) c2.budget = F64_BUDGET_BIG_LEAF;
-    run_batch_closest(b, q, qoff.as<int64_t>(), n, c2, 64, idx, dist, cpt, errout, s);
+    run_batch_closest(b, q, nullptr, n, c2, 64, idx, dist, cpt, errout, s);
     return;
   }
   if (cp.precision == THEA_PRECISION_FP32_REFERENCE && !errout && !b->query_order &&
@@ -1101,11 +1094,9 @@ void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams c
     }
     // Persistent lanes with a step budget, then one warp per query over budget (the BVH is a one-mesh forest). The
     // same searches, so the same results.
-    Scratch qoff(2 * sizeof(int64_t), s);
-    THEA_LAUNCH(query_range_kernel, 1, 1, 0, s, qoff.as<int64_t>(), n);
     ClosestParams c2 = cp;
     c2.budget = n < CLOSEST_WARP_MAX ? CLOSEST_WARP_BUDGET : CLOSEST_TWO_PHASE_BUDGET;
-    run_batch_closest(b, q, qoff.as<int64_t>(), n, c2, 64, idx, dist, cpt, nullptr, s);
+    run_batch_closest(b, q, nullptr, n, c2, 64, idx, dist, cpt, nullptr, s);
     return;
   }
   // FP64 re-check: warps of Morton-ordered queries share band candidates (config 0: 2.64 -> 2.26 ms), so the order is
