@@ -5,11 +5,11 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-LINE = 1 << 18
+LINE = 1 << 21
 
 
 @pytest.mark.parametrize("width,leaf", [(4, 1), (8, 1), (4, 5)])
-@pytest.mark.parametrize("n", [LINE - 1, LINE, LINE + 1, 3 * LINE + 7])
+@pytest.mark.parametrize("n", [262145, LINE, LINE + 1, 2 * LINE + 7])
 def test_sizes(n, width, leaf):
     import torch
     import thea_gb300 as T

@@ -45,8 +45,8 @@ def test_mixed_precision_scratch_is_bounded(run):
     assert "batches bounded" in run("scratch_check")
 
 
-def test_build_scratch_scales(run):
-    assert "builds scale" in run("scratch_check", "build")
+def test_build_scratch_is_bounded(run):
+    assert "builds bounded" in run("scratch_check", "build")
 
 
 def test_small_calls_ask_little_of_the_runtime(run):

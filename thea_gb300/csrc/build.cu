@@ -624,10 +624,12 @@ __global__ void point_records_kernel(float const * __restrict__ P, int64_t n, in
 
 // Blocks of a level up to which the emitting kernel sums the counts of the blocks before it by itself
 constexpr int64_t COLLAPSE_SUM_BLOCKS = 1024;
-// Elements up to which the node array is first sized by the worst case; larger builds count their nodes first, at the price
-// of one more synchronisation. The worst case takes 107 bytes an element at width 4 and 165 at width 8 (leaves of one): 28
-// and 43 MB of scratch at this line, which the scratch pool keeps mapped; at 4,194,304 elements 447 and 690.
-constexpr int64_t COLLAPSE_BOUND_MAX = 1 << 18;
+// Elements up to which the node array is first sized by the worst case and the nodes copied out; larger builds count their
+// nodes first, at the price of one more synchronisation and of a larger array in the handle (the count bounds them too, but
+// less tightly). The worst case takes 107 bytes an element at width 4 and 165 at width 8 (leaves of one): 224 and 346 MB of
+// scratch at this line, which the scratch pool keeps mapped (with a line at 4,194,304 elements 447 and 690). Counted, the
+// array of a 2,093,058-triangle mesh made its build 7.6 ms instead of 6.9.
+constexpr int64_t COLLAPSE_BOUND_MAX = 1 << 21;
 
 // What the build reads back, in one copy: the collapse's two alternating levels, whether a face index was out of range,
 // and the bounds of every segment (12 ordered ints each, see elem_box_kernel)
