@@ -51,3 +51,7 @@ def test_build_scratch_is_bounded(run):
 
 def test_small_calls_ask_little_of_the_runtime(run):
     assert "small calls are small" in run("small_call_check")
+
+
+def test_closest_point_routes(run):
+    assert "routes as measured" in run("closest_routes_check")

@@ -580,22 +580,14 @@ constexpr int64_t CLOSEST_WARP_MAX = 57344;
 constexpr int CLOSEST_WARP_BUDGET = 16;
 constexpr int64_t CLOSEST_TWO_PHASE_MIN = 98304;
 constexpr int CLOSEST_TWO_PHASE_BUDGET = 256;
+//  * at width 8, where a step of 16 lanes expands two nodes, the teams end at CLOSEST_TEAM_MAX_W8: 81,920 triangles, leaves of
+//    four, 32,768 queries in the box 0.63 ms with 16 lanes, 0.51 in two kernels (six streams at once 2.98 and 2.41).
 
-// FP64 re-check calls on one BVH. Call times in ms, queries near the surface / uniform in the box grown by half:
-//  * fewer than F64_WARP_MAX queries (F64_WARP_MAX_SMALL on small meshes): a warp per query. 1,000 queries on 20,480
-//    triangles: 0.066 / 0.075, against 0.143 / 0.491 one query per thread.
-//  * otherwise the collecting and resolving kernels with a step budget of 64, 128 from 8,192 queries and 256 from 32,768:
-//    20,480 triangles, 12,000 queries 0.162 / 0.602 -> 0.136 / 0.383, 100,000: 0.436 / 1.23 -> 0.361 / 0.934, 250,000:
-//    0.691 / 1.95 -> 0.665 / 1.70; 81,920 triangles, 250,000: 0.983 / 2.53 -> 0.881 / 1.85.
-//  * on small meshes (F64_SMALL_MESH triangles; four times as many from F64_SMALL_LARGE_BATCH queries on) one query per
-//    thread, in Morton order, with slabs, the form compared with above: nodes and records stay in L1 or nearly, and a
-//    warp of neighbours reads them together. 1,280 triangles, 100,000 queries: 0.254 / 0.511 against 0.215 / 0.670 collected
-//    and resolved; 5,120 triangles: 0.323 / 0.769 against 0.269 / 0.937, but 50,000 queries 0.245 / 0.608 against 0.173 /
-//    0.597.
-//  * a step tests one element of a width-4 leaf, so with leaves of 8 the budget is F64_BUDGET_BIG_LEAF: 81,920 triangles,
-//    queries in the box, 65,536: 1.34 ms at 256, 1.12 at 512, 1.45 at 1,024; 262,144: 4.20, 2.54, 2.80 (3.48 one query per
-//    thread); near the surface the same.
-constexpr int F64_BUDGET_BIG_LEAF = 512;
+constexpr int64_t CLOSEST_TEAM_MAX_W8 = 16384;
+// FP64 re-check calls on one BVH: fewer than F64_WARP_MAX queries (F64_WARP_MAX_SMALL on small meshes) run as a warp per
+// query; the others through the collecting and resolving kernels with a step budget, or one query per thread, in Morton
+// order, with slabs. 1,000 queries on 20,480 triangles, near the surface / uniform in the box grown by half: a warp per query
+// 0.066 / 0.075 ms, one per thread 0.143 / 0.491.
 constexpr int64_t F64_WARP_MAX = 3072;
 constexpr int64_t F64_WARP_MAX_SMALL = 2048;
 constexpr int64_t F64_SMALL_MESH = 2048;
@@ -605,6 +597,38 @@ constexpr int64_t F64_SMALL_LARGE_BATCH = 65536;
 // Points within a radius (BvhN::rangeQueryIndices with a Ball3 range, BvhN.hpp:1208-1219, 2118-2171; BallN::contains,
 // BallN.hpp:83: (p - center).squaredNorm() <= radius * radius, inclusive, FP32). Counting pass, then a filling pass into
 // each query's slice of a CSR list; the slices are then put in ascending element order.
+bool f64_small_mesh(thea_bvh const * b, int64_t n) {
+  return b->n <= F64_SMALL_MESH || (b->n <= 4 * F64_SMALL_MESH && n >= F64_SMALL_LARGE_BATCH);
+}
+
+// Step budget of the collecting kernel, or 0 for one query per thread. The collected form is taken where no kind of query
+// (near the surface, in the box grown by half, in [-1, 1]^3, all deep inside, far outside) is slower in it. Its time over that
+// of one query per thread, the best kind and the worst, on 20,480, 81,920 and 327,680 triangles (budget):
+//  * width 4, leaves of one and two: 3,500 queries 0.27 - 0.76 (128), 8,192 0.45 - 0.87 (256), 32,768 0.57 - 0.82 (256), 65,536
+//    0.63 - 1.09 (256), 100,003 0.56 - 1.01 (256) and 0.58 - 1.03 (224; half the kinds 3 to 5 % faster), 131,072 0.59 - 1.16 (256) and 0.61 - 1.01 (384), 163,840 0.63 - 1.04 (384),
+//    262,144 0.70 - 1.33 (384): the slow ones are the queries deep inside, which the slabs of the one-per-thread form shorten
+//    tenfold. 5,120 triangles: 8,192 0.61 - 0.87 (128) and 0.67 - 1.18 (256).
+//  * width 4, larger leaves: 3,500 0.32 - 0.74 (128), 16,384 0.57 - 0.82 (128), 32,768 0.65 - 0.98 (256), 65,536 0.70 - 1.12
+//    (256), 262,144 0.74 - 1.60.
+//  * width 8, leaves of one and two: 3,500 0.34 - 0.71 (128), 16,384 0.61 - 0.85 (128), 32,768 0.58 - 0.95 (256), 131,072 0.46
+//    - 1.00 (256), 262,144 0.57 - 1.26. Leaves of four: 16,384 0.74 - 1.02 (128), 65,536 0.73 - 1.09 (256). Leaves of eight
+//    and sixteen: 8,192 0.56 - 1.19 (128), 65,536 0.74 - 1.73 (256).
+//  * small meshes: nodes and records stay in L1 or nearly, and a warp of neighbours reads them together. 1,280 triangles,
+//    100,000 queries in the box: 0.511 ms one per thread, 0.670 collected.
+// Calls of several streams at once pay for the warps that finish the queries over budget: six streams with 16,384 queries
+// each took 0.81 - 1.33 times as long as one per thread with these budgets (256; 1.01 - 1.50 with 128), at 0.52 - 0.92 of its
+// time on one stream.
+int f64_collect_budget(thea_bvh const * b, int64_t n) {
+  if (f64_small_mesh(b, n)) return 0;
+  if (b->width == 4) {
+    if (n < 8192 || (b->n <= 4 * F64_SMALL_MESH && n < 65536)) return 128;
+    if (b->leaf_size <= 2) return n < 81920 ? 256 : n < 114688 ? 224 : n < 163840 ? 384 : 0;
+    return n < 32768 ? 128 : n < 65536 ? 256 : 0;
+  }
+  if (b->leaf_size <= 2) return n < 32768 ? 128 : n < 131072 ? 256 : 0;
+  return b->leaf_size < 8 && n < 32768 ? 128 : 0;
+}
+
 //============================================================================================================================
 
 // Calls visit(leaf position, record) for every point under a node child whose box reaches within `lim` of p. Every such
@@ -1073,22 +1097,21 @@ bool small_stack_ok(thea_bvh const * b) {
 void run_closest(thea_bvh const * b, float const * q, int64_t n, ClosestParams const & cp, int32_t * idx, float * dist,
                  float * cpt, float * errout, unsigned * err, cudaStream_t s) {
   if (n <= 0) return;
-  bool f64_small = b->n <= F64_SMALL_MESH || (b->n <= 4 * F64_SMALL_MESH && n >= F64_SMALL_LARGE_BATCH);
-  if (cp.precision == THEA_PRECISION_FP64_RECHECK && n < (f64_small ? F64_WARP_MAX_SMALL : F64_WARP_MAX) &&
-      small_stack_ok(b)) {
-    run_closest_warps_f64(b, q, n, cp, idx, dist, cpt, errout, s);
-    return;
-  }
-  if (cp.precision == THEA_PRECISION_FP64_RECHECK && !f64_small) {
+  if (cp.precision == THEA_PRECISION_FP64_RECHECK) {
+    if (n < (f64_small_mesh(b, n) ? F64_WARP_MAX_SMALL : F64_WARP_MAX) && small_stack_ok(b)) {
+      run_closest_warps_f64(b, q, n, cp, idx, dist, cpt, errout, s);
+      return;
+    }
     ClosestParams c2 = cp;
-    c2.budget = n < 8192 ? 64 : (n < 32768 ? 128 : CLOSEST_TWO_PHASE_BUDGET);
-    if (b->width == 4 && b->leaf_size >= 8 && n >= 32768) c2.budget = F64_BUDGET_BIG_LEAF;
-    run_batch_closest(b, q, nullptr, n, c2, 64, idx, dist, cpt, errout, s);
-    return;
+    c2.budget = f64_collect_budget(b, n);
+    if (c2.budget > 0) {
+      run_batch_closest(b, q, nullptr, n, c2, 64, idx, dist, cpt, errout, s);
+      return;
+    }
   }
   if (cp.precision == THEA_PRECISION_FP32_REFERENCE && !errout && !b->query_order &&
       (n < CLOSEST_WARP_MAX || n >= CLOSEST_TWO_PHASE_MIN)) {
-    if (n < CLOSEST_WARP_MAX && small_stack_ok(b)) {
+    if (n < (b->width == 4 ? CLOSEST_WARP_MAX : CLOSEST_TEAM_MAX_W8) && small_stack_ok(b)) {
       run_closest_teams(b, q, n, cp, idx, dist, cpt, s);
       return;
     }
