@@ -369,7 +369,8 @@ THEA_API thea_status thea_point_forest_build(const float * points, const int64_t
  * that this replaces is the reference's only form.
  * hard_query_budget (closest element only): each query first runs on one thread for at most this many traversal steps;
  * queries that need more (points deep inside a closed mesh, where thousands of nodes lie within the bound) are then
- * finished by a whole warp each, 32 lanes expanding nodes together. 0 = default (32; 256 from 98,304 queries on),
+ * finished by a whole warp each, 32 lanes expanding nodes together. 0 = default (32; from 98,304
+ * queries on 128 at width 4 and 64 at width 8, from 786,432 on twice that),
  * negative = one thread per query throughout (THEA_PRECISION_FP64_RECHECK: but for a query with more than eight elements
  * within its error band, which goes to a warp at any budget). Results do not depend on it. */
 THEA_API thea_status thea_batch_closest_element(const thea_bvh * mesh_forest, const float * queries,

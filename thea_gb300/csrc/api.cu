@@ -1140,7 +1140,8 @@ THEA_API thea_status thea_batch_closest_element(const thea_bvh * mesh_forest, co
     ClosestParams cp;
     cp.precision = precision;
     cp.scene_scale = scene_scale_of(mesh_forest);
-    cp.budget = hard_query_budget == 0 ? batch_closest_budget(num_queries) : (hard_query_budget < 0 ? 0 : hard_query_budget);
+    cp.budget = hard_query_budget == 0 ? batch_closest_budget(num_queries, mesh_forest->width)
+                                       : (hard_query_budget < 0 ? 0 : hard_query_budget);
     // each mesh applies the bound as closestElement on that mesh alone would (BoundCut): per-mesh cuts on the device
     cudaStream_t s = (cudaStream_t)stream;
     Scratch cuts;
@@ -1264,9 +1265,9 @@ THEA_API thea_status thea_autotune_batch_closest(const float * vertices, int64_t
     best.milliseconds = INFINITY;
     int tried = 0;
     int const widths[2] = {4, 8}, leaves[3] = {1, 2, 4}, chunks[3] = {32, 64, 128};
-    // step budgets around the default of the sample's size (batch_closest_budget)
+    // step budgets on both sides of the default of the sample's size (batch_closest_budget)
     std::vector<int> budgets = {12, 32, 128};
-    if (batch_closest_budget(num_queries) > 128) budgets.insert(budgets.end(), {256, 384});
+    if (num_queries >= BATCH_BUDGET_MIN) budgets.insert(budgets.end(), {256, 384});
     for (int w : widths)
       for (int l : leaves) {
         thea_build_config cfg{};

@@ -23,12 +23,18 @@ BatchForest forest_view(thea_bvh const * b);
 
 // Step budget of a batched closest-point search whose caller names none. A query past its budget is finished by a whole
 // warp, which shortens the launch's longest chains but costs the GPU about five times a thread's search, so a batch that
-// fills the GPU hands over only its longest queries. 256 meshes of 320 to 327,680 triangles with 5.2 M queries: FP32 9.0 /
-// 8.6 ms at budgets of 256 / 384 (with the searches as they were before: 33.3 / 17.7 / 12.4 / 12.3 at 32 / 128 / 256 / 384),
-// FP64 re-check 35.1 / 23.6 / 20.3 / 19.5 at 128 / 192 / 256 / 384; 64 meshes with 210,677 queries: FP32 1.28 / 0.80 / 0.80
-// / 0.89 at 32 / 160 / 256 / 384, FP64 1.60 / 1.42 / 1.40 / 1.48 at 128 / 192 / 256 / 384. A small batch is bound by its
-// longest chain instead (81,920 triangles, two kernels: 32,768 queries 0.44 ms at 16 steps, 0.89 at 256).
-inline int batch_closest_budget(int64_t nq) { return nq >= 98304 ? 256 : 32; }
+// fills the GPU hands over only its longest queries, while a small one is bound by its longest chain. Times over those at 32
+// (each in the kernels of before, the best and the worst of near the surface, in the box, in [-1, 1]^3 and all deep inside;
+// 64 meshes of 1,280 triangles and 16 of 20,480; FP32): width 4, 98,304 queries 0.26 - 1.09 at 128 and 0.26 - 1.53 at 256;
+// 393,216 0.17 - 1.04 and 0.17 - 1.05; 1,048,576 0.15 - 0.66 and 0.15 - 0.80. Width 8, whose steps test twice as many boxes
+// and whole leaves: 98,304 queries 0.40 - 1.11 at 64 and 0.38 - 1.58 at 256; 393,216 0.35 - 1.08 and 0.35 - 1.32; 1,048,576
+// 0.32 - 0.99 at 128 and 0.32 - 1.10 at 256.
+constexpr int64_t BATCH_BUDGET_MIN = 98304, BATCH_BUDGET_LARGE = 786432;
+inline int batch_closest_budget(int64_t nq, int width) {
+  if (nq < BATCH_BUDGET_MIN) return 32;
+  int budget = nq < BATCH_BUDGET_LARGE ? 128 : 256;
+  return width == 4 ? budget : budget / 2;
+}
 
 // qoff: device array of M + 1 query offsets (queries of segment m are [qoff[m], qoff[m+1])), or null for one segment, whose
 // queries are all of them. chunk: queries a warp takes per fetch (a multiple of 32).
