@@ -16,17 +16,29 @@ namespace {
 
 constexpr int QUERY_THREADS = 128;
 
-// Queries a warp of the one-query-per-thread kernels takes: all its lanes once that gives every SM 24 warps, fewer below.
-// The lanes of a warp wait for one another's branches and for the slowest of them, and a small batch packed 32 to a warp
-// leaves most of the GPU idle meanwhile. Call times at 8 / 16 / 24 / 32 / 64 warps per SM, and always packed: 1,000 rays on
-// 32,768 triangles 55 / 60 / 49 / 64 / 50, 64 us; 10,000 rays on 178,802 78 / 72 / 64 / 66 / 75, 78 us; the 8 nearest of
+// Queries a warp of the one-query-per-thread kernels takes: all its lanes once that gives every SM `warps_per_sm` warps, fewer
+// below. The lanes of a warp wait for one another's branches and for the slowest of them, and a small batch packed 32 to a
+// warp leaves most of the GPU idle meanwhile. Call times at 8 / 16 / 24 / 32 / 64 warps per SM, and always packed: 1,000 rays
+// on 32,768 triangles 55 / 60 / 49 / 64 / 50, 64 us; 10,000 rays on 178,802 78 / 72 / 64 / 66 / 75, 78 us; the 8 nearest of
 // 262,144 points, 1,000 queries of 65,536: 70 / 71 / 66 / 70 / 73, 105 us; 10,000: 118 / 108 / 108 / 114 / 137, 124 us.
 constexpr int SPARSE_WARPS_PER_SM = 24;
-int queries_per_warp(int64_t n, int most = 8) {
-  int64_t warps = (int64_t)sm_count() * SPARSE_WARPS_PER_SM;
+int queries_per_warp(int64_t n, int most = 8, int warps_per_sm = SPARSE_WARPS_PER_SM) {
+  int64_t warps = (int64_t)sm_count() * warps_per_sm;
   int per = 1;
   while ((int64_t)per * warps < n) per *= 2;
   return per <= most ? per : 32;
+}
+// For k-NN searches (K: the list's capacity). An insertion costs a warp the same whichever of its lanes make it, so spread lists
+// spend the GPU faster than they gain, the longer the list the more: fewer warps an SM, up to 16 queries each. Spread over 24
+// warps an SM, calls of 16,384 queries on six streams at once took 1.5 times as long as the packed sorted lists of before for the
+// 16 nearest of 262,144 points at width 4, and 2.1 times for the 32 nearest at width 8. As below, calls of 4,000 to 16,384
+// queries for 8, 16 and 32 nearest take 0.71 - 0.99 of it on six streams and 0.51 - 0.90 on one.
+// Triangles (the sorted lists of before): likewise, with 8 and 16 nearest spread as far as 16 points and 32 less.
+int knn_queries_per_warp(int64_t n, int width, int K, bool triangles, bool self) {
+  int warps_per_sm = width == 4 ? (K <= 4 ? SPARSE_WARPS_PER_SM : K <= 8 ? 12 : 7) : (K <= 2 ? SPARSE_WARPS_PER_SM : K <= 4 ? 12 : 4);
+  if (triangles) warps_per_sm = K <= 4 ? 12 : K <= 16 && width == 4 ? 7 : 4;
+  int most = warps_per_sm < SPARSE_WARPS_PER_SM ? 16 : 8;
+  return queries_per_warp(n, self ? most / 2 : most, warps_per_sm);
 }
 unsigned sparse_grid(int64_t n, int per) { return (unsigned)ceil_div(ceil_div(n, per) * 32, QUERY_THREADS); }
 // This thread's query, or n where it has none
@@ -1046,10 +1058,12 @@ void launch_ray(thea_bvh const * b, float const * o, float const * d, int64_t n,
                 d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order, per);
 }
 
+constexpr int64_t KNN_MESH_PACKED = 2048;
+
 template <int W, int K, int STACK>
 void launch_knn_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,
                   int32_t * idx, float * d2, unsigned * err, uint32_t const * order, float const * ib, cudaStream_t s) {
-  int per = queries_per_warp(n, q ? 8 : 4);
+  int per = knn_queries_per_warp(n, W, K, /*triangles=*/false, /*self=*/!q);
   THEA_LAUNCH((knn_kernel<W, K, STACK>), sparse_grid(n, per), QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes,
               b->pt_rec, q, n, k, thresh, ex, idx, d2, err, order, ib, per);
 }
@@ -1057,7 +1071,9 @@ void launch_knn_k(thea_bvh const * b, float const * q, int64_t n, int k, float t
 template <int W, int K, int STACK>
 void launch_knn_mesh_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,
                        int32_t * idx, float * d2, unsigned * err, uint32_t const * order, cudaStream_t s) {
-  int per = queries_per_warp(n);
+  // (a small mesh's queries share its records in L1: 1,000 queries around 1,280 triangles, their nearest, 0.38 ms packed and
+  // 0.52 spread)
+  int per = b->n <= KNN_MESH_PACKED ? 32 : knn_queries_per_warp(n, W, K, /*triangles=*/true, /*self=*/false);
   THEA_LAUNCH((knn_mesh_kernel<W, K, STACK>), sparse_grid(n, per), QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes,
               b->cp_rec, q, n, k, thresh, ex, idx, d2, err, order, per);
 }
