@@ -742,8 +742,11 @@ batch_ray_kernel(BatchForest f, float const * __restrict__ origins, float const 
   }
 }
 
-template <int W, int K, int STACK>
-__global__ void __launch_bounds__(BATCH_THREADS, K <= 16 ? 8 : 4)
+// SORTED: the K best in a sorted list in shared memory (knn_search_shared), for batches that fill the GPU (see
+// knn_sorted_lists). Its insertions shift K / 2 entries, but it needs 50 registers at K = 32 where the unsorted list and its
+// final sort need 88, so seven blocks of 128 threads are resident instead of five.
+template <int W, int K, int STACK, bool SORTED>
+__global__ void __launch_bounds__(BATCH_THREADS, SORTED ? (K == 32 ? 1 : 8) : knn_point_min_blocks<K>())
 batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t const * __restrict__ qoff, int64_t nq,
                  int k_out, float thresh, int32_t * __restrict__ out_index, float * __restrict__ out_d2,
                  unsigned long long * counter, int chunk) {
@@ -753,30 +756,56 @@ batch_knn_kernel(BatchForest f, float const * __restrict__ queries, int64_t cons
     int64_t end = base + chunk < nq ? base + chunk : nq;
     for (int64_t q = base + (threadIdx.x & 31); q < end; q += 32) {
       int m = mesh_of_query(qoff, f.M, q);
-      int pad = K - k_out;
-      float start = thresh + 0.0f;  // (no negative zero)
-      bool any = start >= 0.f;      // a negative threshold admits nothing
-      uint64_t none = knn_key(any ? start : 0.f, INT_MAX);
-      auto entry = [&](int j) { return j < pad ? (uint64_t)0 : none; };
       V3 p = load_v3(queries + 3 * q);
       int root = __ldg(f.seg_root + m);
       int64_t ebase = __ldg(f.seg_start + m);
-      uint64_t keys[K];
-      // lists in shared memory as in knn_kernel (width 4, K = 8, 200,000 queries over 100 sets of 2,000 points: 0.322 ms, in
-      // registers 0.237)
-      if constexpr (K >= 16 || (W == 8 && K >= 8)) {
-        __shared__ uint64_t s_list[K][BATCH_THREADS];
-        SharedKnnList<K, BATCH_THREADS> list(s_list);
-        list.init(entry);
-        if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
-        list.finish(keys);
+      if constexpr (SORTED) {
+        __shared__ float s_d[K][BATCH_THREADS];
+        __shared__ int s_i[K][BATCH_THREADS];
+        int t = threadIdx.x;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          s_d[j][t] = thresh;
+          s_i[j][t] = INT_MAX;
+        }
+        float kth = thresh;
+        int kth_i = INT_MAX;
+        knn_search_shared<W, K, STACK, BATCH_THREADS, W == 8>(nodes, root, ebase, p, -1, s_d, s_i, kth, kth_i, f.err,
+                                                              [&](int64_t k, int & idx, float & d2) {
+                                                                float4 a = __ldg(f.pt_rec + k);
+                                                                idx = __float_as_int(a.w);
+                                                                d2 = squared_norm(xyz(a) - p);
+                                                                return true;
+                                                              });
+        // the row from shared memory
+        for (int j = 0; j < k_out; ++j) {
+          int i = s_i[j][t];
+          out_index[q * k_out + j] = i != INT_MAX ? i : -1;
+          out_d2[q * k_out + j] = i != INT_MAX ? s_d[j][t] : -1.f;
+        }
       } else {
-        RegisterKnnList<K> list;
-        list.init(entry);
-        if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
-        list.finish(keys);
+        int pad = K - k_out;
+        float start = thresh + 0.0f;  // (no negative zero)
+        bool any = start >= 0.f;      // a negative threshold admits nothing
+        uint64_t none = knn_key(any ? start : 0.f, INT_MAX);
+        auto entry = [&](int j) { return j < pad ? (uint64_t)0 : none; };
+        uint64_t keys[K];
+        // lists in shared memory as in knn_kernel (width 4, K = 8, 200,000 queries over 100 sets of 2,000 points: 0.322 ms,
+        // in registers 0.237)
+        if constexpr (knn_lists_shared<W, K>()) {
+          __shared__ uint64_t s_list[K][BATCH_THREADS];
+          SharedKnnList<K, BATCH_THREADS> list(s_list);
+          list.init(entry);
+          if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
+          list.finish(keys);
+        } else {
+          RegisterKnnList<K> list;
+          list.init(entry);
+          if (any) knn_points_search<W, STACK>(nodes, f.pt_rec, root, ebase, p, -1, 0, 0, list, f.err);
+          list.finish(keys);
+        }
+        write_knn_keys<K>(out_index, out_d2, q, k_out, keys);
       }
-      write_knn_keys<K>(out_index, out_d2, q, k_out, keys);
     }
   }
 }
@@ -881,12 +910,24 @@ void launch_batch_ray(BatchForest const & f, float const * o, float const * d, i
               chunk);
 }
 
+// Batches that keep the sorted lists: K = 32 (17 neighbours and more) from 98,304 queries on, and K = 16 at width 8, where the
+// unsorted list shares the registers with 256-byte nodes, from 524,288. Call times in ms, sorted and unsorted, over 100 sets of
+// 1,000 points, 32 nearest, width 4: 300,000 queries 1.62 / 2.05, 1,000,000 4.01 / 5.54; width 8: 1.79 / 2.20, 4.63 / 6.86; 16
+// nearest, width 8: 1,000,000 2.17 / 2.34. (50,000 queries, 32 nearest: 0.94 / 0.73.)
+template <int W, int K> bool knn_sorted_lists(int64_t nq) {
+  if (K == 32) return nq >= 98304;
+  return W == 8 && K == 16 && nq >= 524288;
+}
+
 template <int W, int K, int STACK>
 void launch_batch_knn_k(BatchForest const & f, float const * q, int64_t const * qoff, int64_t nq, int k, float thresh,
                         int32_t * idx, float * d2, unsigned long long * counter, int chunk, cudaStream_t s) {
-  auto kern = batch_knn_kernel<W, K, STACK>;
-  THEA_LAUNCH_NAMED("batch_knn_kernel", kern, persistent_grid((void const *)kern), BATCH_THREADS, 0, s, f, q, qoff, nq, k, thresh, idx, d2,
-              counter, chunk);
+  auto kern = batch_knn_kernel<W, K, STACK, false>;
+  if constexpr (K == 32 || (W == 8 && K == 16)) {
+    if (knn_sorted_lists<W, K>(nq)) kern = batch_knn_kernel<W, K, STACK, true>;
+  }
+  THEA_LAUNCH_NAMED("batch_knn_kernel", kern, persistent_grid((void const *)kern), BATCH_THREADS, 0, s, f, q, qoff, nq, k,
+                    thresh, idx, d2, counter, chunk);
 }
 
 template <int W, int STACK>

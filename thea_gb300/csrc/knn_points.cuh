@@ -17,6 +17,14 @@ __device__ __forceinline__ uint64_t knn_key(float d2, int idx) {
 __device__ __forceinline__ float knn_key_d2(uint64_t key) { return __uint_as_float((uint32_t)(key >> 32)); }
 __device__ __forceinline__ int knn_key_index(uint64_t key) { return (int)(uint32_t)key; }
 
+// Kernels over points keep their K best in shared memory from K = 16 on (width-8 trees, whose 256-byte nodes leave fewer
+// registers, from K = 8 on), and in registers below. Shared memory against registers, 262,144 queries: K = 8, width 4,
+// 0.266 / 0.251 ms; K = 8, width 8, 0.408 / 0.420; K = 16, width 4, 0.403 / 0.454 (five resident blocks). The register
+// allocator is asked for eight resident blocks of 128 threads (four for K = 32, whose lists take 32 KB). The lists of
+// triangles (knn_mesh_kernel) are in shared memory from K = 8 on.
+template <int W, int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 16 || (W == 8 && K >= 8); }
+template <int K> constexpr int knn_point_min_blocks() { return K <= 16 ? 8 : 4; }
+
 // Compare-exchange network sorting K keys ascending (bitonic; every thread the same instructions)
 template <int K> __device__ __forceinline__ void sort_keys(uint64_t (&r)[K]) {
 #pragma unroll
@@ -63,7 +71,7 @@ template <int K> struct RegisterKnnList {
   }
 };
 
-// Lists of 16 and more (knn_lists_shared): unsorted in shared memory ([K][B], entry j of thread t at [j][t]: no bank conflicts), in groups of
+// Larger lists (knn_lists_shared): unsorted in shared memory ([K][B], entry j of thread t at [j][t]: no bank conflicts), in groups of
 // four with each group's largest key in a register. An insertion replaces the largest key of all and looks at its group
 // alone: one store, three loads and a fixed sequence of selects, where a sorted list shifts K / 2 entries on average and
 // a warp waits for the longest shift of its lanes. The row is sorted once, at the end, by a network all lanes run

@@ -442,14 +442,6 @@ void launch_ray_stream(thea_bvh const * b, float const * o, float const * d, int
 // BoundedSortedArrayN.hpp:137-214)
 //============================================================================================================================
 
-// Kernels over points keep their K best in shared memory from K = 16 on (width-8 trees, whose 256-byte nodes leave fewer
-// registers, from K = 8 on), and in registers below. Shared memory against registers, 262,144 queries: K = 8, width 4,
-// 0.266 / 0.251 ms; K = 8, width 8, 0.408 / 0.420; K = 16, width 4, 0.403 / 0.454 (five resident blocks). The register
-// allocator is asked for eight resident blocks of 128 threads (four for K = 32, whose lists take 32 KB). The lists of
-// triangles (knn_mesh_kernel) are in shared memory from K = 8 on.
-template <int W, int K> __host__ __device__ constexpr bool knn_lists_shared() { return K >= 16 || (W == 8 && K >= 8); }
-template <int K> constexpr int knn_point_min_blocks() { return K <= 16 ? 8 : 4; }
-
 // Row `row` of the k-NN outputs from a K-entry list read through gd(j) / gi(j) (registers or shared memory): -1 for
 // empty entries. Whole rows go out as 16-byte stores when they can: rows land at scattered element indices (self
 // mode), and full-sector writes keep the L2 from sending partial sectors to DRAM.
@@ -588,14 +580,14 @@ knn_mesh_kernel(WideNode<W> const * __restrict__ nodes, float4 const * __restric
 //  * up to CLOSEST_TWO_PHASE_MIN: one query per thread (65,536 queries in the box: 0.71 ms; 0.72 with a 16-step budget);
 //  * from there: two kernels with a 256-step budget (persistent lanes, then a warp per query past it; 262,144 queries in
 //    the box: 1.06 ms against 1.84 one per thread).
+//  * at width 8, where a step of 16 lanes expands two nodes, the teams end at CLOSEST_TEAM_MAX_W8: 81,920 triangles, leaves of
+//    four, 32,768 queries in the box 0.63 ms with 16 lanes, 0.51 in two kernels (six streams at once 2.98 and 2.41).
 constexpr int64_t CLOSEST_WARP_MAX = 57344;
+constexpr int64_t CLOSEST_TEAM_MAX_W8 = 16384;
 constexpr int CLOSEST_WARP_BUDGET = 16;
 constexpr int64_t CLOSEST_TWO_PHASE_MIN = 98304;
 constexpr int CLOSEST_TWO_PHASE_BUDGET = 256;
-//  * at width 8, where a step of 16 lanes expands two nodes, the teams end at CLOSEST_TEAM_MAX_W8: 81,920 triangles, leaves of
-//    four, 32,768 queries in the box 0.63 ms with 16 lanes, 0.51 in two kernels (six streams at once 2.98 and 2.41).
 
-constexpr int64_t CLOSEST_TEAM_MAX_W8 = 16384;
 // FP64 re-check calls on one BVH: fewer than F64_WARP_MAX queries (F64_WARP_MAX_SMALL on small meshes) run as a warp per
 // query; the others through the collecting and resolving kernels with a step budget, or one query per thread, in Morton
 // order, with slabs. 1,000 queries on 20,480 triangles, near the surface / uniform in the box grown by half: a warp per query
@@ -605,10 +597,6 @@ constexpr int64_t F64_WARP_MAX_SMALL = 2048;
 constexpr int64_t F64_SMALL_MESH = 2048;
 constexpr int64_t F64_SMALL_LARGE_BATCH = 65536;
 
-//============================================================================================================================
-// Points within a radius (BvhN::rangeQueryIndices with a Ball3 range, BvhN.hpp:1208-1219, 2118-2171; BallN::contains,
-// BallN.hpp:83: (p - center).squaredNorm() <= radius * radius, inclusive, FP32). Counting pass, then a filling pass into
-// each query's slice of a CSR list; the slices are then put in ascending element order.
 bool f64_small_mesh(thea_bvh const * b, int64_t n) {
   return b->n <= F64_SMALL_MESH || (b->n <= 4 * F64_SMALL_MESH && n >= F64_SMALL_LARGE_BATCH);
 }
@@ -641,6 +629,10 @@ int f64_collect_budget(thea_bvh const * b, int64_t n) {
   return b->leaf_size < 8 && n < 32768 ? 128 : 0;
 }
 
+//============================================================================================================================
+// Points within a radius (BvhN::rangeQueryIndices with a Ball3 range, BvhN.hpp:1208-1219, 2118-2171; BallN::contains,
+// BallN.hpp:83: (p - center).squaredNorm() <= radius * radius, inclusive, FP32). Counting pass, then a filling pass into
+// each query's slice of a CSR list; the slices are then put in ascending element order.
 //============================================================================================================================
 
 // Calls visit(leaf position, record) for every point under a node child whose box reaches within `lim` of p. Every such
@@ -1058,8 +1050,6 @@ void launch_ray(thea_bvh const * b, float const * o, float const * d, int64_t n,
                 d, n, rp.max_time, t, idx, nrm, t64, idx64, flags, err, order, per);
 }
 
-constexpr int64_t KNN_MESH_PACKED = 2048;
-
 template <int W, int K, int STACK>
 void launch_knn_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,
                   int32_t * idx, float * d2, unsigned * err, uint32_t const * order, float const * ib, cudaStream_t s) {
@@ -1067,6 +1057,8 @@ void launch_knn_k(thea_bvh const * b, float const * q, int64_t n, int k, float t
   THEA_LAUNCH((knn_kernel<W, K, STACK>), sparse_grid(n, per), QUERY_THREADS, 0, s, (WideNode<W> const *)b->nodes,
               b->pt_rec, q, n, k, thresh, ex, idx, d2, err, order, ib, per);
 }
+
+constexpr int64_t KNN_MESH_PACKED = 2048;
 
 template <int W, int K, int STACK>
 void launch_knn_mesh_k(thea_bvh const * b, float const * q, int64_t n, int k, float thresh, int32_t const * ex,

@@ -37,6 +37,25 @@ __device__ __forceinline__ void load_line(float4 const * p, float4 (&r)[8]) {
   for (int j = 0; j < 8; j += 2) ldg8(p + j, r[j], r[j + 1]);
 }
 
+// The same node through 16-byte loads, which the compiler may place where their values are used: fewer registers at width 8,
+// where a node is 256 bytes, for kernels that need the resident warps more than the data pipe
+template <int W> __device__ __forceinline__ void load_node_16(WideNode<W> const * __restrict__ nodes, int idx,
+                                                              NodeRegs<W> & r) {
+  float4 const * p = reinterpret_cast<float4 const *>(nodes + idx);
+  constexpr int Q = W / 4;
+  float * const rows[6] = {r.lox, r.hix, r.loy, r.hiy, r.loz, r.hiz};
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+      float4 u = __ldg(p + a * Q + q);
+      rows[a][4 * q] = u.x; rows[a][4 * q + 1] = u.y; rows[a][4 * q + 2] = u.z; rows[a][4 * q + 3] = u.w;
+    }
+    int4 c = __ldg(reinterpret_cast<int4 const *>(p + 6 * Q + q));
+    r.child[4 * q] = c.x; r.child[4 * q + 1] = c.y; r.child[4 * q + 2] = c.z; r.child[4 * q + 3] = c.w;
+  }
+}
+
 template <int W> __device__ __forceinline__ void load_node(WideNode<W> const * __restrict__ nodes, int idx,
                                                            NodeRegs<W> & r) {
   float4 const * p = reinterpret_cast<float4 const *>(nodes + idx);

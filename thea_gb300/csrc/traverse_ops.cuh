@@ -1216,7 +1216,7 @@ template <int K> __device__ __forceinline__ void knn_insert(float (&bd)[K], int 
 // kth / kth_i for the reject test. An insertion shifts the larger entries up one place (the same (distance, index)
 // order as knn_insert). Holding the lists out of registers lets twice as many warps stay resident. `elem(k, idx, d2)`
 // gives element k's index and squared distance (false: skip it).
-template <int W, int K, int STACK, int B, class Elem>
+template <int W, int K, int STACK, int B, bool LOADS_16 = false, class Elem>
 __device__ __forceinline__ void knn_search_shared(WideNode<W> const * __restrict__ nodes, int root, int64_t elem_base,
                                                   V3 p, int excl, float (*sd)[B], int (*si)[B], float & kth,
                                                   int & kth_i, unsigned * err, Elem elem) {
@@ -1235,7 +1235,8 @@ __device__ __forceinline__ void knn_search_shared(WideNode<W> const * __restrict
     next = CHILD_EMPTY;
     if (code >= 0) {
       NodeRegs<W> nd;
-      load_node(nodes, code, nd);
+      if constexpr (LOADS_16) load_node_16(nodes, code, nd);
+      else load_node(nodes, code, nd);
       float lb[W];
       point_child_bounds<W>(nd, p, lb);
       push_children_next<W>(nd, lb, kth * PRUNE_SLACK, stk, sp, next, err);
