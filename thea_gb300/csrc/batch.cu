@@ -722,6 +722,55 @@ closest_stream_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long lo
   }
 }
 
+// First hit at width 8 for the batched kernel: the search of ray_query with node and leaf read where they are used, and the
+// node through 16-byte loads: 61 registers and eight resident blocks instead of 80 and six. 2,097,152 rays over 16 meshes of
+// 20,480 triangles: 1.06 ms, through ray_query 1.49.
+template <int STACK>
+__device__ __forceinline__ RayOut ray_query_w8(WideNode<8> const * __restrict__ nodes, float4 const * __restrict__ rec,
+                                               int root, int64_t elem_base, V3 o, V3 d, float max_time, unsigned * err) {
+  RayState ray;
+  ray_setup(ray, o, d);
+  RayOut out;
+  out.t = max_time >= 0.f ? max_time : INFINITY;
+  out.idx = INT_MAX;
+  out.slot = -1;
+  LocalStack<STACK> stk;
+  int sp = 0;
+  int next = root;
+  while (next != CHILD_EMPTY || sp > 0) {
+    int code = next;
+    if (code == CHILD_EMPTY) {
+      --sp;
+      int2 top = stk.get(sp);
+      code = top.x;
+      if (__int_as_float(top.y) > out.t * PRUNE_SLACK) continue;
+    }
+    next = CHILD_EMPTY;
+    if (code >= 0) {
+      NodeRegs<8> nd;
+      load_node_16(nodes, code, nd);
+      float lb[8];
+      ray_child_bounds<8>(nd, ray, lb);
+      push_children_next<8, LocalStack<STACK>, false>(nd, lb, out.t * PRUNE_SLACK, stk, sp, next, err);
+    } else {
+      int first, count;
+      decode_leaf(code, first, count);
+      for (int64_t k = elem_base + first; k < elem_base + first + count; ++k) {
+        float4 const * r = rec + k * RAY_REC_F4;
+        float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
+        float t = ray_triangle_time(o, d, xyz(a), xyz(b), xyz(c));
+        int idx = __float_as_int(a.w);
+        if (t >= 0.f && t <= out.t && (t < out.t || idx < out.idx)) {
+          out.t = t;
+          out.idx = idx;
+          out.slot = k;
+        }
+      }
+    }
+  }
+  return out;
+}
+
 template <int W, int STACK>
 __global__ void __launch_bounds__(BATCH_THREADS)
 batch_ray_kernel(BatchForest f, float const * __restrict__ origins, float const * __restrict__ dirs,
@@ -733,8 +782,13 @@ batch_ray_kernel(BatchForest f, float const * __restrict__ origins, float const 
     int64_t end = base + chunk < nq ? base + chunk : nq;
     for (int64_t q = base + (threadIdx.x & 31); q < end; q += 32) {
       int m = mesh_of_query(qoff, f.M, q);
-      RayOut r = ray_query<W, STACK, false>(nodes, f.ray_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m),
-                                            load_v3(origins + 3 * q), load_v3(dirs + 3 * q), max_time, f.err);
+      RayOut r;
+      if constexpr (W == 8)
+        r = ray_query_w8<STACK>(nodes, f.ray_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m), load_v3(origins + 3 * q),
+                                load_v3(dirs + 3 * q), max_time, f.err);
+      else
+        r = ray_query<W, STACK, false>(nodes, f.ray_rec, __ldg(f.seg_root + m), __ldg(f.seg_start + m),
+                                       load_v3(origins + 3 * q), load_v3(dirs + 3 * q), max_time, f.err);
       bool found = r.idx != INT_MAX;
       out_time[q] = found ? r.t : -1.f;
       if (out_index) out_index[q] = found ? r.idx : -1;

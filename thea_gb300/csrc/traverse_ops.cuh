@@ -280,7 +280,7 @@ struct ClosestOut {
 // order: the nearest is returned in `next` (the
 // next step visits it without a stack round trip) and the others are pushed farthest first as packed (code, bound bits)
 // entries, one 8-byte access each. `next` is CHILD_EMPTY when no child is kept.
-template <int W, class Stk>
+template <int W, class Stk, bool FAST_PATH = true>
 __device__ __forceinline__ void push_children_next(NodeRegs<W> const & nd, float const (&lb)[W], float lim,
                                                    Stk & stk, int & sp, int & next, unsigned * err) {
   uint32_t key[W];
@@ -293,7 +293,7 @@ __device__ __forceinline__ void push_children_next(NodeRegs<W> const & nd, float
   }
   sort_children<W>(key, cc);
   next = key[0] != 0xffffffffu ? cc[0] : CHILD_EMPTY;
-  if (sp + W - 1 <= Stk::FAST) {  // room for every child in the stack's first part: no test per push
+  if (FAST_PATH && sp + W - 1 <= Stk::FAST) {  // room for every child in the stack's first part: no test per push
 #pragma unroll
     for (int c = W - 1; c >= 1; --c)
       if (key[c] != 0xffffffffu) stk.set_fast(sp++, make_int2(cc[c], (int)key[c]));
