@@ -409,10 +409,10 @@ closest_collect_kernel(BatchForest f, ClosestArgs a, int64_t nq, unsigned long l
           load_node(nodes, code, nd);
           children(nd);
         } else {
-          for (int kr = first; kr < first + count; ++kr) {
-            V3 cp;
-            take(cp_record_test(f.cp_rec, ebase + kr, p, cp), kr);
-          }
+          V3 cp;
+          take(cp_record_test(f.cp_rec, ebase + first, p, cp), first);
+          if (count > 1) next = encode_leaf(first + 1, count - 1);
+          steps -= leaf_rest(code, next);
         }
       }
     }

@@ -123,8 +123,9 @@ serve_closest_kernel(ServeTask const * __restrict__ tasks, int64_t const * __res
       r = f64_result(s);
       dist = (float)sqrt(r.d2_64);
     } else {
-      // (not FUSED: several slots' launches share the SMs)
-      if (active) r = closest_query<W, STACK, false>(nodes, rec, 0, 0, p, t->thresh, t->err, budget, t->slabs);
+      // (not FUSED: several slots' launches share the SMs; at width 8 16-byte loads for the same reason, 72 registers and
+      // seven resident blocks instead of 76 and six)
+      if (active) r = closest_query<W, STACK, false, W == 8>(nodes, rec, 0, 0, p, t->thresh, t->err, budget, t->slabs);
       dist = sqrtf(r.d2);
     }
     if (active && !r.done) {

@@ -135,12 +135,21 @@ __device__ __forceinline__ float cp_record_eval(float4 const (&r)[8], V3 p, V3 &
   return squared_norm(cp - p);
 }
 
-// Squared distance and closest point of the record at sorted position k (FP32, reference arithmetic)
+// Squared distance and closest point of the record at sorted position k (FP32, reference arithmetic). LOADS_16: through
+// 16-byte loads (see load_node_16)
+template <bool LOADS_16 = false>
 __device__ __forceinline__ float cp_record_test(float4 const * __restrict__ rec, int64_t k, V3 p, V3 & cp) {
   float4 const * r = rec + k * CP_REC_F4;
   float4 a, b, c, nn;
-  ldg8(r, a, b);
-  ldg8(r + 2, c, nn);
+  if constexpr (LOADS_16) {
+    a = __ldg(r);
+    b = __ldg(r + 1);
+    c = __ldg(r + 2);
+    nn = __ldg(r + 3);
+  } else {
+    ldg8(r, a, b);
+    ldg8(r + 2, c, nn);
+  }
   V3 v0 = xyz(a), v1 = xyz(b), v2 = xyz(c), nrm = xyz(nn);
   // HyperplaneN::closestPoint: p - signedDistance(p) * normal, signedDistance = p . normal - dist
   float sd = dot(p, nrm) - a.w;
@@ -149,8 +158,14 @@ __device__ __forceinline__ float cp_record_test(float4 const * __restrict__ rec,
     cp = proj;
   } else {
     float4 e0, e1, e2, unused;
-    ldg8(r + 4, e0, e1);
-    ldg8(r + 6, e2, unused);
+    if constexpr (LOADS_16) {
+      e0 = __ldg(r + 4);
+      e1 = __ldg(r + 5);
+      e2 = __ldg(r + 6);
+    } else {
+      ldg8(r + 4, e0, e1);
+      ldg8(r + 6, e2, unused);
+    }
     cp = closest_on_perimeter(v0, v1, v2, xyz(e0), b.w, xyz(e1), c.w, xyz(e2), e0.w, p);
   }
   return squared_norm(cp - p);
@@ -513,7 +528,7 @@ __device__ __forceinline__ int leaf_rest(int code, int next) { return code < 0 &
 // 0.694 ms; width 4). Otherwise node and leaf code each read what they need: 69 registers instead of 78, seven resident
 // blocks of 128 threads instead of six. Kernels that several streams run at once are bound by that: the serving loop's
 // 1,048,576 queries in 16 batches on six streams 7.51 ms fused, 6.33 not (one stream: 13.2 both).
-template <int W, int STACK, bool FUSED = W == 4>
+template <int W, int STACK, bool FUSED = W == 4, bool LOADS_16 = false>
 __device__ __forceinline__ ClosestOut closest_query(WideNode<W> const * __restrict__ nodes,
                                                     float4 const * __restrict__ rec, int root, int64_t elem_base, V3 p,
                                                     float thresh, unsigned * err, int budget = 0,
@@ -547,7 +562,8 @@ __device__ __forceinline__ ClosestOut closest_query(WideNode<W> const * __restri
       next = CHILD_EMPTY;
       if (code >= 0) {
         NodeRegs<W> nd;
-        load_node(nodes, code, nd);
+        if constexpr (LOADS_16) load_node_16(nodes, code, nd);
+        else load_node(nodes, code, nd);
         float lb[W];
         point_child_bounds<W>(nd, p, lb);
         if (slabs) {
@@ -634,13 +650,14 @@ __device__ __forceinline__ void f64_take(F64Search & s, float4 const * __restric
 
 // Element tests of one leaf for the mixed-precision search: FP32 distances, band limit `lim` and FP32 best `best32`
 // updated, band entries kept in s (an entry pushed out of a full list is evaluated in FP64 at once).
+template <int W>
 __device__ __forceinline__ void cp_leaf_f64(float4 const * __restrict__ rec, int64_t elem_base, int first, int count,
                                             V3 p, double bound2, float abs_tol, float & lim, float & best32,
                                             F64Search & s) {
   float const REL = 1.0f + 1.0f / 16384.0f;
   for (int kr = first; kr < first + count; ++kr) {
     V3 cp;
-    float d2 = cp_record_test(rec, elem_base + kr, p, cp);
+    float d2 = cp_record_test<W == 8>(rec, elem_base + kr, p, cp);
     if (!(d2 <= lim)) continue;
     if (d2 < best32) {
       best32 = d2;
@@ -730,7 +747,7 @@ __device__ __forceinline__ void closest_search_f64(WideNode<W> const * __restric
     } else {
       int first, count;
       decode_leaf(code, first, count);
-      cp_leaf_f64(rec, elem_base, first, count, p, bound2, abs_tol, lim, best32, s);
+      cp_leaf_f64<W>(rec, elem_base, first, count, p, bound2, abs_tol, lim, best32, s);
     }
   }
   s.lim = lim;
