@@ -16,6 +16,7 @@
 #include "bvh.hpp"
 #include "device_util.cuh"
 #include "query.hpp"
+#include "slab_range.cuh"
 #include "traverse_ops.cuh"
 
 #include <algorithm>
@@ -877,9 +878,10 @@ thea_bvh * build_forest(bool is_mesh, float const * V, int64_t nv, int32_t const
 //============================================================================================================================
 // Oriented slabs of the child slots (slab_normal / slab_lower_bound in traverse_ops.cuh): n = the area-weighted mean of
 // the slot's triangle normals (triangles with a non-finite normal or area left out; +z if the mean vanishes), encoded and
-// decoded as the searches decode it, and the range of n . v over the slot's vertices, widened by the rounding of its
-// FP32 evaluation (in FP64 the pass took 64 us for 81,920 triangles, most of it on the FP64 pipe). Slots with no elements
-// get an empty slab.
+// decoded as the searches decode it, and the range of n . v over the slot's vertices, rounded outwards to float
+// (slab_project, slab_range.cuh: the values of an FP64 evaluation at 19 us a pass for 81,920 triangles; FP64 itself took
+// 64, most of it on the FP64 pipe). Slots with no elements get an empty slab. The sums of the normals are added in the order
+// the lanes arrive, so a slab may differ from one build to the next, within its own rules; answers do not depend on it.
 //
 // Every element contributes to the slot of each of its ancestors, so both passes (normals, then ranges) run one thread
 // per element, which climbs from its leaf's slot to the root. A warp's elements are neighbours in leaf order, hence
@@ -948,12 +950,15 @@ __global__ void slab_leaf_kernel(WideNode<W> const * __restrict__ nodes, int64_t
 }
 
 // Adds (or takes the minimum and maximum of) a float at x without a return value; fmin/fmax of floats of either sign
-// through their integer encodings, with *x starting at +inf (minimum) or -inf (maximum).
+// through their integer encodings, with *x starting at +inf (minimum) or -inf (maximum). A negative zero, which the
+// encodings would order below every negative float, counts as zero.
 __device__ __forceinline__ void atomic_min_float(float * x, float v) {
+  v += 0.f;
   if (v >= 0.f) atomicMin(reinterpret_cast<int *>(x), __float_as_int(v));
   else atomicMax(reinterpret_cast<unsigned *>(x), __float_as_uint(v));
 }
 __device__ __forceinline__ void atomic_max_float(float * x, float v) {
+  v += 0.f;
   if (v >= 0.f) atomicMax(reinterpret_cast<int *>(x), __float_as_int(v));
   else atomicMin(reinterpret_cast<unsigned *>(x), __float_as_uint(v));
 }
@@ -994,26 +999,14 @@ slab_climb_kernel(int64_t n, int const * __restrict__ leaf_slot, uint8_t const *
       if (on) {
         float2 enc = *reinterpret_cast<float2 const *>(slabs + slot);
         V3 nv = slab_normal(make_float4(enc.x, enc.y, 0.f, 0.f));
-        // n . v in FP32 is within 3 * 2^-24 of m = sum |n_i v_i| of its value; 2^-21 m also covers the subtraction
         V3 v[3] = {v0, v1, v2};
-        float m = 0.f;
-        bool finite = true;
-        a = INFINITY;
-        b = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          float x = nv.x * v[j].x, y = nv.y * v[j].y, z = nv.z * v[j].z;
-          float d = x + y + z;
-          float mag = fabsf(x) + fabsf(y) + fabsf(z);
-          finite = finite && mag < INFINITY;
-          m = fmaxf(m, mag);
-          a = fminf(a, d);
-          b = fmaxf(b, d);
+          float lo, hi;
+          slab_project(nv.x, nv.y, nv.z, v[j].x, v[j].y, v[j].z, lo, hi);
+          a = fminf(a, lo);
+          b = fmaxf(b, hi);
         }
-        m = m * (1.0f / 2097152.0f) + 1e-44f;  // (the constant: products below the normal range)
-        a -= m;
-        b += m;
-        if (!finite) a = -INFINITY, b = INFINITY;  // the slab bounds nothing
       }
     } else if (on) {
       a = v0.x;
