@@ -734,7 +734,8 @@ __device__ __forceinline__ void closest_search_f64(WideNode<W> const * __restric
     next = CHILD_EMPTY;
     if (code >= 0) {
       NodeRegs<W> nd;
-      load_node(nodes, code, nd);
+      if constexpr (W == 8) load_node_16(nodes, code, nd);
+      else load_node(nodes, code, nd);
       float lb[W];
       point_child_bounds<W>(nd, p, lb);
       if (slabs) {
