@@ -604,29 +604,31 @@ bool f64_small_mesh(thea_bvh const * b, int64_t n) {
 // Step budget of the collecting kernel, or 0 for one query per thread. The collected form is taken where no kind of query
 // (near the surface, in the box grown by half, in [-1, 1]^3, all deep inside, far outside) is slower in it. Its time over that
 // of one query per thread, the best kind and the worst, on 20,480, 81,920 and 327,680 triangles (budget):
-//  * width 4, leaves of one and two: 3,500 queries 0.27 - 0.76 (128), 8,192 0.45 - 0.87 (256), 32,768 0.57 - 0.82 (256), 65,536
-//    0.63 - 1.09 (256), 100,003 0.56 - 1.01 (256) and 0.58 - 1.03 (224; half the kinds 3 to 5 % faster), 131,072 0.59 - 1.16 (256) and 0.61 - 1.01 (384), 163,840 0.63 - 1.04 (384),
-//    262,144 0.70 - 1.33 (384): the slow ones are the queries deep inside, which the slabs of the one-per-thread form shorten
-//    tenfold. 5,120 triangles: 8,192 0.61 - 0.87 (128) and 0.67 - 1.18 (256).
-//  * width 4, larger leaves: 3,500 0.32 - 0.74 (128), 16,384 0.57 - 0.82 (128), 32,768 0.65 - 0.98 (256), 65,536 0.70 - 1.12
+//  * width 4, leaves of one and two: 3,500 queries 0.22 - 0.88 (64), 8,192 0.40 - 0.81 (128), 16,384 0.54 - 0.87 (192), 32,768
+//    0.57 - 0.82 (256), 65,536 0.63 - 1.09 (256), 100,003 0.56 - 1.01 (256) and 0.58 - 1.03 (224; half the kinds 3 to 5 %
+//    faster), 131,072 0.59 - 1.16 (256) and 0.61 - 1.01 (384), 163,840 0.63 - 1.04 (384), 262,144 0.70 - 1.33 (384): the slow
+//    ones are the queries deep inside, which the slabs of the one-per-thread form shorten tenfold. 5,120 triangles: 16,384
+//    0.75 - 0.88 (128) and 0.75 - 1.22 (256).
+//  * width 4, larger leaves: 3,500 0.24 - 0.79 (64), 16,384 0.57 - 0.82 (128), 32,768 0.65 - 0.98 (256), 65,536 0.70 - 1.12
 //    (256), 262,144 0.74 - 1.60.
-//  * width 8, leaves of one and two: 3,500 0.34 - 0.71 (128), 16,384 0.61 - 0.85 (128), 32,768 0.58 - 0.95 (256), 131,072 0.46
+//  * width 8, leaves of one and two: 3,500 0.25 - 0.73 (64), 16,384 0.61 - 0.85 (128), 32,768 0.58 - 0.95 (256), 131,072 0.46
 //    - 1.00 (256), 262,144 0.57 - 1.26. Leaves of four: 16,384 0.74 - 1.02 (128), 65,536 0.73 - 1.09 (256). Leaves of eight
 //    and sixteen: 8,192 0.56 - 1.19 (128), 65,536 0.74 - 1.73 (256).
 //  * small meshes: nodes and records stay in L1 or nearly, and a warp of neighbours reads them together. 1,280 triangles,
 //    100,000 queries in the box: 0.511 ms one per thread, 0.670 collected.
 // Calls of several streams at once pay for the warps that finish the queries over budget: six streams with 16,384 queries
-// each took 0.81 - 1.33 times as long as one per thread with these budgets (256; 1.01 - 1.50 with 128), at 0.52 - 0.92 of its
-// time on one stream.
+// each took 0.97 - 1.28 times as long as one per thread with these budgets (192; 1.01 - 1.50 with 128, 0.81 - 1.33 with 256),
+// at 0.54 - 0.87 of its time on one stream.
 int f64_collect_budget(thea_bvh const * b, int64_t n) {
   if (f64_small_mesh(b, n)) return 0;
   if (b->width == 4) {
-    if (n < 8192 || (b->n <= 4 * F64_SMALL_MESH && n < 65536)) return 128;
-    if (b->leaf_size <= 2) return n < 81920 ? 256 : n < 114688 ? 224 : n < 163840 ? 384 : 0;
+    if (n < 6144) return 64;
+    if (n < 12288 || (b->n <= 4 * F64_SMALL_MESH && n < 65536)) return 128;
+    if (b->leaf_size <= 2) return n < 24576 ? 192 : n < 81920 ? 256 : n < 114688 ? 224 : n < 163840 ? 384 : 0;
     return n < 32768 ? 128 : n < 65536 ? 256 : 0;
   }
-  if (b->leaf_size <= 2) return n < 32768 ? 128 : n < 131072 ? 256 : 0;
-  return b->leaf_size < 8 && n < 32768 ? 128 : 0;
+  if (b->leaf_size <= 2) return n < 6144 ? 64 : n < 32768 ? 128 : n < 131072 ? 256 : 0;
+  return b->leaf_size < 8 && n < 32768 ? (n < 6144 ? 64 : 128) : 0;
 }
 
 //============================================================================================================================
