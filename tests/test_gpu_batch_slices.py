@@ -1,11 +1,11 @@
-"""Mixed-precision batches longer than one slice of 4,194,304 queries: the queries on both sides of a slice's end, with a step
+"""Mixed-precision batches longer than one slice of 16,777,216 queries: the queries on both sides of a slice's end, with a step
 budget and without, answer as in calls of their own."""
 
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-SLICE = 4194304
+SLICE = 1 << 24
 
 
 @pytest.mark.parametrize("n", [SLICE, SLICE + 1, 2 * SLICE + 77])
