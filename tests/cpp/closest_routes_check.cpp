@@ -2,6 +2,7 @@
 #include "fake_cuda.hpp"
 
 #include "../../thea_gb300/csrc/common.cuh"
+#include "../../thea_gb300/csrc/batch.hpp"
 #include "../../thea_gb300/csrc/bvh.hpp"
 #include "../../thea_gb300/csrc/query.hpp"
 
@@ -50,6 +51,15 @@ int main() {
   // and of the teams
   ok = check(4, 1, 81920, 57343, f32, teams) && check(4, 1, 81920, 57344, f32, threads) && ok;
   ok = check(8, 4, 81920, 16383, f32, teams) && check(8, 4, 81920, 16384, f32, lanes) && ok;
+  // default step budgets of batches
+  int64_t const at[] = {1, 98303, 98304, 786431, 786432, 16777216};
+  int const w4[] = {32, 32, 128, 128, 256, 256}, w8[] = {32, 32, 64, 64, 128, 128};
+  for (int i = 0; i < 6; ++i)
+    if (batch_closest_budget(at[i], 4) != w4[i] || batch_closest_budget(at[i], 8) != w8[i]) {
+      std::printf("%lld queries: budgets %d and %d\n", (long long)at[i], batch_closest_budget(at[i], 4),
+                  batch_closest_budget(at[i], 8));
+      ok = false;
+    }
   if (!ok) return 1;
   std::printf("routes as measured\n");
   return 0;
