@@ -40,9 +40,9 @@ __device__ __forceinline__ bool next_chunk(unsigned long long * counter, int chu
 }
 
 //============================================================================================================================
-// Closest element. Each warp works in rounds of 32 queries, one per lane; every lane of the warp takes part in every
-// round (lanes past the end of the chunk carry no query), so the warp-wide FP64 step of the mixed-precision search and
-// the FP64 error estimate run with all lanes together.
+// Closest element. With error estimates (batch_closest_kernel) each warp works in rounds of 32 queries, one per lane; every
+// lane of the warp takes part in every round (lanes past the end of the chunk carry no query), so the FP64 error estimate
+// runs with all lanes together. Without, and in the mixed-precision mode, lanes take new queries as theirs end.
 //
 // Two-phase form: with budget > 0, phase 1 stops a query after that many steps (nodes and leaves) and queues it with the best
 // element found so far (a valid upper bound); phase 2 finishes the queued queries with one warp per query.

@@ -53,11 +53,6 @@ __device__ __forceinline__ int segment_of(int64_t const * __restrict__ start, in
   return lo;
 }
 
-// Per-segment bounds, 12 ordered ints per segment: [0..2] min of box centres, [3..5] max of box centres,
-// [6..8] min of box lo, [9..11] max of box hi. A warp whose lanes share one segment reduces before its atomics, and a
-// block whose warps all share one segment reduces once more, so a single large segment takes 12 atomics per block
-// rather than per warp (the per-warp form spent 0.5 ms of contended atomics on 2 M triangles).
-//
 // A face index outside [0, nv) sets *bad and reads vertex 0 in its place (nv > 0); the host refuses the build when it next
 // synchronizes.
 __device__ __forceinline__ int64_t face_vertex(int32_t const * __restrict__ F, int64_t k, int64_t nv, bool & out) {
@@ -67,6 +62,10 @@ __device__ __forceinline__ int64_t face_vertex(int32_t const * __restrict__ F, i
   return 0;
 }
 
+// Per-segment bounds, 12 ordered ints per segment: [0..2] min of box centres, [3..5] max of box centres,
+// [6..8] min of box lo, [9..11] max of box hi. A warp whose lanes share one segment reduces before its atomics, and a
+// block whose warps all share one segment reduces once more, so a single large segment takes 12 atomics per block
+// rather than per warp (the per-warp form spent 0.5 ms of contended atomics on 2 M triangles).
 __global__ void elem_box_kernel(float const * __restrict__ V, int64_t nv, int32_t const * __restrict__ F, int64_t n,
                                 int is_mesh, int64_t const * __restrict__ seg_start, int M, float4 * __restrict__ elo,
                                 float4 * __restrict__ ehi, int * __restrict__ bounds, int * __restrict__ bad) {
@@ -152,7 +151,8 @@ __global__ void elem_box_kernel(float const * __restrict__ V, int64_t nv, int32_
   }
 }
 
-// Start values: bounds, the error words and, for one segment, its start, its root and the collapse's first level
+// Start values: bounds, the error words and, for one segment, its start (single_root_kernel and segment_roots_kernel write the
+// roots and the collapse's first level)
 __global__ void build_init_kernel(int * __restrict__ bounds, int M, int * __restrict__ bad, unsigned * __restrict__ err,
                                   int64_t * __restrict__ seg_start, int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,12 +271,12 @@ __device__ __forceinline__ void child_box(int code, float4 const * __restrict__ 
   }
 }
 
-// Bottom-up refit: the second thread to reach a node merges its two children and continues upwards.
 __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
   float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
   return x * y + y * z + z * x;
 }
 
+// Bottom-up refit: the second thread to reach a node merges its two children and continues upwards.
 __global__ void refit_kernel(int64_t n, int const * __restrict__ left, int const * __restrict__ right,
                              int const * __restrict__ first, int const * __restrict__ last,
                              int const * __restrict__ parent, int const * __restrict__ leaf_parent,
