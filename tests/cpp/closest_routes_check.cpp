@@ -51,13 +51,15 @@ int main() {
   // and of the teams
   ok = check(4, 1, 81920, 57343, f32, teams) && check(4, 1, 81920, 57344, f32, threads) && ok;
   ok = check(8, 4, 81920, 16383, f32, teams) && check(8, 4, 81920, 16384, f32, lanes) && ok;
-  // default step budgets of batches
-  int64_t const at[] = {1, 98303, 98304, 786431, 786432, 16777216};
-  int const w4[] = {32, 32, 128, 128, 256, 256}, w8[] = {32, 32, 64, 64, 128, 128};
-  for (int i = 0; i < 6; ++i)
-    if (batch_closest_budget(at[i], 4) != w4[i] || batch_closest_budget(at[i], 8) != w8[i]) {
-      std::printf("%lld queries: budgets %d and %d\n", (long long)at[i], batch_closest_budget(at[i], 4),
-                  batch_closest_budget(at[i], 8));
+  // default step budgets of batches: width, leaf size, queries, budget
+  int64_t const budgets[][4] = {{4, 2, 98303, 32},   {4, 2, 98304, 128},  {4, 2, 262143, 128}, {4, 4, 262144, 256},
+                                {4, 8, 786431, 128}, {4, 8, 786432, 256}, {8, 2, 98303, 32},   {8, 2, 98304, 64},
+                                {8, 4, 196607, 64},  {8, 4, 196608, 128}, {8, 2, 393215, 128}, {8, 2, 393216, 256},
+                                {8, 4, 1 << 24, 128}, {8, 8, 786431, 64}, {8, 8, 786432, 128}};
+  for (auto const & c : budgets)
+    if (batch_closest_budget(c[2], (int)c[0], (int)c[1]) != c[3]) {
+      std::printf("width %d, leaves of %d, %lld queries: budget %d\n", (int)c[0], (int)c[1], (long long)c[2],
+                  batch_closest_budget(c[2], (int)c[0], (int)c[1]));
       ok = false;
     }
   if (!ok) return 1;

@@ -1140,7 +1140,7 @@ THEA_API thea_status thea_batch_closest_element(const thea_bvh * mesh_forest, co
     ClosestParams cp;
     cp.precision = precision;
     cp.scene_scale = scene_scale_of(mesh_forest);
-    cp.budget = hard_query_budget == 0 ? batch_closest_budget(num_queries, mesh_forest->width)
+    cp.budget = hard_query_budget == 0 ? batch_closest_budget(num_queries, mesh_forest->width, mesh_forest->leaf_size)
                                        : (hard_query_budget < 0 ? 0 : hard_query_budget);
     // each mesh applies the bound as closestElement on that mesh alone would (BoundCut): per-mesh cuts on the device
     cudaStream_t s = (cudaStream_t)stream;

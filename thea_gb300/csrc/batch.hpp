@@ -25,15 +25,19 @@ BatchForest forest_view(thea_bvh const * b);
 // warp, which shortens the launch's longest chains but costs the GPU about five times a thread's search, so a batch that
 // fills the GPU hands over only its longest queries, while a small one is bound by its longest chain. Times over those at 32
 // (each in the kernels of before, the best and the worst of near the surface, in the box, in [-1, 1]^3 and all deep inside;
-// 64 meshes of 1,280 triangles and 16 of 20,480; FP32): width 4, 98,304 queries 0.26 - 1.09 at 128 and 0.26 - 1.53 at 256;
-// 393,216 0.17 - 1.04 and 0.17 - 1.05; 1,048,576 0.15 - 0.66 and 0.15 - 0.80. Width 8, whose steps test twice as many boxes
-// and whole leaves: 98,304 queries 0.40 - 1.11 at 64 and 0.38 - 1.58 at 256; 393,216 0.35 - 1.08 and 0.35 - 1.32; 1,048,576
-// 0.32 - 0.99 at 128 and 0.32 - 1.10 at 256.
+// 64 meshes of 1,280 triangles, 16 of 20,480 and 153 of 320 to 81,920; FP32) at budgets of 128 / 256 and, width 8, 64 / 128 / 256:
+//  * width 4, leaves of one to four: 98,304 queries 0.26 - 1.21 / 0.26 - 1.53; 196,608 up to 1.01 / up to 0.87 (leaves of
+//    four 1.04); 262,144 up to 1.03 / 0.99; 393,216 0.17 - 1.03 / 0.17 - 0.84; 1,048,576 0.15 - 0.66 / 0.15 - 0.63.
+//    Leaves of eight: 393,216 0.31 - 0.91 / 0.31 - 1.05; 1,048,576 0.29 - 0.66 / 0.29 - 0.80.
+//  * width 8, whose steps test twice as many boxes and whole leaves, leaves of one to four: 98,304 queries up to 1.16 / 1.14 /
+//    1.47; 196,608 1.06 / 1.01 / 1.27 (leaves up to two 1.04 / 1.01 / 1.02); 393,216 1.07 / 1.00 / 1.04 (1.06 / 1.00 / 0.86).
+//    Leaves of eight: 393,216 0.39 - 1.08 / 1.10 / 1.32; 1,048,576 0.37 - 0.95 / 0.99 / 1.10.
 constexpr int64_t BATCH_BUDGET_MIN = 98304, BATCH_BUDGET_LARGE = 786432;
-inline int batch_closest_budget(int64_t nq, int width) {
+inline int batch_closest_budget(int64_t nq, int width, int leaf) {
   if (nq < BATCH_BUDGET_MIN) return 32;
-  int budget = nq < BATCH_BUDGET_LARGE ? 128 : 256;
-  return width == 4 ? budget : budget / 2;
+  if (width == 4) return nq < (leaf <= 4 ? BATCH_BUDGET_LARGE / 3 : BATCH_BUDGET_LARGE) ? 128 : 256;
+  if (leaf <= 2 && nq >= BATCH_BUDGET_LARGE / 2) return 256;
+  return nq < (leaf <= 4 ? BATCH_BUDGET_LARGE / 4 : BATCH_BUDGET_LARGE) ? 64 : 128;
 }
 
 // qoff: device array of M + 1 query offsets (queries of segment m are [qoff[m], qoff[m+1])), or null for one segment, whose
