@@ -370,9 +370,9 @@ THEA_API thea_status thea_point_forest_build(const float * points, const int64_t
  * hard_query_budget (closest element only): each query first runs on one thread for at most this many traversal steps;
  * queries that need more (points deep inside a closed mesh, where thousands of nodes lie within the bound) are then
  * finished by a whole warp each, 32 lanes expanding nodes together. 0 = default (32 below 98,304 queries; above,
- * 64 to 256 by number of queries, tree width and leaf size), negative = one thread per query throughout (THEA_PRECISION_FP64_RECHECK:
- * but for a query with more than eight elements within its error band, which goes to a warp at any budget). Results do
- * not depend on it. */
+ * 64 to 256 by number of queries, tree width and leaf size), negative = one thread per query throughout
+ * (THEA_PRECISION_FP64_RECHECK: but for a query with more than eight elements within its error band, which goes to a warp
+ * at any budget). Results do not depend on it. */
 THEA_API thea_status thea_batch_closest_element(const thea_bvh * mesh_forest, const float * queries,
                                                 const int64_t * query_offsets, int64_t num_queries, float dist_bound,
                                                 int32_t precision, int32_t queries_per_warp, int32_t hard_query_budget,
